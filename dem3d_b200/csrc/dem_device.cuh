@@ -139,6 +139,10 @@ constexpr int EPI_STORE = 0;    // store a/alpha into the target arrays only
 constexpr int EPI_PREDICT = 1;  // MoveParticles predictor (pass 1)
 constexpr int EPI_CORRECT = 2;  // MoveParticles corrector (pass 2)
 
+// Columns of the ABM ring and of the corrector's sums are laid out for an
+// even number of particles, so that every column starts on 16 bytes.
+__device__ __host__ __forceinline__ size_t ring_stride(int n) { return (size_t)((n + 1) & ~1); }
+
 struct RingMap {
   int phys[5];  // phys[k] = physical slot of logical ipc(k+1); phys[nprev] = spare
 };
@@ -208,24 +212,80 @@ __device__ __forceinline__ unsigned long long sweep_key(int cell, int rank) {
   return ((unsigned long long)(unsigned)cell << 32) | (unsigned)rank;
 }
 
+// 32-byte loads and stores (one instruction and one whole sector each on
+// sm_100; a double4 through two 16-byte accesses looks its sector up twice).
+// The address must be a multiple of 32 bytes.
+struct F8 {
+  float v[8];
+};
+__device__ __forceinline__ double4 ld32(const double4* a) {
+  double4 r;
+  asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+               : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w)
+               : "l"(a));
+  return r;
+}
+__device__ __forceinline__ void st32(double4* a, double4 r) {
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(a), "d"(r.x), "d"(r.y),
+               "d"(r.z), "d"(r.w)
+               : "memory");
+}
+__device__ __forceinline__ F8 ld32(const F8* a) {
+  F8 r;
+  asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=f"(r.v[0]), "=f"(r.v[1]), "=f"(r.v[2]), "=f"(r.v[3]), "=f"(r.v[4]),
+                 "=f"(r.v[5]), "=f"(r.v[6]), "=f"(r.v[7])
+               : "l"(a));
+  return r;
+}
+__device__ __forceinline__ void st32(F8* a, const F8& r) {
+  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(a),
+               "f"(r.v[0]), "f"(r.v[1]), "f"(r.v[2]), "f"(r.v[3]), "f"(r.v[4]), "f"(r.v[5]),
+               "f"(r.v[6]), "f"(r.v[7])
+               : "memory");
+}
+// a velocity copy (double4: one access; float4: 16 bytes)
+__device__ __forceinline__ double4 ldv(const double4* a) { return ld32(a); }
+__device__ __forceinline__ float4 ldv(const float4* a) { return *a; }
+__device__ __forceinline__ void stv(double4* a, double4 r) { st32(a, r); }
+__device__ __forceinline__ void stv(float4* a, float4 r) { *a = r; }
+
 // Contact results handed from the pair kernel to the fold kernel.
 //  - "j" side: what particle j adds for one contact that particle i
 //    evaluated (Force(j) - FN - FT, Torque(j) + Rj*(Nij x FT)), with i's sweep
-//    key; record s of particle j at s*stride + j.
+//    key; slot s of particle j.  A slot holds, for every particle, the
+//    values in whole 32-byte pieces (in_head) and then 16 bytes with the last
+//    value and the key (in_tail): mixed 32 + 16, FP64 64 + 16 bytes.
 //  - "i" side: what particle i adds for the same contact (iForce + FN + FT,
-//    iTorque + (Ri*Nij) x FT), at the contact's place in the contact list.
-struct alignas(16) InRec64 {
-  double2 a, b, c, d, e;  // (key, FN.x) (FN.y, FN.z) (FT.x, FT.y) (FT.z, NxFT.x) (NxFT.y, NxFT.z)
+//    iTorque + (Ri*Nij) x FT), at the contact's place in the contact list:
+//    32-byte pieces (PassArgs::irec) and the ninth value (PassArgs::irec9).
+struct InRec32 {
+  F8 a;  // FN.xyz, FT.xyz (FT = FT + FT remainder), NxFT.xy
+  float z;
 };
-struct alignas(16) InRec32 {
-  float4 a, b, c;  // (key lo, key hi, FN.x, FN.y) (FN.z, FT.xyz) (NxFT.xyz, 0)
+struct InRec64 {
+  double4 a, b;  // FN.xyz FT.x; FT.yz NxFT.xy
+  double z;
 };
-struct alignas(16) IRec64 {
-  double2 a, b, c, d, e;  // (FN.x, FN.y) (FN.z, FT.x) (FT.y, FT.z) (tq.x, tq.y) (tq.z, 0)
+struct IRec32 {
+  F8 a;  // FN.xyz, FT.xyz, tq.xy
+  float z;
 };
-struct alignas(16) IRec32 {
-  float4 a, b, c;  // (FN.xyz, FT.x) (FT.yz, tq.xy) (tq.z, 0, 0, 0); FT = FT + FT remainder
+struct IRec64 {
+  double4 a, b;  // FN.xyz FT.x; FT.yz tq.xy
+  double z;
 };
+// bytes of a "j" slot per particle: mixed, FP64
+constexpr int IN_BYTES32 = 48, IN_BYTES64 = 80;
+// the 32-byte pieces and the 16-byte tail of slot s of particle q, for slots
+// of `rec` bytes per particle laid out for `stride` particles (even, so that
+// every piece is aligned)
+__device__ __host__ __forceinline__ size_t in_head(int rec, int stride, int s, int q) {
+  return (size_t)s * stride * rec + (size_t)q * (rec - 16);
+}
+__device__ __host__ __forceinline__ size_t in_tail(int rec, int stride, int s, int q) {
+  return (size_t)s * stride * rec + (size_t)stride * (rec - 16) + (size_t)q * 16;
+}
 
 // Arguments of the two kernels of a force pass (contact kernel, fold
 // kernel).  V4/W2 are the velocity copies the pass reads for partners
@@ -253,7 +313,8 @@ struct PassArgs {
   double4* Xn;       // positions of the next pass (written by the epilogue)
   V4* v4n;
   W2* w2n;
-  double* ring;      // [(slot*9 + comp)*n + orig]
+  double* ring;      // [(slot*9 + comp)*ring_stride(n) + orig]
+  int nprev;         // ring slots in use (method order - 1, at most 3)
   RingMap rm;
   Counters* cnt;
   int tag;  // 2*(step within a captured chunk) + pass
@@ -265,7 +326,7 @@ struct PassArgs {
   // them back (k_settle_state) before a call reads or changes particle data.
   int lazy;
   // EPI_PREDICT/EPI_CORRECT: the corrector's ring sums sum_k AM(k)*
-  // Previous(ipc(k)) (v, a, alpha: [9][n]), formed by the predictor pass,
+  // Previous(ipc(k)) (v, a, alpha: [9][ring_stride(n)]), formed by the predictor pass,
   // which holds every term of them.  EPI_STORE: ComputeAccelerations'
   // Force(i) and Torque(i) before the division by mass and inertia
   // (src/MForces.f90:319-333) as amsum[3p+k], then amsum[3n+3p+k]; NULL: not
@@ -283,6 +344,7 @@ struct PassArgs {
   int* cstart;
   int* ccount;
   void* irec;
+  void* irec9;
   int cl_cap;
   int* in_cnt;
   void* in_rec;

@@ -304,10 +304,11 @@ __global__ void k_ring_store(int n, StateArrays Q, double* __restrict__ ring, in
   if (cnt->abort) return;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  double* rg = ring + (size_t)slot * 9 * n + i;
-  rg[0 * (size_t)n] = Q.vx[i]; rg[1 * (size_t)n] = Q.vy[i]; rg[2 * (size_t)n] = Q.vz[i];
-  rg[3 * (size_t)n] = Q.ax[i]; rg[4 * (size_t)n] = Q.ay[i]; rg[5 * (size_t)n] = Q.az[i];
-  rg[6 * (size_t)n] = Q.lx[i]; rg[7 * (size_t)n] = Q.ly[i]; rg[8 * (size_t)n] = Q.lz[i];
+  const size_t m = ring_stride(n);
+  double* rg = ring + (size_t)slot * 9 * m + i;
+  rg[0 * m] = Q.vx[i]; rg[1 * m] = Q.vy[i]; rg[2 * m] = Q.vz[i];
+  rg[3 * m] = Q.ax[i]; rg[4 * m] = Q.ay[i]; rg[5 * m] = Q.az[i];
+  rg[6 * m] = Q.lx[i]; rg[7 * m] = Q.ly[i]; rg[8 * m] = Q.lz[i];
 }
 
 // The values the predictor passes leave out (PassArgs::lazy) written back:
@@ -322,9 +323,10 @@ __global__ void k_settle_state(int n, StateArrays Q, StateArrays R, const double
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   if (nprev > 0) {
-    const double* rg = ring + (size_t)slot0 * 9 * n + i;
-    Q.ax[i] = rg[3 * (size_t)n]; Q.ay[i] = rg[4 * (size_t)n]; Q.az[i] = rg[5 * (size_t)n];
-    Q.lx[i] = rg[6 * (size_t)n]; Q.ly[i] = rg[7 * (size_t)n]; Q.lz[i] = rg[8 * (size_t)n];
+    const size_t m = ring_stride(n);
+    const double* rg = ring + (size_t)slot0 * 9 * m + i;
+    Q.ax[i] = rg[3 * m]; Q.ay[i] = rg[4 * m]; Q.az[i] = rg[5 * m];
+    Q.lx[i] = rg[6 * m]; Q.ly[i] = rg[7 * m]; Q.lz[i] = rg[8 * m];
   }
   const double4 x = X1[i];
   R.px[i] = x.x; R.py[i] = x.y; R.pz[i] = x.z;
@@ -535,8 +537,8 @@ __global__ void __launch_bounds__(256) k_prepare(const DevParams* __restrict__ P
       atomicExch(&cnt->nonfinite, 1);
       atomicExch(&cnt->abort, 1);
     }
-    X[p] = make_double4(x[0], x[1], x[2], radius[p]);
-    v4[p] = mk_v4<V4>(src.vx[p], src.vy[p], src.vz[p], src.wx[p]);
+    st32(X + p, make_double4(x[0], x[1], x[2], radius[p]));
+    stv(v4 + p, mk_v4<V4>(src.vx[p], src.vy[p], src.vz[p], src.wx[p]));
     w2[p] = mk_w2<W2>(src.wy[p], src.wz[p]);
     L.mflag[p] = 0;
     note_cell(L, cnt, par, p, cell_cur[p], current_cell(P, x[0], x[1], x[2]));
@@ -703,8 +705,8 @@ __device__ __forceinline__ void pair_fp64_body(const PassArgs<double4, double2>&
 #pragma unroll
     for (int r = 0; r < KSPEC; r++) kspec[r] = r < A.Hr.cap ? A.Hr.key[hslot(A.Hr, p, r)] : -1;
     const DevParams& P = sys_params(A.P, A.sysid, p);
-    const double4 p4 = A.X[p], q4 = A.X[q];
-    const double4 pv4 = A.v4[p], qv4 = A.v4[q];
+    const double4 p4 = ld32(A.X + p), q4 = ld32(A.X + q);
+    const double4 pv4 = ld32(A.v4 + p), qv4 = ld32(A.v4 + q);
     const double2 pw2 = A.w2[p], qw2 = A.w2[q];
     const int cp = PP ? 0 : A.comp[p], cq = PP ? 0 : A.comp[q];
     // Rij = x_j - x_i (minimum image, src/MForces.f90:209-217)
@@ -740,13 +742,12 @@ __device__ __forceinline__ void pair_fp64_body(const PassArgs<double4, double2>&
                  out);
     // "j" half into q's incoming records
     if (s_in < A.in_cap) {
-      InRec64* rec = (InRec64*)A.in_rec + (size_t)s_in * A.in_stride + q;
-      rec->a = make_double2(__longlong_as_double((long long)sweep_key(A.cell_cur[p], A.rank[p])),
-                            out.FN[0]);
-      rec->b = make_double2(out.FN[1], out.FN[2]);
-      rec->c = make_double2(out.FT[0], out.FT[1]);
-      rec->d = make_double2(out.FT[2], out.NxFT[0]);
-      rec->e = make_double2(out.NxFT[1], out.NxFT[2]);
+      char* const in = (char*)A.in_rec;
+      double4* const h = (double4*)(in + in_head(IN_BYTES64, A.in_stride, s_in, q));
+      st32(h, make_double4(out.FN[0], out.FN[1], out.FN[2], out.FT[0]));
+      st32(h + 1, make_double4(out.FT[1], out.FT[2], out.NxFT[0], out.NxFT[1]));
+      *(double2*)(in + in_tail(IN_BYTES64, A.in_stride, s_in, q)) = make_double2(
+          out.NxFT[2], __longlong_as_double((long long)sweep_key(A.cell_cur[p], A.rank[p])));
     } else {
       in_over = true;
     }
@@ -756,12 +757,10 @@ __device__ __forceinline__ void pair_fp64_body(const PassArgs<double4, double2>&
 #pragma unroll
     for (int d = 0; d < 3; d++) RN[d] = p4.w * out.N[d];
     cross3(RN, out.FT, tq);
-    IRec64* ir = (IRec64*)A.irec + s;
-    ir->a = make_double2(out.FN[0], out.FN[1]);
-    ir->b = make_double2(out.FN[2], out.FT[0]);
-    ir->c = make_double2(out.FT[1], out.FT[2]);
-    ir->d = make_double2(tq[0], tq[1]);
-    ir->e = make_double2(tq[2], 0.0);
+    double4* const ir = (double4*)A.irec + 2 * (size_t)s;
+    st32(ir, make_double4(out.FN[0], out.FN[1], out.FN[2], out.FT[0]));
+    st32(ir + 1, make_double4(out.FT[1], out.FT[2], tq[0], tq[1]));
+    ((double*)A.irec9)[s] = tq[2];
     // UpdatePairContact: the record goes to i's new table, in row order
     if (update) {
       if (ord < A.Hw.cap) hist_write(A.Hw, p, ord, q, out.FT, out.VT);
@@ -790,41 +789,57 @@ __global__ void __launch_bounds__(128, MINB) k_pair_fp64(PassArgs<double4, doubl
 // sweep order, a = F/m, alpha = T/I, then the integrator epilogue.  WALLS:
 // some system has walls.
 template <bool PP, int EPI, bool WALLS>
-__device__ __forceinline__ void fold_fp64_body(const PassArgs<double4, double2>& A, int vblock) {
+__device__ __forceinline__ void fold_fp64_body(const PassArgs<double4, double2>& A, int vblock,
+                                               double* stage) {
   __shared__ double s_w[WALLS ? NWM : 1][128];  // |FN| of each wall contact
   __shared__ int s_abort;
-  // one decision for the whole block (it meets block barriers later)
-  if (threadIdx.x == 0) s_abort = A.cnt->abort;
-  __syncthreads();
-  if (s_abort) return;
+  const int p0 = vblock * blockDim.x + threadIdx.x;
+  const int p = p0 < A.n ? p0 : 0;
+  // the integrator's columns and the particle's own data are requested
+  // together, ahead of the abort word
+  stage_epilogue<EPI, false>(A, vblock * blockDim.x, stage);
+  const int c = A.cell_cur[p];
+  const int rank = A.rank[p];
+  const int ni = A.in_cnt[p];
+  const unsigned matched = A.matched[p];
+  const int nc = A.ccount[p];
+  const int st0 = A.cstart[p];
+  const double4 p4 = ld32(A.X + p);
+  const double4 pv4 = ld32(A.v4 + p);
+  const double2 pw2 = A.w2[p];
+  // one decision for the warp (with walls, for the block: it meets block
+  // barriers later)
+  int stop = 0;
+  if (WALLS) {
+    if (threadIdx.x == 0) s_abort = A.cnt->abort;
+    __syncthreads();
+    stop = s_abort;
+  } else {
+    if ((threadIdx.x & 31) == 0) stop = A.cnt->abort;
+    stop = __shfl_sync(0xffffffffu, stop, 0);
+  }
+  if (stop) {
+    stage_wait();
+    return;
+  }
   if (WALLS)
     for (int w = 0; w < A.nw_max; w++) s_w[w][threadIdx.x] = 0.0;
   if (vblock == 0 && threadIdx.x == 0) atomicAdd(&A.cnt->pass_id, 1);  // this pass is done
-  const int p0 = vblock * blockDim.x + threadIdx.x;
-  const int p = p0 < A.n ? p0 : 0;
   // (a slab of a decomposition advances only its own particles)
-  const bool valid = p0 < A.n && in_slab(sys_params(A.P, A.sysid, p), A.cell_cur[p]);
+  const bool valid = p0 < A.n && in_slab(sys_params(A.P, A.sysid, p), c);
+  const int most = __reduce_max_sync(0xffffffffu, valid ? ni : 0);
   const bool update = A.update != 0;
   unsigned n_wc = 0;
   int need = 0;
   bool overflow = false;
-  double d2 = 0.0;
+  double d2 = 0.0, acc[3] = {0.0, 0.0, 0.0}, alp[3] = {0.0, 0.0, 0.0};
   if (valid) {
     const DevParams& P = sys_params(A.P, A.sysid, p);
-    prefetch_epilogue<EPI>(A, P, p, false);
-    const int c = A.cell_cur[p];
-    const unsigned long long key_p = sweep_key(c, A.rank[p]);
-    const int ni = A.in_cnt[p];
+    const unsigned long long key_p = sweep_key(c, rank);
     if (ni) A.in_cnt[p] = 0;  // for the next pass's pair kernel
-    const unsigned matched = A.matched[p];
     if (matched) A.matched[p] = 0u;
-    const int nc = A.ccount[p];
-    const int st0 = A.cstart[p];
-    const double4 p4 = A.X[p];
     const double xp[3] = {p4.x, p4.y, p4.z};
     const double Rp = p4.w;
-    const double4 pv4 = A.v4[p];
-    const double2 pw2 = A.w2[p];
     const double vp[3] = {pv4.x, pv4.y, pv4.z};
     const double wp[3] = {pv4.w, pw2.x, pw2.y};
     const int cp = PP ? 0 : A.comp[p];
@@ -834,15 +849,26 @@ __device__ __forceinline__ void fold_fp64_body(const PassArgs<double4, double2>&
     double iF[3], iT[3] = {0.0, 0.0, 0.0};
 #pragma unroll
     for (int k = 0; k < 3; k++) iF[k] = eff_m * P.gravity[k];
-    const IRec64* ir = (const IRec64*)A.irec + st0;
-    for (int k = 0; k < nc; k++) {
-      const IRec64 r = ir[k];
-      const double FN[3] = {r.a.x, r.a.y, r.b.x}, FT[3] = {r.b.y, r.c.x, r.c.y};
-      const double tq[3] = {r.d.x, r.d.y, r.e.x};
+    auto add_ir = [&](const IRec64& r) {
+      const double FN[3] = {r.a.x, r.a.y, r.a.z}, FT[3] = {r.a.w, r.b.x, r.b.y};
+      const double tq[3] = {r.b.z, r.b.w, r.z};
 #pragma unroll
       for (int d = 0; d < 3; d++) iF[d] = iF[d] + FN[d] + FT[d];
 #pragma unroll
       for (int d = 0; d < 3; d++) iT[d] = iT[d] + tq[d];
+    };
+    auto load_ir = [&](int k) {
+      const double4* a = (const double4*)A.irec + 2 * (size_t)(st0 + k);
+      return IRec64{ld32(a), ld32(a + 1), ((const double*)A.irec9)[st0 + k]};
+    };
+    const char* const in = (const char*)A.in_rec;
+    const SweepOrder ord = sweep_order(ni, most, key_p, in, IN_BYTES64, A.in_stride, p);
+    for (int k = 0; k < nc; k += 2) {  // (two records in flight at a time)
+      const IRec64 r0 = load_ir(k);
+      IRec64 r1;
+      if (k + 1 < nc) r1 = load_ir(k + 1);
+      add_ir(r0);
+      if (k + 1 < nc) add_ir(r1);
     }
     int hw_n = nc;  // the pair kernel wrote the records of the contacts
     // ---- walls (src/MForces.f90:274-314)
@@ -934,13 +960,13 @@ __device__ __forceinline__ void fold_fp64_body(const PassArgs<double4, double2>&
       need = hw_n;
     }
     // ---- Force and Torque in sweep order
-    const InRec64* in = (const InRec64*)A.in_rec + p;
-    const size_t st = (size_t)A.in_stride;
     double F[3] = {0.0, 0.0, 0.0}, T[3] = {0.0, 0.0, 0.0};
     fold_in_order(
-        ni, key_p,
+        ni, key_p, ord, in, IN_BYTES64, A.in_stride, p,
         [&](int e) {
-          return (unsigned long long)__double_as_longlong(((const double*)(in + e * st))[0]);
+          const double4* h = (const double4*)(in + in_head(IN_BYTES64, A.in_stride, e, p));
+          return InRec64{ld32(h), ld32(h + 1),
+                         *(const double*)(in + in_tail(IN_BYTES64, A.in_stride, e, p))};
         },
         [&]() {
 #pragma unroll
@@ -948,10 +974,9 @@ __device__ __forceinline__ void fold_fp64_body(const PassArgs<double4, double2>&
 #pragma unroll
           for (int k = 0; k < 3; k++) T[k] = T[k] + iT[k];
         },
-        [&](int e) {
-          const InRec64 r = in[e * st];
-          const double FN[3] = {r.a.y, r.b.x, r.b.y}, FT[3] = {r.c.x, r.c.y, r.d.x};
-          const double NxFT[3] = {r.d.y, r.e.x, r.e.y};
+        [&](const InRec64& r) {
+          const double FN[3] = {r.a.x, r.a.y, r.a.z}, FT[3] = {r.a.w, r.b.x, r.b.y};
+          const double NxFT[3] = {r.b.z, r.b.w, r.z};
 #pragma unroll
           for (int k = 0; k < 3; k++) F[k] = F[k] - FN[k] - FT[k];
 #pragma unroll
@@ -964,36 +989,42 @@ __device__ __forceinline__ void fold_fp64_body(const PassArgs<double4, double2>&
 #pragma unroll
       for (int k = 0; k < 3; k++) A.amsum[n3 + (size_t)3 * p + k] = T[k];
     }
-    double acc[3], alp[3];
 #pragma unroll
     for (int k = 0; k < 3; k++) acc[k] = F[k] * inv_m;
 #pragma unroll
     for (int k = 0; k < 3; k++) alp[k] = T[k] * inv_i;
-    epilogue<EPI>(A, P, p, xp, Rp, vp, wp, acc, alp, c, d2);
+  }
+  stage_wait();
+  if (valid) {
+    const DevParams& P = sys_params(A.P, A.sysid, p);
+    const double xp[3] = {p4.x, p4.y, p4.z};
+    const double vp[3] = {pv4.x, pv4.y, pv4.z}, wp[3] = {pv4.w, pw2.x, pw2.y};
+    epilogue<EPI>(A, P, p, xp, p4.w, vp, wp, acc, alp, c, stage + threadIdx.x, d2);
   }
   if (WALLS && A.nw_max > 0) wall_partials(s_w, A.nw_max, A.wall_part, vblock);
   if (overflow) {
     atomicExch(&A.cnt->overflow, 1);
     set_abort(A.cnt, A.tag);
   }
-  publish_counts_block(A.cnt, update, 0u, 0u, n_wc, (unsigned)need, 0u);
-  if (EPI != EPI_STORE) publish_disp_block(A.cnt, d2);
+  publish_fold(A.cnt, n_wc, (unsigned)need, d2);
 }
 
 // (STRIDE: grid-stride over blocks of 128 particles, like k_test.  Register
-// budget without walls: 6 blocks of 128 per SM, 80 registers; the predictor
-// spills a little there and still runs faster than at 5 blocks, 135 against
-// 146 us per launch at 1M spheres.)
+// budget without walls: 5 blocks of 128 per SM, 96 registers: 131 us per
+// launch at 1M spheres with 0.6 contacts each, 142 at 6 blocks, where it
+// spills; 153 before the integrator's columns were staged and the records
+// read in 32-byte pieces.)
 template <bool PP, int EPI, bool WALLS, bool STRIDE>
-__global__ void __launch_bounds__(128, WALLS ? 4 : 6) k_fold_fp64(PassArgs<double4, double2> A) {
+__global__ void __launch_bounds__(128, WALLS ? 4 : 5) k_fold_fp64(PassArgs<double4, double2> A) {
   pass_kernel_entry();
+  __shared__ __align__(16) double stage[EpiStage<EPI, false>::SIZE];
   if (!STRIDE) {
-    fold_fp64_body<PP, EPI, WALLS>(A, blockIdx.x);
+    fold_fp64_body<PP, EPI, WALLS>(A, blockIdx.x, stage);
     return;
   }
   const int nvb = (A.n + 127) / 128;
   for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
-    fold_fp64_body<PP, EPI, WALLS>(A, vb);
+    fold_fp64_body<PP, EPI, WALLS>(A, vb, stage);
     __syncthreads();  // the block's shared arrays are reused by the next block of particles
   }
 }
@@ -1014,6 +1045,7 @@ template <bool PP, bool WALLS>
 __global__ void __launch_bounds__(128, 4) k_chunk_fp64(const ChunkPass64* __restrict__ prog,
                                                        int npass, GridSync g) {
   __shared__ ChunkPass64 sp;
+  __shared__ __align__(16) double stage[EpiStage<EPI_PREDICT, false>::SIZE];  // (the larger of the two)
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   const int nthreads = gridDim.x * blockDim.x;
   for (int k = 0; k < npass; k++) {
@@ -1027,8 +1059,8 @@ __global__ void __launch_bounds__(128, 4) k_chunk_fp64(const ChunkPass64* __rest
     pair_fp64_body<PP>(sp.a, blockIdx.x, gridDim.x);
     if (!grid_sync(g)) return;
     for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
-      if (sp.epi == EPI_PREDICT) fold_fp64_body<PP, EPI_PREDICT, WALLS>(sp.a, vb);
-      else fold_fp64_body<PP, EPI_CORRECT, WALLS>(sp.a, vb);
+      if (sp.epi == EPI_PREDICT) fold_fp64_body<PP, EPI_PREDICT, WALLS>(sp.a, vb, stage);
+      else fold_fp64_body<PP, EPI_CORRECT, WALLS>(sp.a, vb, stage);
       __syncthreads();
     }
     if (!grid_sync(g)) return;  // (also: every block is done with sp)

@@ -109,11 +109,12 @@ struct dem_ctx {
   double* amsum = nullptr;  // [9*ncap] corrector ring sums (predictor -> corrector)
   int amsum_cap = 0;
   // test -> pair -> fold kernels of a pass: the contact list (cl_cap
-  // contacts, their "i" results IRec64/IRec32), each particle's place in
+  // contacts, their "i" results in irec and irec9), each particle's place in
   // it, the "j" results per particle (count, in_cap records of
-  // InRec64/InRec32 laid out for pass_cap rows) and the matched record bits
+  // of them laid out for in_stride particles) and the matched record bits
   int2* clist = nullptr;
   void* irec = nullptr;
+  void* irec9 = nullptr;
   int cl_cap = 0;
   int* cstart = nullptr;
   int* ccount = nullptr;
@@ -124,6 +125,7 @@ struct dem_ctx {
   int nw_max = 0;               // walls of the system with the most
   int in_cap = 4;
   int pass_cap = 0;
+  int in_stride = 0;  // pass_cap rounded up to an even number
   double2* pour_cand = nullptr;  // candidate points of one PourParticle call
   int* pour_fits = nullptr;
   int pour_cap = 0;
@@ -383,6 +385,7 @@ void free_lists(dem_ctx* c) {
   cudaFree(c->wall_part);
   cudaFree(c->clist);
   cudaFree(c->irec);
+  cudaFree(c->irec9);
   cudaFree(c->cstart);
   cudaFree(c->ccount);
   cudaFree(c->matched);
@@ -391,6 +394,7 @@ void free_lists(dem_ctx* c) {
   c->wall_part = nullptr;
   c->clist = nullptr;
   c->irec = nullptr;
+  c->irec9 = nullptr;
   c->cstart = nullptr;
   c->ccount = nullptr;
   c->matched = nullptr;
@@ -534,6 +538,7 @@ int grow_capacity(dem_ctx* c, int newcap) {
   c->gid = nullptr;
   c->gid_cap = 0;
   c->L.gid = nullptr;
+  newcap = (newcap + 1) & ~1;  // (the state's columns start on 16 bytes)
   const size_t n = (size_t)c->n, N = (size_t)newcap;
   auto fresh = [&](auto*& p, size_t elems, size_t keep) -> cudaError_t {
     using T = std::remove_reference_t<decltype(*p)>;
@@ -564,7 +569,8 @@ int grow_capacity(dem_ctx* c, int newcap) {
   c->Pr = make_state(sb + 15 * N, N);
   const size_t slots9 = 9 * (size_t)(c->nprev + 1);
   CK(fresh(c->staging, 15 * N, 0));
-  CK(fresh(c->ring, slots9 * N, slots9 * n));  // laid out for n: the first slots9*n
+  // laid out for n: the first slots9 columns
+  CK(fresh(c->ring, slots9 * N, slots9 * ring_stride(c->n)));
   CK(fresh(c->radius, N, n));
   CK(fresh(c->comp, N, n));
   CK(fresh(c->S.orig, N, 0));
@@ -722,6 +728,7 @@ PassArgs<V4, W2> pass_args(dem_ctx* c, int side, bool update, double dt, const R
   A.v4n = (V4*)c->v4[side ^ 1];
   A.w2n = (W2*)c->w2[side ^ 1];
   A.ring = c->ring;
+  A.nprev = c->nprev;
   A.rm = rm;
   A.cnt = c->cnt;
   A.tag = tag;
@@ -733,11 +740,12 @@ PassArgs<V4, W2> pass_args(dem_ctx* c, int side, bool update, double dt, const R
   A.cstart = c->cstart;
   A.ccount = c->ccount;
   A.irec = c->irec;
+  A.irec9 = c->irec9;
   A.cl_cap = c->cl_cap;
   A.in_cnt = c->in_cnt;
   A.in_rec = c->in_rec;
   A.in_cap = c->in_cap;
-  A.in_stride = c->pass_cap;
+  A.in_stride = c->in_stride;
   A.matched = c->matched;
   A.wall_part = c->wall_part;
   A.nw_max = c->nw_max;
@@ -747,14 +755,15 @@ PassArgs<V4, W2> pass_args(dem_ctx* c, int side, bool update, double dt, const R
 }
 
 size_t in_rec_bytes(const dem_ctx* c) {
-  return c->precision == DEM_PREC_MIXED ? sizeof(InRec32) : sizeof(InRec64);
+  return c->precision == DEM_PREC_MIXED ? (size_t)IN_BYTES32 : (size_t)IN_BYTES64;
 }
 
 // the "j" records of a pass laid out for in_cap records of pass_cap rows
 int alloc_incoming(dem_ctx* c, int cap) {
   cudaFree(c->in_rec);
   c->in_rec = nullptr;
-  CK(cudaMalloc(&c->in_rec, in_rec_bytes(c) * (size_t)cap * (size_t)c->pass_cap));
+  c->in_stride = (c->pass_cap + 1) & ~1;  // (the 32-byte pieces stay aligned)
+  CK(cudaMalloc(&c->in_rec, in_rec_bytes(c) * (size_t)cap * (size_t)c->in_stride));
   c->in_cap = cap;
   return DEM_OK;
 }
@@ -763,11 +772,15 @@ int alloc_incoming(dem_ctx* c, int cap) {
 int alloc_contacts(dem_ctx* c, int cap) {
   cudaFree(c->clist);
   cudaFree(c->irec);
+  cudaFree(c->irec9);
   c->clist = nullptr;
   c->irec = nullptr;
-  const size_t rb = c->precision == DEM_PREC_MIXED ? sizeof(IRec32) : sizeof(IRec64);
-  CK(cudaMalloc(&c->clist, sizeof(int2) * (size_t)std::max(cap, 1)));
-  CK(cudaMalloc(&c->irec, rb * (size_t)std::max(cap, 1)));
+  c->irec9 = nullptr;
+  const bool mixed = c->precision == DEM_PREC_MIXED;
+  const size_t m = (size_t)std::max(cap, 1);
+  CK(cudaMalloc(&c->clist, sizeof(int2) * m));
+  CK(cudaMalloc(&c->irec, (mixed ? sizeof(F8) : 2 * sizeof(double4)) * m));
+  CK(cudaMalloc(&c->irec9, (mixed ? sizeof(float) : sizeof(double)) * m));
   c->cl_cap = cap;
   return DEM_OK;
 }
@@ -1338,7 +1351,7 @@ int update_particle_list_impl(dem_ctx* c, int64_t* removed) {
     // the ring and the history tables laid out for n1 particles
     const int slots9 = 9 * (c->nprev + 1);
     double* nr = nullptr;
-    CK(cudaMalloc(&nr, sizeof(double) * (size_t)slots9 * (size_t)std::max(n1, 1)));
+    CK(cudaMalloc(&nr, sizeof(double) * (size_t)slots9 * ring_stride(std::max(n1, 1))));
     if (n1 > 0)
       launch(c, "ring_restride", k_ring_restride, 592u, 256u, (const double*)c->ring, nr, slots9,
              n0, n1);
@@ -1843,11 +1856,11 @@ SlabCols slab_ghost_cols(const dem_ctx* c, int side, int hrows) {
 // pass copies of both sides, both cell entries, both history tables
 SlabCols slab_full_cols(const dem_ctx* c) {
   const bool mixed = c->precision == DEM_PREC_MIXED;
-  const long long N = c->ncap, n = c->n;
+  const long long N = c->ncap, m = (long long)ring_stride(c->n);
   SlabCols C = slab_cols_begin();
   slab_col(C, c->state_block, 8, 30, N * 8);
-  if (c->nprev > 0) slab_col(C, c->ring, 8, 9 * (c->nprev + 1), n * 8);
-  if (c->amsum) slab_col(C, c->amsum, 8, 9, n * 8);
+  if (c->nprev > 0) slab_col(C, c->ring, 8, 9 * (c->nprev + 1), m * 8);
+  if (c->amsum) slab_col(C, c->amsum, 8, 9, m * 8);
   for (int b = 0; b < 2; b++) {
     slab_col(C, c->X[b], 32, 1, 0);
     slab_col(C, c->v4[b], mixed ? 16 : 32, 1, 0);
@@ -2449,6 +2462,7 @@ int dem_set_state(dem_ctx* c, int32_t n, const int32_t* comp, const double* radi
   if (!c->pp && c->nsys == 1)
     for (int i = 0; i < n; i++) c->comp_count[(size_t)comp[i]]++;
   size_t N = (size_t)std::max(std::max(std::max(n, c->ncap_hint), pour_capacity(c, c->comp_count, n)), 1);
+  N = (N + 1) & ~(size_t)1;  // (the state's columns start on 16 bytes)
   c->ncap = (int)N;
   CK(cudaMalloc(&c->state_block, sizeof(double) * 30 * N));
   CK(cudaMalloc(&c->staging, sizeof(double) * 15 * N));
@@ -2643,7 +2657,7 @@ int dem_set_integration(dem_ctx* c, const double* previous, const int32_t* ipc) 
   if (!c || !previous || !ipc) return DEM_ERR_INVALID;
   RESTORE_ORDER;
   if (!c->state_set) return fail(c, DEM_ERR_STATE, "no state");
-  size_t N = (size_t)std::max(c->n, 1);
+  const size_t N = ring_stride(std::max(c->n, 1));
   // logical slot k (ipc(k+1)) -> physical slot k; spare = nprev
   std::vector<double> tmp(9 * N * (c->nprev + 1), 0.0);
   for (int k = 0; k < c->nprev; k++) {
@@ -2664,7 +2678,7 @@ int dem_get_integration(dem_ctx* c, double* previous, int32_t* ipc) {
   if (!c) return DEM_ERR_INVALID;
   RESTORE_ORDER;
   if (!c->state_set) return fail(c, DEM_ERR_STATE, "no state");
-  size_t N = (size_t)std::max(c->n, 1);
+  const size_t N = ring_stride(std::max(c->n, 1));
   std::vector<double> tmp(9 * N * (c->nprev + 1));
   CK(cudaStreamSynchronize(c->stream));
   CK(cudaMemcpy(tmp.data(), c->ring, sizeof(double) * tmp.size(), cudaMemcpyDeviceToHost));
@@ -3912,7 +3926,7 @@ int dem_slab_pack(dem_ctx* c, int32_t what, void* buf, int64_t cap, int64_t* byt
       CK(cudaMemcpyAsync(buf, h, sizeof(h), cudaMemcpyHostToDevice, c->stream));
       launch(c, "slab_jhalf_pack", k_slab_jhalf_pack, blocks_for(c->n_ghosts, 128), 128,
              (const int*)c->slab_ghosts, c->n_ghosts, c->in_cnt, (const char*)c->in_rec,
-             slots, c->pass_cap, rec, c->matched, (char*)buf + SLAB_HEAD + 16);
+             slots, c->in_stride, rec, c->matched, (char*)buf + SLAB_HEAD + 16);
       CK(cudaStreamSynchronize(c->stream));
       return DEM_OK;
     }
@@ -4004,7 +4018,7 @@ int dem_slab_unpack(dem_ctx* c, int32_t what, const void* buf, int64_t bytes) {
       if (r != (int)in_rec_bytes(c) || slots > c->in_cap || rec != SLAB_ID + slots * r)
         return fail(c, DEM_ERR_INVALID, "slab: results from a slab with another layout");
       launch(c, "slab_jhalf_unpack", k_slab_jhalf_unpack, blocks_for(count, 128), 128, recs,
-             count, c->in_cnt, (char*)c->in_rec, c->in_cap, slots, c->pass_cap, r, c->matched,
+             count, c->in_cnt, (char*)c->in_rec, c->in_cap, slots, c->in_stride, r, c->matched,
              c->cnt);
       break;
     }

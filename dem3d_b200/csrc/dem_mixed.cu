@@ -295,7 +295,7 @@ __device__ __forceinline__ void pair_mixed_body(const PassArgs<float4, float2>& 
 #pragma unroll
     for (int r = 0; r < KSPEC; r++) kspec[r] = r < Hr.cap ? Hr.key[hslot(Hr, p, r)] : -1;
     const DevParams& P = sys_params(A.P, A.sysid, p);
-    const double4 p4 = A.X[p], q4 = A.X[q];
+    const double4 p4 = ld32(A.X + p), q4 = ld32(A.X + q);
     const float4 pv4 = A.v4[p], qv4 = A.v4[q];
     const float2 pw2 = A.w2[p], qw2 = A.w2[q];
     const int cp = PP ? 0 : A.comp[p], cq = PP ? 0 : A.comp[q];
@@ -334,21 +334,21 @@ __device__ __forceinline__ void pair_mixed_body(const PassArgs<float4, float2>& 
     // "j" half into q's incoming records
     if (s_in < A.in_cap) {
       const unsigned long long key = sweep_key(A.cell_cur[p], A.rank[p]);
-      InRec32* rec = (InRec32*)A.in_rec + (size_t)s_in * A.in_stride + q;
-      rec->a = make_float4(__uint_as_float((unsigned)key), __uint_as_float((unsigned)(key >> 32)),
-                           out.FN.x, out.FN.y);
-      rec->b = make_float4(out.FN.z, FTs.x, FTs.y, FTs.z);
-      rec->c = make_float4(out.NxFT.x, out.NxFT.y, out.NxFT.z, 0.f);
+      char* const in = (char*)A.in_rec;
+      st32((F8*)(in + in_head(IN_BYTES32, A.in_stride, s_in, q)),
+           F8{{out.FN.x, out.FN.y, out.FN.z, FTs.x, FTs.y, FTs.z, out.NxFT.x, out.NxFT.y}});
+      *(float4*)(in + in_tail(IN_BYTES32, A.in_stride, s_in, q)) =
+          make_float4(out.NxFT.z, 0.f, __uint_as_float((unsigned)key),
+                      __uint_as_float((unsigned)(key >> 32)));
     } else {
       in_over = true;
     }
     need_in = need_in > s_in + 1 ? need_in : s_in + 1;
     // "i" half at the contact's place
     const F3 tq = cross(Ra * out.N, out.FT);
-    IRec32* ir = (IRec32*)A.irec + s;
-    ir->a = make_float4(out.FN.x, out.FN.y, out.FN.z, FTs.x);
-    ir->b = make_float4(FTs.y, FTs.z, tq.x, tq.y);
-    ir->c = make_float4(tq.z, 0.f, 0.f, 0.f);
+    st32((F8*)A.irec + s,
+         F8{{out.FN.x, out.FN.y, out.FN.z, FTs.x, FTs.y, FTs.z, tq.x, tq.y}});
+    ((float*)A.irec9)[s] = tq.z;
     if (update) {
       if (ord < Hw.cap) {
         const size_t i = hslot(Hw, p, ord);
@@ -384,39 +384,54 @@ __global__ void __launch_bounds__(128, MINB) k_pair_mixed(PassArgs<float4, float
 // `vblock` of particles.)
 template <bool PP, int EPI, bool WALLS, bool CONE>
 __device__ __forceinline__ void fold_mixed_body(const PassArgs<float4, float2>& A,
-                                                const MixedView& V, int vblock) {
+                                                const MixedView& V, int vblock, double* stage) {
   __shared__ float s_w[WALLS ? NWM : 1][128];  // |FN| of each wall contact
   __shared__ int s_abort;
-  // one decision for the whole block (it meets block barriers later)
-  if (threadIdx.x == 0) s_abort = A.cnt->abort;
-  __syncthreads();
-  if (s_abort) return;
+  const int p0 = vblock * blockDim.x + threadIdx.x;
+  const int p = p0 < A.n ? p0 : 0;
+  // the integrator's columns and the particle's own data are requested
+  // together, ahead of the abort word
+  stage_epilogue<EPI, true>(A, vblock * blockDim.x, stage);
+  const int c = A.cell_cur[p];
+  const int rank = A.rank[p];
+  const int ni = A.in_cnt[p];
+  const unsigned matched = A.matched[p];
+  const int nc = A.ccount[p];
+  const int st0 = A.cstart[p];
+  const double4 p4 = ld32(A.X + p);
+  // one decision for the warp (with walls, for the block: it meets block
+  // barriers later)
+  int stop = 0;
+  if (WALLS) {
+    if (threadIdx.x == 0) s_abort = A.cnt->abort;
+    __syncthreads();
+    stop = s_abort;
+  } else {
+    if ((threadIdx.x & 31) == 0) stop = A.cnt->abort;
+    stop = __shfl_sync(0xffffffffu, stop, 0);
+  }
+  if (stop) {
+    stage_wait();
+    return;
+  }
   if (WALLS)
     for (int w = 0; w < A.nw_max; w++) s_w[w][threadIdx.x] = 0.f;
   if (vblock == 0 && threadIdx.x == 0) atomicAdd(&A.cnt->pass_id, 1);  // this pass is done
-  const int p0 = vblock * blockDim.x + threadIdx.x;
-  const int p = p0 < A.n ? p0 : 0;
   // (a slab of a decomposition advances only its own particles)
-  const bool valid = p0 < A.n && in_slab(sys_params(A.P, A.sysid, p), A.cell_cur[p]);
+  const bool valid = p0 < A.n && in_slab(sys_params(A.P, A.sysid, p), c);
+  const int most = __reduce_max_sync(0xffffffffu, valid ? ni : 0);
   const bool update = A.update != 0;
   const History& Hr = A.Hr;
   const History& Hw = A.Hw;
   unsigned n_wc = 0;
   int need = 0;
   bool overflow = false;
-  double d2 = 0.0;
+  double d2 = 0.0, acc[3] = {0.0, 0.0, 0.0}, alp[3] = {0.0, 0.0, 0.0};
   if (valid) {
     const DevParams& P = sys_params(A.P, A.sysid, p);
-    prefetch_epilogue<EPI>(A, P, p, true);
-    const int c = A.cell_cur[p];
-    const unsigned long long key_p = sweep_key(c, A.rank[p]);
-    const int ni = A.in_cnt[p];
+    const unsigned long long key_p = sweep_key(c, rank);
     if (ni) A.in_cnt[p] = 0;  // for the next pass's pair kernel
-    const unsigned matched = A.matched[p];
     if (matched) A.matched[p] = 0u;
-    const int nc = A.ccount[p];
-    const int st0 = A.cstart[p];
-    const double4 p4 = A.X[p];
     const double xp[3] = {p4.x, p4.y, p4.z};
     const double Rpd = p4.w;
     const float Rp = (float)Rpd;
@@ -427,11 +442,22 @@ __device__ __forceinline__ void fold_mixed_body(const PassArgs<float4, float2>& 
     F3 iF = mk(eff_m * (float)P.gravity[0], eff_m * (float)P.gravity[1],
                eff_m * (float)P.gravity[2]);
     F3 iT = mk(0.f, 0.f, 0.f);
-    const IRec32* ir = (const IRec32*)A.irec + st0;
-    for (int k = 0; k < nc; k++) {
-      const IRec32 r = ir[k];
-      iF = iF + mk(r.a.x, r.a.y, r.a.z) + mk(r.a.w, r.b.x, r.b.y);
-      iT = iT + mk(r.b.z, r.b.w, r.c.x);
+    // (two records in flight at a time)
+    auto load_ir = [&](int k) {
+      return IRec32{ld32((const F8*)A.irec + (st0 + k)), ((const float*)A.irec9)[st0 + k]};
+    };
+    auto add_ir = [&](const IRec32& r) {
+      iF = iF + mk(r.a.v[0], r.a.v[1], r.a.v[2]) + mk(r.a.v[3], r.a.v[4], r.a.v[5]);
+      iT = iT + mk(r.a.v[6], r.a.v[7], r.z);
+    };
+    const char* const in = (const char*)A.in_rec;
+    const SweepOrder ord = sweep_order(ni, most, key_p, in, IN_BYTES32, A.in_stride, p);
+    for (int k = 0; k < nc; k += 2) {
+      const IRec32 r0 = load_ir(k);
+      IRec32 r1;
+      if (k + 1 < nc) r1 = load_ir(k + 1);
+      add_ir(r0);
+      if (k + 1 < nc) add_ir(r1);
     }
     int hw_n = nc;  // the pair kernel wrote the records of the contacts
     if (WALLS) {
@@ -505,24 +531,20 @@ __device__ __forceinline__ void fold_mixed_body(const PassArgs<float4, float2>& 
       need = hw_n;
     }
     // ---- Force and Torque in sweep order
-    const InRec32* in = (const InRec32*)A.in_rec + p;
-    const size_t st = (size_t)A.in_stride;
     D3 F = D3{0.0, 0.0, 0.0}, T = D3{0.0, 0.0, 0.0};
     fold_in_order(
-        ni, key_p,
+        ni, key_p, ord, in, IN_BYTES32, A.in_stride, p,
         [&](int e) {
-          const float2 k = *(const float2*)(in + e * st);
-          return (unsigned long long)__float_as_uint(k.x) |
-                 ((unsigned long long)__float_as_uint(k.y) << 32);
+          return InRec32{ld32((const F8*)(in + in_head(IN_BYTES32, A.in_stride, e, p))),
+                         *(const float*)(in + in_tail(IN_BYTES32, A.in_stride, e, p))};
         },
         [&]() {
           F = F + iF;
           T = T + iT;
         },
-        [&](int e) {
-          const InRec32 r = in[e * st];
-          const F3 FN = mk(r.a.z, r.a.w, r.b.x), FTs = mk(r.b.y, r.b.z, r.b.w);
-          const F3 NxFT = mk(r.c.x, r.c.y, r.c.z);
+        [&](const InRec32& r) {
+          const F3 FN = mk(r.a.v[0], r.a.v[1], r.a.v[2]), FTs = mk(r.a.v[3], r.a.v[4], r.a.v[5]);
+          const F3 NxFT = mk(r.a.v[6], r.a.v[7], r.z);
           F = F - FN - FTs;
           T = T + Rp * NxFT;
         });
@@ -531,43 +553,60 @@ __device__ __forceinline__ void fold_mixed_body(const PassArgs<float4, float2>& 
       A.amsum[q] = F.x; A.amsum[q + 1] = F.y; A.amsum[q + 2] = F.z;
       A.amsum[n3 + q] = T.x; A.amsum[n3 + q + 1] = T.y; A.amsum[n3 + q + 2] = T.z;
     }
-    const double acc[3] = {F.x * (double)inv_m, F.y * (double)inv_m, F.z * (double)inv_m};
-    const double alp[3] = {T.x * (double)inv_i, T.y * (double)inv_i, T.z * (double)inv_i};
+    acc[0] = F.x * (double)inv_m;
+    acc[1] = F.y * (double)inv_m;
+    acc[2] = F.z * (double)inv_m;
+    alp[0] = T.x * (double)inv_i;
+    alp[1] = T.y * (double)inv_i;
+    alp[2] = T.z * (double)inv_i;
+  }
+  stage_wait();
+  if (valid) {
     // the integrator runs on FP64 velocities: Particle's for the predictor,
     // Predicted's for the corrector (the pass copies are FP32)
+    const DevParams& P = sys_params(A.P, A.sysid, p);
+    const double* const cols = stage + threadIdx.x;
+    const double xp[3] = {p4.x, p4.y, p4.z};
     double vd[3] = {0.0, 0.0, 0.0}, wd[3] = {0.0, 0.0, 0.0};
     if (EPI == EPI_PREDICT) {
-      vd[0] = A.part.vx[p]; vd[1] = A.part.vy[p]; vd[2] = A.part.vz[p];
-      wd[0] = A.part.wx[p]; wd[1] = A.part.wy[p]; wd[2] = A.part.wz[p];
+#pragma unroll
+      for (int d = 0; d < 3; d++) vd[d] = cols[(27 + d) * 128];
+#pragma unroll
+      for (int d = 0; d < 3; d++) wd[d] = cols[(30 + d) * 128];
     } else if (EPI == EPI_CORRECT) {
-      vd[0] = A.pred.vx[p]; vd[1] = A.pred.vy[p]; vd[2] = A.pred.vz[p];
+#pragma unroll
+      for (int d = 0; d < 3; d++) vd[d] = cols[(18 + d) * 128];
     }
-    epilogue<EPI>(A, P, p, xp, Rpd, vd, wd, acc, alp, c, d2);
+    epilogue<EPI>(A, P, p, xp, p4.w, vd, wd, acc, alp, c, cols, d2);
   }
   if (WALLS && A.nw_max > 0) wall_partials(s_w, A.nw_max, A.wall_part, vblock);
   if (overflow) {
     atomicExch(&A.cnt->overflow, 1);
     set_abort(A.cnt, A.tag);
   }
-  publish_counts_block(A.cnt, update, 0u, 0u, n_wc, (unsigned)need, 0u);
-  if (EPI != EPI_STORE) publish_disp_block(A.cnt, d2);
+  publish_fold(A.cnt, n_wc, (unsigned)need, d2);
 }
 
-// (STRIDE: grid-stride over blocks of 128 particles.  Register budget: 6
-// blocks of 128 per SM, 80 registers.  The predictor spills a few registers
-// at that budget and still runs faster than at 5 blocks: 127.6 against
-// 137.9 us per launch at 1M spheres, 611 against 695 us with walls at 4M.)
+// (STRIDE: grid-stride over blocks of 128 particles.  The kernel is bound by
+// the latency of the contact results it gathers and by instruction issue,
+// not by its streams: the staged columns alone move at 6.2 TB/s.  Register
+// budget: 5 blocks of 128 per SM, 96 registers, no spills without cones; at 6
+// blocks the packing with 6.6 contacts per sphere loses (210 against 196 us
+// per launch at 1M spheres) what the one with 0.6 gains (119 against 126).
+// Before the columns were staged, the records read in 32-byte pieces two at
+// a time and the block barriers dropped: 212 and 142 us.)
 template <bool PP, int EPI, bool WALLS, bool CONE, bool STRIDE>
-__global__ void __launch_bounds__(128, 6)
+__global__ void __launch_bounds__(128, 5)
     k_fold_mixed(PassArgs<float4, float2> A, MixedView V) {
   pass_kernel_entry();
+  __shared__ __align__(16) double stage[EpiStage<EPI, true>::SIZE];
   if (!STRIDE) {
-    fold_mixed_body<PP, EPI, WALLS, CONE>(A, V, blockIdx.x);
+    fold_mixed_body<PP, EPI, WALLS, CONE>(A, V, blockIdx.x, stage);
     return;
   }
   const int nvb = (A.n + 127) / 128;
   for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
-    fold_mixed_body<PP, EPI, WALLS, CONE>(A, V, vb);
+    fold_mixed_body<PP, EPI, WALLS, CONE>(A, V, vb, stage);
     __syncthreads();  // the block's shared arrays are reused by the next block of particles
   }
 }
@@ -584,6 +623,7 @@ template <bool PP, bool WALLS, bool CONE>
 __global__ void __launch_bounds__(128, 4) k_chunk_mixed(const ChunkPassMx* __restrict__ prog,
                                                         int npass, GridSync g) {
   __shared__ ChunkPassMx sp;
+  __shared__ __align__(16) double stage[EpiStage<EPI_PREDICT, true>::SIZE];  // (the larger of the two)
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   const int nthreads = gridDim.x * blockDim.x;
   for (int k = 0; k < npass; k++) {
@@ -597,8 +637,8 @@ __global__ void __launch_bounds__(128, 4) k_chunk_mixed(const ChunkPassMx* __res
     pair_mixed_body<PP>(sp.a, sp.v, blockIdx.x, gridDim.x);
     if (!grid_sync(g)) return;
     for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
-      if (sp.epi == EPI_PREDICT) fold_mixed_body<PP, EPI_PREDICT, WALLS, CONE>(sp.a, sp.v, vb);
-      else fold_mixed_body<PP, EPI_CORRECT, WALLS, CONE>(sp.a, sp.v, vb);
+      if (sp.epi == EPI_PREDICT) fold_mixed_body<PP, EPI_PREDICT, WALLS, CONE>(sp.a, sp.v, vb, stage);
+      else fold_mixed_body<PP, EPI_CORRECT, WALLS, CONE>(sp.a, sp.v, vb, stage);
       __syncthreads();
     }
     if (!grid_sync(g)) return;  // (also: every block is done with sp)
@@ -804,14 +844,14 @@ void mixed_pass(MixedBuffers& M, bool pp, int epi, int variant, bool walls, bool
   if (part == 0) {
 #define PCASE(PPV, MB) launch_pass(early, k_pair_mixed<PPV, MB>, pair_blocks, 128, st, A, V)
     if (variant == 1) {
-      if (pp) PCASE(true, 3);
-      else PCASE(false, 3);
-    } else if (variant == 2) {
-      if (pp) PCASE(true, 5);
-      else PCASE(false, 5);
-    } else {
       if (pp) PCASE(true, 4);
       else PCASE(false, 4);
+    } else if (variant == 2) {
+      if (pp) PCASE(true, 8);
+      else PCASE(false, 8);
+    } else {
+      if (pp) PCASE(true, 6);
+      else PCASE(false, 6);
     }
 #undef PCASE
     return;

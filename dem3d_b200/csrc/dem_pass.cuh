@@ -115,18 +115,22 @@ __device__ __forceinline__ void publish_counts_block(Counters* cnt, bool update,
   }
 }
 
-// The largest displacement of the block into the pass maximum (one atomic
-// per block of at most 256 threads).  All threads of the block call.
-__device__ __forceinline__ void publish_disp_block(Counters* cnt, double d2) {
-  __shared__ unsigned s_d[8];
-  const unsigned bits = __float_as_uint(__double2float_ru(sqrt(d2)));
-  const unsigned m = __reduce_max_sync(0xffffffffu, bits);
-  if ((threadIdx.x & 31) == 0) s_d[threadIdx.x >> 5] = m;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    unsigned t = 0u;
-    for (int w = 0; w < (int)(blockDim.x >> 5); w++) t = t > s_d[w] ? t : s_d[w];
-    if (t) atomicMax(&cnt->disp_max, t);
+// The fold kernel's statistics per warp: wall contacts, the most records a
+// particle needs and the largest displacement (rounded up twice in FP32: it
+// is a bound).  The two maxima only grow
+// during a pass, so a warp whose value is not above the current one sends
+// nothing (a stale read only costs an atomic); no block barrier.
+__device__ __forceinline__ void publish_fold(Counters* cnt, unsigned n_wc, unsigned need,
+                                             double d2) {
+  const unsigned FULL = 0xffffffffu;
+  n_wc = __reduce_add_sync(FULL, n_wc);
+  need = __reduce_max_sync(FULL, need);
+  const unsigned d =
+      __reduce_max_sync(FULL, __float_as_uint(__fsqrt_ru(__double2float_ru(d2))));
+  if ((threadIdx.x & 31) == 0) {
+    if (n_wc) atomicAdd(&cnt->wall_contacts, (unsigned long long)n_wc);
+    if ((int)need > *(volatile int*)&cnt->need_capacity) atomicMax(&cnt->need_capacity, (int)need);
+    if (d > *(volatile unsigned*)&cnt->disp_max) atomicMax(&cnt->disp_max, d);
   }
 }
 
@@ -141,28 +145,87 @@ __device__ __forceinline__ int find_record(const History& H, int lo, int hi) {
 // The "j" results a particle received in this pass, in the order of the
 // givers' blocks in the sweep (their keys), with the particle's own block
 // (key_p) at its place: the order in which ComputeAccelerations adds them to
-// Force(p) and Torque(p) (src/MForces.f90:254-259, 319-320).  key_of(e)
-// returns the key of record e; own() and add(e) fold.  The keys of the first
-// 8 records are kept in registers; records past those are rare.
-template <class KeyOf, class Own, class Add>
-__device__ __forceinline__ void fold_in_order(int ni, unsigned long long key_p, KeyOf&& key_of,
-                                              Own&& own, Add&& add) {
-  unsigned long long kr[8];
+// Force(p) and Torque(p) (src/MForces.f90:254-259, 319-320).
+//
+// SweepOrder: turn t of the first 8 records in 4 bits each (the record's
+// number), and the turns before the particle's own block.  The keys of one
+// particle's records differ (a giver evaluates a pair once), so a record's
+// turn is the number of smaller keys; with the order in one register the
+// keys need none while the records are read and added.  More than 8 records
+// (rare): the keys are searched turn by turn.
+struct SweepOrder {
+  unsigned perm;
+  int own;
+};
+__device__ __forceinline__ unsigned long long in_key(const char* in, int rec, int stride, int e,
+                                                     int p) {
+  return *(const unsigned long long*)(in + in_tail(rec, stride, e, p) + 8);
+}
+// (at most M records per particle of the warp)
+template <int M>
+__device__ __forceinline__ SweepOrder order_of(int ni, unsigned long long key_p, const char* in,
+                                               int rec, int stride, int p) {
+  SweepOrder o{0u, 0};
+  unsigned long long kr[M];
+  int t[M];
 #pragma unroll
-  for (int e = 0; e < 8; e++) kr[e] = e < ni ? key_of(e) : ~0ull;
+  for (int e = 0; e < M; e++) kr[e] = e < ni ? in_key(in, rec, stride, e, p) : ~0ull;
+#pragma unroll
+  for (int e = 0; e < M; e++) t[e] = e;  // (every earlier one smaller, as far as is known)
+#pragma unroll
+  for (int e = 0; e < M; e++)
+#pragma unroll
+    for (int f = e + 1; f < M; f++)
+      if (kr[f] < kr[e]) {
+        t[e]++;
+        t[f]--;
+      }
+#pragma unroll
+  for (int e = 0; e < M; e++) {
+    o.perm |= (unsigned)e << (4 * t[e]);
+    if (kr[e] < key_p) o.own++;
+  }
+  return o;
+}
+// All threads of the warp that hold a particle call (`most`: the largest
+// count of them): the order is formed for 2, 4 or 8 records.
+__device__ __forceinline__ SweepOrder sweep_order(int ni, int most, unsigned long long key_p,
+                                                  const char* in, int rec, int stride, int p) {
+  if (most == 0) return SweepOrder{0u, 0};
+  if (most <= 2) return order_of<2>(ni, key_p, in, rec, stride, p);
+  if (most <= 4) return order_of<4>(ni, key_p, in, rec, stride, p);
+  return order_of<8>(ni, key_p, in, rec, stride, p);
+}
+
+// load(e) reads a record, own() and add(record) fold; two records are in
+// flight at a time.
+template <class Load, class Own, class Add>
+__device__ __forceinline__ void fold_in_order(int ni, unsigned long long key_p, SweepOrder o,
+                                              const char* in, int rec, int stride, int p,
+                                              Load&& load, Own&& own, Add&& add) {
+  if (ni <= 8) {
+    for (int t = 0; t < ni; t += 2) {
+      auto r0 = load((int)(o.perm & 15u));
+      decltype(r0) r1;
+      if (t + 1 < ni) r1 = load((int)((o.perm >> 4) & 15u));
+      o.perm >>= 8;
+      if (t == o.own) own();
+      add(r0);
+      if (t + 1 < ni) {
+        if (t + 1 == o.own) own();
+        add(r1);
+      }
+    }
+    if (o.own >= ni) own();
+    return;
+  }
   bool own_done = false;
   unsigned long long lo = 0ull;  // every key >= lo is still to be folded
   for (int t = 0; t < ni; t++) {
-    int best = -1;
+    int best = 0;
     unsigned long long km = ~0ull;
-#pragma unroll
-    for (int e = 0; e < 8; e++)
-      if (e < ni && kr[e] >= lo && kr[e] < km) {
-        km = kr[e];
-        best = e;
-      }
-    for (int e = 8; e < ni; e++) {
-      const unsigned long long k = key_of(e);
+    for (int e = 0; e < ni; e++) {
+      const unsigned long long k = in_key(in, rec, stride, e, p);
       if (k >= lo && k < km) {
         km = k;
         best = e;
@@ -172,7 +235,7 @@ __device__ __forceinline__ void fold_in_order(int ni, unsigned long long key_p, 
       own();
       own_done = true;
     }
-    add(best);
+    add(load(best));
     lo = km + 1ull;
   }
   if (!own_done) own();
@@ -203,40 +266,73 @@ __device__ __forceinline__ void prefetch_l2(const void* ptr) {
   asm volatile("prefetch.global.L2 [%0];" ::"l"(ptr));
 }
 
-// The state the integrator epilogue of particle p will read, requested into
-// L2 at the start of the fold kernel so that those reads overlap the fold
-// (they do not depend on it).  mixed: the FP64 velocities of Particle
-// (predictor) or Predicted (corrector) come from the state arrays.
-template <int EPI, class V4, class W2>
-__device__ __forceinline__ void prefetch_epilogue(const PassArgs<V4, W2>& A, const DevParams& P,
-                                                  int p, bool mixed) {
+// The state the integrator epilogues of a warp's 32 particles will read,
+// copied into the block's shared memory with cp.async: column c of the
+// block's 128 particles at [c*128 + thread].  The copies are requested as the
+// first thing of the fold kernel and hold no registers while they are in
+// flight; in 16-byte pieces they pass by the L1, which the contact results
+// read in between need (8-byte pieces go through it).  A half-warp copies the
+// 32 particles of one column, so an instruction moves two columns; every
+// column starts on 16 bytes and the block's first particle is a multiple of
+// 128.  Predictor: the ring slots (9 columns each), then (mixed) Particle
+// v, w; corrector: the ring sums, Particle x, v, w, then (mixed) Predicted v.
+template <int EPI, bool MIXED>
+struct EpiStage {
+  static constexpr int COLS = EPI == EPI_STORE     ? 0
+                              : EPI == EPI_PREDICT ? 27 + (MIXED ? 6 : 0)
+                                                   : 18 + (MIXED ? 3 : 0);
+  static constexpr int SIZE = COLS > 0 ? COLS * 128 : 1;  // doubles of a block
+};
+
+__device__ __forceinline__ void async_copy16(double* dst, const double* src) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+}
+
+// p0: the block's first particle; stage: the block's columns.  All threads
+// of the warp call.
+template <int EPI, bool MIXED, class V4, class W2>
+__device__ __forceinline__ void stage_epilogue(const PassArgs<V4, W2>& A, int p0, double* stage) {
   if (EPI == EPI_STORE) return;
-  const size_t n = (size_t)A.n;
+  const int lane = threadIdx.x & 31;
+  const int at = (threadIdx.x & ~31) + 2 * (lane & 15);  // place in the block
+  const int p = p0 + at;
+  if (p >= A.n) return;  // (a piece may end one particle past the last: padding)
+  const int half = lane >> 4;
+  const size_t n = ring_stride(A.n);
   if (EPI == EPI_PREDICT) {
-    for (int k = 0; k < P.nprev; k++) {
-      const double* rg = A.ring + (size_t)A.rm.phys[k] * 9 * n + p;
+    const int nc = 9 * A.nprev;
 #pragma unroll
-      for (int d = 0; d < 9; d++) prefetch_l2(rg + d * n);
+    for (int k = 0; k < 28; k += 2) {
+      const int c = k + half;
+      const int slot = c / 9;
+      if (c < nc)
+        async_copy16(stage + c * 128 + at,
+                     A.ring + ((size_t)A.rm.phys[slot] * 9 + (c - 9 * slot)) * n + p);
     }
-    if (mixed) {
+    if (MIXED) {
       const double* v[6] = {A.part.vx, A.part.vy, A.part.vz, A.part.wx, A.part.wy, A.part.wz};
 #pragma unroll
-      for (int d = 0; d < 6; d++) prefetch_l2(v[d] + p);
+      for (int d = 0; d < 6; d += 2)
+        async_copy16(stage + (27 + d + half) * 128 + at, (half ? v[d + 1] : v[d]) + p);
     }
   } else {
     if (A.amsum)
 #pragma unroll
-      for (int d = 0; d < 9; d++) prefetch_l2(A.amsum + d * n + p);
-    const double* q[9] = {A.part.px, A.part.py, A.part.pz, A.part.vx, A.part.vy,
-                          A.part.vz, A.part.wx, A.part.wy, A.part.wz};
+      for (int d = 0; d < 10; d += 2)
+        if (d + half < 9) async_copy16(stage + (d + half) * 128 + at, A.amsum + (d + half) * n + p);
+    const double* q[12] = {A.part.px, A.part.py, A.part.pz, A.part.vx, A.part.vy, A.part.vz,
+                           A.part.wx, A.part.wy, A.part.wz, A.pred.vx, A.pred.vy, A.pred.vz};
 #pragma unroll
-    for (int d = 0; d < 9; d++) prefetch_l2(q[d] + p);
-    if (mixed) {
-      prefetch_l2(A.pred.vx + p);
-      prefetch_l2(A.pred.vy + p);
-      prefetch_l2(A.pred.vz + p);
-    }
+    for (int d = 0; d < (MIXED ? 12 : 10); d += 2)
+      if (d + half < (MIXED ? 12 : 9))
+        async_copy16(stage + (9 + d + half) * 128 + at, (half ? q[d + 1] : q[d]) + p);
   }
+}
+// the warp's columns have arrived (all threads of the warp call)
+__device__ __forceinline__ void stage_wait() {
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncwarp();
 }
 
 // The integrator part of a pass, after a = F/m and alpha = T/I
@@ -249,91 +345,70 @@ __device__ __forceinline__ void prefetch_epilogue(const PassArgs<V4, W2>& A, con
 //  EPI_CORRECT the AM corrector (src/MDEM.f90:340-367) with v~ = vp; the new
 //              x(t+dt) is the next pass's position.
 // d2 receives the squared displacement from this pass's position to the next.
+// s: the thread's staged columns (stage_epilogue; the caller has waited).
 template <int EPI, class V4, class W2>
 __device__ __forceinline__ void epilogue(const PassArgs<V4, W2>& A, const DevParams& P, int p,
                                          const double xp[3], double Rp, const double vp[3],
                                          const double wp[3], const double acc[3],
-                                         const double alp[3], int c_cur, double& d2) {
+                                         const double alp[3], int c_cur, const double* s,
+                                         double& d2) {
   const Box& B = P.box;
-  const size_t n = (size_t)A.n;
+  const size_t n = ring_stride(A.n);
   if (EPI == EPI_STORE) {
     A.tgt.ax[p] = acc[0]; A.tgt.ay[p] = acc[1]; A.tgt.az[p] = acc[2];
     A.tgt.lx[p] = alp[0]; A.tgt.ly[p] = alp[1]; A.tgt.lz[p] = alp[2];
     return;
-  }
-  double sv[3] = {0.0, 0.0, 0.0}, sa[3] = {0.0, 0.0, 0.0}, sl[3] = {0.0, 0.0, 0.0};
-  if (EPI == EPI_CORRECT && A.amsum) {
-    // sum_k AM(k)*Previous(ipc(k)) over the rotated ring, as the predictor
-    // pass formed it (same terms, same order)
-#pragma unroll
-    for (int d = 0; d < 3; d++) sv[d] = A.amsum[d * n + p];
-#pragma unroll
-    for (int d = 0; d < 3; d++) sa[d] = A.amsum[(3 + d) * n + p];
-#pragma unroll
-    for (int d = 0; d < 3; d++) sl[d] = A.amsum[(6 + d) * n + p];
-  } else {
-    // the predictor also forms the corrector's sums: after the ring rotation
-    // its slot k is this pass's (v, a, alpha) for k = 0, else the slot k-1
-    // read here
-    const bool am = EPI == EPI_PREDICT && A.amsum && P.nprev > 0;
-    double mv[3], ma[3], ml[3];
-    if (am) {
-#pragma unroll
-      for (int d = 0; d < 3; d++) mv[d] = 0.0 + P.am[0] * vp[d];
-#pragma unroll
-      for (int d = 0; d < 3; d++) ma[d] = 0.0 + P.am[0] * acc[d];
-#pragma unroll
-      for (int d = 0; d < 3; d++) ml[d] = 0.0 + P.am[0] * alp[d];
-    }
-    for (int k = 0; k < P.nprev; k++) {
-      const double C = EPI == EPI_PREDICT ? P.ab[k] : P.am[k];
-      const double* rg = A.ring + (size_t)A.rm.phys[k] * 9 * n + p;
-      double t[9];
-#pragma unroll
-      for (int d = 0; d < 9; d++) t[d] = rg[d * n];
-#pragma unroll
-      for (int d = 0; d < 3; d++) sv[d] = sv[d] + C * t[d];
-#pragma unroll
-      for (int d = 0; d < 3; d++) sa[d] = sa[d] + C * t[3 + d];
-#pragma unroll
-      for (int d = 0; d < 3; d++) sl[d] = sl[d] + C * t[6 + d];
-      if (am && k + 1 < P.nprev) {
-        const double M = P.am[k + 1];
-#pragma unroll
-        for (int d = 0; d < 3; d++) mv[d] = mv[d] + M * t[d];
-#pragma unroll
-        for (int d = 0; d < 3; d++) ma[d] = ma[d] + M * t[3 + d];
-#pragma unroll
-        for (int d = 0; d < 3; d++) ml[d] = ml[d] + M * t[6 + d];
-      }
-    }
-    if (am) {
-#pragma unroll
-      for (int d = 0; d < 3; d++) A.amsum[d * n + p] = mv[d];
-#pragma unroll
-      for (int d = 0; d < 3; d++) A.amsum[(3 + d) * n + p] = ma[d];
-#pragma unroll
-      for (int d = 0; d < 3; d++) A.amsum[(6 + d) * n + p] = ml[d];
-    }
   }
   double x[3], v[3], w[3];
   if (EPI == EPI_PREDICT) {
     const StateArrays& Q = A.part;
     const StateArrays& R = A.pred;
     // (with A.lazy, a and alpha stay in the new ring slot only)
-    if (!A.lazy || P.nprev == 0) {
+    if (!A.lazy || A.nprev == 0) {
       Q.ax[p] = acc[0]; Q.ay[p] = acc[1]; Q.az[p] = acc[2];
       Q.lx[p] = alp[0]; Q.ly[p] = alp[1]; Q.lz[p] = alp[2];
     }
+    // the predictor also forms the corrector's sums: after the ring rotation
+    // its slot k is this pass's (v, a, alpha) for k = 0, else the slot k-1
+    // read here
+    const bool am = A.amsum && A.nprev > 0;
+    double* rg = A.ring + (size_t)A.rm.phys[A.nprev] * 9 * n + p;
 #pragma unroll
-    for (int d = 0; d < 3; d++) x[d] = xp[d] + P.ab0 * vp[d] + sv[d];
+    for (int d = 0; d < 3; d++) {
+      double sv = 0.0, sa = 0.0, sl = 0.0;
+      double mv = 0.0 + P.am[0] * vp[d], ma = 0.0 + P.am[0] * acc[d],
+             ml = 0.0 + P.am[0] * alp[d];
 #pragma unroll
-    for (int d = 0; d < 3; d++) v[d] = vp[d] + P.ab0 * acc[d] + sa[d];
-#pragma unroll
-    for (int d = 0; d < 3; d++) w[d] = wp[d] + P.ab0 * alp[d] + sl[d];
-#pragma unroll
-    for (int d = 0; d < 3; d++)
+      for (int k = 0; k < 3; k++)
+        if (k < A.nprev) {
+          const double C = P.ab[k];
+          const double tv = s[(9 * k + d) * 128], ta = s[(9 * k + 3 + d) * 128],
+                       tl = s[(9 * k + 6 + d) * 128];
+          sv = sv + C * tv;
+          sa = sa + C * ta;
+          sl = sl + C * tl;
+          if (k + 1 < 3 && k + 1 < A.nprev) {
+            const double M = P.am[k + 1 < 3 ? k + 1 : 0];
+            mv = mv + M * tv;
+            ma = ma + M * ta;
+            ml = ml + M * tl;
+          }
+        }
+      if (am) {
+        A.amsum[d * n + p] = mv;
+        A.amsum[(3 + d) * n + p] = ma;
+        A.amsum[(6 + d) * n + p] = ml;
+      }
+      x[d] = xp[d] + P.ab0 * vp[d] + sv;
+      v[d] = vp[d] + P.ab0 * acc[d] + sa;
+      w[d] = wp[d] + P.ab0 * alp[d] + sl;
       if (B.pbc[d]) x[d] = x[d] - B.lbox[d] * fnint(x[d] * B.inv_lbox[d]);
+      if (A.nprev > 0) {
+        rg[d * n] = vp[d];
+        rg[(3 + d) * n] = acc[d];
+        rg[(6 + d) * n] = alp[d];
+      }
+    }
     // (with A.lazy, Predicted x stays in the position copy Xn, and with
     // FP64 copies Predicted v, w stay in v4n, w2n; the mixed corrector reads
     // Predicted v, and its FP32 copies do not hold v, w exactly)
@@ -344,46 +419,34 @@ __device__ __forceinline__ void epilogue(const PassArgs<V4, W2>& A, const DevPar
       R.vx[p] = v[0]; R.vy[p] = v[1]; R.vz[p] = v[2];
       R.wx[p] = w[0]; R.wy[p] = w[1]; R.wz[p] = w[2];
     }
-    if (P.nprev > 0) {
-      double* rg = A.ring + (size_t)A.rm.phys[P.nprev] * 9 * n + p;
-#pragma unroll
-      for (int d = 0; d < 3; d++) rg[d * n] = vp[d];
-#pragma unroll
-      for (int d = 0; d < 3; d++) rg[(3 + d) * n] = acc[d];
-#pragma unroll
-      for (int d = 0; d < 3; d++) rg[(6 + d) * n] = alp[d];
-    }
   } else {
     const StateArrays& Q = A.part;
     const StateArrays& R = A.pred;
     R.ax[p] = acc[0]; R.ay[p] = acc[1]; R.az[p] = acc[2];
     R.lx[p] = alp[0]; R.ly[p] = alp[1]; R.lz[p] = alp[2];
-    x[0] = Q.px[p]; x[1] = Q.py[p]; x[2] = Q.pz[p];
-    v[0] = Q.vx[p]; v[1] = Q.vy[p]; v[2] = Q.vz[p];
-    w[0] = Q.wx[p]; w[1] = Q.wy[p]; w[2] = Q.wz[p];
-#pragma unroll
-    for (int d = 0; d < 3; d++) x[d] = x[d] + P.am0 * vp[d] + sv[d];
-#pragma unroll
-    for (int d = 0; d < 3; d++) v[d] = v[d] + P.am0 * acc[d] + sa[d];
-#pragma unroll
-    for (int d = 0; d < 3; d++) w[d] = w[d] + P.am0 * alp[d] + sl[d];
-#pragma unroll
-    for (int d = 0; d < 3; d++)
-      if (B.pbc[d]) x[d] = x[d] - B.lbox[d] * fnint(x[d] * B.inv_lbox[d]);
-    Q.px[p] = x[0]; Q.py[p] = x[1]; Q.pz[p] = x[2];
-    Q.vx[p] = v[0]; Q.vy[p] = v[1]; Q.vz[p] = v[2];
-    Q.wx[p] = w[0]; Q.wy[p] = w[1]; Q.wz[p] = w[2];
+    double* q[9] = {Q.px, Q.py, Q.pz, Q.vx, Q.vy, Q.vz, Q.wx, Q.wy, Q.wz};
     bool out = false;
 #pragma unroll
     for (int d = 0; d < 3; d++) {
+      // sum_k AM(k)*Previous(ipc(k)) over the rotated ring, as the predictor
+      // pass formed it (no ring: empty sums)
+      const double sv = A.amsum ? s[d * 128] : 0.0, sa = A.amsum ? s[(3 + d) * 128] : 0.0,
+                   sl = A.amsum ? s[(6 + d) * 128] : 0.0;
+      x[d] = s[(9 + d) * 128] + P.am0 * vp[d] + sv;
+      v[d] = s[(12 + d) * 128] + P.am0 * acc[d] + sa;
+      w[d] = s[(15 + d) * 128] + P.am0 * alp[d] + sl;
+      if (B.pbc[d]) x[d] = x[d] - B.lbox[d] * fnint(x[d] * B.inv_lbox[d]);
+      q[d][p] = x[d];
+      q[3 + d][p] = v[d];
+      q[6 + d][p] = w[d];
       const double h = 0.5 * B.lbox[d];
       out = out || (x[d] > h) || (x[d] < -h);
     }
     if (out) atomicAdd(&A.cnt->escaped, 1ull);
   }
   // the next pass's copies, cell and displacement
-  A.Xn[p] = make_double4(x[0], x[1], x[2], Rp);
-  A.v4n[p] = mk_v4<V4>(v[0], v[1], v[2], w[0]);
+  st32(A.Xn + p, make_double4(x[0], x[1], x[2], Rp));
+  stv(A.v4n + p, mk_v4<V4>(v[0], v[1], v[2], w[0]));
   A.w2n[p] = mk_w2<W2>(w[1], w[2]);
   note_cell(A.L, A.cnt, A.par_nxt, p, c_cur, current_cell(P, x[0], x[1], x[2]));
   d2 = disp2(B, x, xp);

@@ -274,7 +274,7 @@ __global__ void __launch_bounds__(RM_THREADS, 1) k_remove(RemovalArgs A) {
       if (t == 16) A.comp[i] = A.comp[NP];
       const int nring = A.ring_slots * 9;
       for (int k = t; k < nring; k += RM_THREADS) {
-        double* r = A.ring + (size_t)k * A.ring_stride;
+        double* r = A.ring + (size_t)k * ring_stride(A.ring_stride);
         r[i] = r[NP];
       }
       // ---- ReplaceParticleIndexInCell (src/MCells.f90:728-743)
@@ -351,7 +351,7 @@ __global__ void k_ring_restride(const double* __restrict__ src, double* __restri
   for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < total;
        k += (size_t)gridDim.x * blockDim.x) {
     const size_t b = k / nd, i = k - b * nd;
-    dst[k] = src[b * ns + i];
+    dst[b * ring_stride(nd) + i] = src[b * ring_stride(ns) + i];
   }
 }
 
@@ -463,7 +463,7 @@ __global__ void k_ring_widen(const double* __restrict__ src, double* __restrict_
   for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < total;
        k += (size_t)gridDim.x * blockDim.x) {
     const size_t b = k / nd, i = k - b * nd;
-    dst[k] = i < (size_t)ns ? src[b * ns + i] : 0.0;
+    dst[b * ring_stride(nd) + i] = i < (size_t)ns ? src[b * ring_stride(ns) + i] : 0.0;
   }
 }
 

@@ -112,8 +112,8 @@ __global__ void k_slab_max(int* __restrict__ dst, const int* __restrict__ src, i
   if (i < m && src[i] > dst[i]) dst[i] = src[i];
 }
 
-// The "j" results (in_cap slots of `rec` bytes, layout [slot * stride + q])
-// and matched-record bits of the ghosts ids[0..count), one record each:
+// The "j" results (in_cap slots of `rec` bytes per particle, laid out by
+// in_head / in_tail) and matched-record bits of the ghosts ids[0..count), one record each:
 // {q, count, matched, 0, slots...}; the ghosts' counts and bits are reset
 // here (their owner folds them).
 __global__ void k_slab_jhalf_pack(const int* __restrict__ ids, int count, int* __restrict__ in_cnt,
@@ -130,8 +130,12 @@ __global__ void k_slab_jhalf_pack(const int* __restrict__ ids, int count, int* _
   h[3] = 0;
   char* d = (char*)(h + 4);
   for (int e = 0; e < m; e++) {
-    const int* s = (const int*)(in_rec + ((size_t)e * stride + q) * rec);
-    for (int w = 0; w < rec / 4; w++) ((int*)(d + (size_t)e * rec))[w] = s[w];
+    int* o = (int*)(d + (size_t)e * rec);
+    const int* h32 = (const int*)(in_rec + in_head(rec, stride, e, q));
+    const int* t16 = (const int*)(in_rec + in_tail(rec, stride, e, q));
+    const int nh = rec / 4 - 4;
+    for (int w = 0; w < nh; w++) o[w] = h32[w];
+    for (int w = 0; w < 4; w++) o[nh + w] = t16[w];
   }
   in_cnt[q] = 0;
   matched[q] = 0u;
@@ -157,8 +161,12 @@ __global__ void k_slab_jhalf_unpack(const char* __restrict__ buf, int count, int
       atomicExch(&cnt->abort, 1);
       break;
     }
-    int* d = (int*)(in_rec + ((size_t)(base + e) * stride + q) * rec);
-    for (int w = 0; w < rec / 4; w++) d[w] = ((const int*)(s + (size_t)e * rec))[w];
+    const int* r = (const int*)(s + (size_t)e * rec);
+    int* h32 = (int*)(in_rec + in_head(rec, stride, base + e, q));
+    int* t16 = (int*)(in_rec + in_tail(rec, stride, base + e, q));
+    const int nh = rec / 4 - 4;
+    for (int w = 0; w < nh; w++) h32[w] = r[w];
+    for (int w = 0; w < 4; w++) t16[w] = r[nh + w];
   }
   in_cnt[q] = min(base + m, in_cap);
 }

@@ -278,7 +278,7 @@ __device__ __forceinline__ void build_row(const DevParams& P, int n, int p, int 
   const int nx = P.nx, ny = P.ny, nz = P.nz;
   const int cl = c - P.coff;
   const int cx = cl % nx, cy = (cl / nx) % ny, cz = cl / (nx * ny);
-  const double4 p4 = X[p];
+  const double4 p4 = ld32(X + p);
   const int cp = PP ? 0 : comp[p];
   int cw = -1, order = 1 << 20;  // the lane's cell, its place in the row
   bool walk = false;
@@ -314,7 +314,7 @@ __device__ __forceinline__ void build_row(const DevParams& P, int n, int p, int 
   }
   const double skin = P.vl_skin;
   auto is_cand = [&](int q) -> bool {
-    const double4 q4 = X[q];
+    const double4 q4 = ld32(X + q);
     double Rij[3] = {__dsub_rn(q4.x, p4.x), __dsub_rn(q4.y, p4.y), __dsub_rn(q4.z, p4.z)};
 #pragma unroll
     for (int k = 0; k < 3; k++) Rij[k] = min_image_rn(Rij[k], P.box, k);
@@ -505,7 +505,7 @@ __device__ __forceinline__ bool row_stays(const TestArgs& A, int pl, int cl, con
       near = true;
       break;
     }
-    const double4 q4 = A.X[q];
+    const double4 q4 = ld32(A.X + q);
     double Rij[3] = {__dsub_rn(q4.x, p4.x), __dsub_rn(q4.y, p4.y), __dsub_rn(q4.z, p4.z)};
 #pragma unroll
     for (int d = 0; d < 3; d++) Rij[d] = min_image_rn(Rij[d], P.box, d);
@@ -565,7 +565,7 @@ __device__ __forceinline__ void test_body(const TestArgs& A, int vblock) {
   const int cp0 = A.cell_cur[p];
   // (a slab of a decomposition tests only its own particles)
   const bool valid = valid0 && (unsigned)(cp0 - A.slab_c0) < A.slab_span;
-  const double4 p4 = A.X[p];
+  const double4 p4 = ld32(A.X + p);
   const int cp = PP ? 0 : A.comp[p];
   int q0[4];
 #pragma unroll
@@ -631,7 +631,7 @@ __device__ __forceinline__ void test_body(const TestArgs& A, int vblock) {
       double4 xq[4];
 #pragma unroll
       for (int u = 0; u < 4; u++)
-        xq[u] = q[u] >= 0 ? A.X[q[u]] : make_double4(0.0, 0.0, 0.0, 0.0);
+        if (q[u] >= 0) xq[u] = ld32(A.X + q[u]);
 #pragma unroll
       for (int u = 0; u < 4; u++) {
         if (q[u] < 0) continue;
