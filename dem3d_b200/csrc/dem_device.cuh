@@ -143,6 +143,10 @@ constexpr int EPI_CORRECT = 2;  // MoveParticles corrector (pass 2)
 // even number of particles, so that every column starts on 16 bytes.
 __device__ __host__ __forceinline__ size_t ring_stride(int n) { return (size_t)((n + 1) & ~1); }
 
+// contact numbers of 255 and more are kept as 255 in the contact list (the
+// pair kernel then counts from the particle's first contact)
+constexpr int ORD_MAX = 255;
+
 struct RingMap {
   int phys[5];  // phys[k] = physical slot of logical ipc(k+1); phys[nprev] = spare
 };
@@ -341,6 +345,7 @@ struct PassArgs {
   // of each particle's table that a contact matched (bit r: record r); the
   // fold kernel resets the counts and the matched bits
   int2* clist;
+  unsigned char* cord;  // a contact's number among its "i"'s, at most ORD_MAX
   int* cstart;
   int* ccount;
   void* irec;

@@ -671,15 +671,11 @@ __global__ void __launch_bounds__(BS, 7 * 128 / BS) k_test(TestArgs A) {
   for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) test_body<PP>(A, vb);
 }
 
-// record keys read before the record count is known (speculatively, within
-// the table's capacity)
-constexpr int KSPEC = 2;
-
-// The pair kernel (FP64): one thread per contact, grid-stride over the list.
-// (Body for block `vblock` of a grid of `vgrid` blocks.)
+// The pair kernel (FP64): one thread per contact (pair_sweep).  (Body for
+// block `vblock` of a grid of `vgrid` blocks.)
 template <bool PP>
 __device__ __forceinline__ void pair_fp64_body(const PassArgs<double4, double2>& A, int vblock,
-                                               int vgrid) {
+                                               int vgrid, int nseg) {
   __shared__ int s_abort;
   if (threadIdx.x == 0) s_abort = A.cnt->abort;
   __syncthreads();
@@ -695,15 +691,32 @@ __device__ __forceinline__ void pair_fp64_body(const PassArgs<double4, double2>&
   unsigned n_col = 0;
   int need = 0, need_in = 0;
   bool overflow = false, in_over = false;
-  for (int s = vblock * blockDim.x + threadIdx.x; s < total; s += vgrid * blockDim.x) {
-    const int2 e = A.clist[s];
+  // (the record's likely place, the next list entry and its data ahead of
+  // time: see pair_mixed_body)
+  const PairSweep w = pair_sweep(total, vblock, vgrid, nseg);
+  const int stride = w.stride, end = w.end;
+  int s = w.first + threadIdx.x;
+  int2 e = make_int2(0, 0);
+  int ord = 0;
+  if (s < end) {
+    e = A.clist[s];
+    ord = A.cord[s];
+  }
+  while (s < end) {
     const int p = e.x, q = e.y;
     const int s_in = atomicAdd(&A.in_cnt[q], 1);  // q's "j" record (returns early)
-    const int ord = s - A.cstart[p];
+    int2 e2 = e;
+    int ord2 = 0;
+    if (s + stride < end) {
+      e2 = A.clist[s + stride];
+      ord2 = A.cord[s + stride];
+    }
+    if (ord == ORD_MAX) ord = s - A.cstart[p];
     const int hc = A.Hr.cnt[p];
-    int kspec[KSPEC];
-#pragma unroll
-    for (int r = 0; r < KSPEC; r++) kspec[r] = r < A.Hr.cap ? A.Hr.key[hslot(A.Hr, p, r)] : -1;
+    const bool room = ord < A.Hr.cap;
+    const int kg = A.Hr.key[hslot(A.Hr, p, room ? ord : 0)];
+    double FT0[3], VT0[3];
+    hist_read(A.Hr, p, room ? ord : 0, FT0, VT0);
     const DevParams& P = sys_params(A.P, A.sysid, p);
     const double4 p4 = ld32(A.X + p), q4 = ld32(A.X + q);
     const double4 pv4 = ld32(A.v4 + p), qv4 = ld32(A.v4 + q);
@@ -720,26 +733,31 @@ __device__ __forceinline__ void pair_fp64_body(const PassArgs<double4, double2>&
     const double va[3] = {pv4.x, pv4.y, pv4.z}, wa[3] = {pv4.w, pw2.x, pw2.y};
     const double vb[3] = {qv4.x, qv4.y, qv4.z}, wb[3] = {qv4.w, qw2.x, qw2.y};
     // VerifyPairContact: i's records, then j's
-    int r = -1;
-#pragma unroll
-    for (int rr = 0; rr < KSPEC; rr++)
-      if (r < 0 && rr < hc && kspec[rr] == q) r = rr;
-    for (int rr = KSPEC; r < 0 && rr < hc; rr++)
-      if (A.Hr.key[hslot(A.Hr, p, rr)] == q) r = rr;
-    double FT0[3] = {0.0, 0.0, 0.0}, VT0[3] = {0.0, 0.0, 0.0};
+    int r = room && ord < hc && kg == q ? ord : -1;
     bool contacting = r >= 0;
-    if (contacting) {
-      hist_read(A.Hr, p, r, FT0, VT0);
-      if (r < 32) atomicOr(&A.matched[p], 1u << r);
-    } else {
-      const int r2 = find_record(A.Hr, q, p);
-      contacting = r2 >= 0;
-      if (contacting) hist_read(A.Hr, q, r2, FT0, VT0);
+    if (!contacting) {
+      r = find_record(A.Hr, p, q);
+      contacting = r >= 0;
+      if (contacting) {
+        hist_read(A.Hr, p, r, FT0, VT0);
+      } else {
+        const int r2 = find_record(A.Hr, q, p);
+        contacting = r2 >= 0;
+        if (contacting) hist_read(A.Hr, q, r2, FT0, VT0);
+      }
     }
+    // (the fold reads the matched bits of history-updating passes only)
+    if (update && r >= 0 && r < 32) atomicOr(&A.matched[p], 1u << r);
     if (!contacting) n_col++;
     ContactOut out;
     pair_contact(Rij, DijSq, Delta, pp, p4.w, va, wa, q4.w, vb, wb, half_dt, contacting, FT0, VT0,
                  out);
+    if (s + stride < end) {
+      prefetch_l2(A.X + e2.y);
+      prefetch_l2(A.v4 + e2.y);
+      prefetch_l2(A.w2 + e2.y);
+      prefetch_l2(A.in_cnt + e2.y);
+    }
     // "j" half into q's incoming records
     if (s_in < A.in_cap) {
       char* const in = (char*)A.in_rec;
@@ -767,6 +785,9 @@ __device__ __forceinline__ void pair_fp64_body(const PassArgs<double4, double2>&
       else overflow = true;
       need = need > ord + 1 ? need : ord + 1;
     }
+    s += stride;
+    e = e2;
+    ord = ord2;
   }
   if (overflow) {
     atomicExch(&A.cnt->overflow, 1);
@@ -780,9 +801,10 @@ __device__ __forceinline__ void pair_fp64_body(const PassArgs<double4, double2>&
 }
 
 template <bool PP, int MINB>
-__global__ void __launch_bounds__(128, MINB) k_pair_fp64(PassArgs<double4, double2> A) {
+__global__ void __launch_bounds__(128, MINB) k_pair_fp64(PassArgs<double4, double2> A,
+                                                         int nseg) {
   pass_kernel_entry();
-  pair_fp64_body<PP>(A, blockIdx.x, gridDim.x);
+  pair_fp64_body<PP>(A, blockIdx.x, gridDim.x, nseg);
 }
 
 // The fold kernel (FP64): p's block of the sweep, its Force and Torque in
@@ -1056,7 +1078,7 @@ __global__ void __launch_bounds__(128, 4) k_chunk_fp64(const ChunkPass64* __rest
     const int nvb = (sp.t.n + 127) / 128;
     for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) test_body<PP, false>(sp.t, vb);
     if (!grid_sync(g)) return;
-    pair_fp64_body<PP>(sp.a, blockIdx.x, gridDim.x);
+    pair_fp64_body<PP>(sp.a, blockIdx.x, gridDim.x, 1);
     if (!grid_sync(g)) return;
     for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
       if (sp.epi == EPI_PREDICT) fold_fp64_body<PP, EPI_PREDICT, WALLS>(sp.a, vb, stage);

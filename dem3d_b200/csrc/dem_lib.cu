@@ -115,6 +115,7 @@ struct dem_ctx {
   int2* clist = nullptr;
   void* irec = nullptr;
   void* irec9 = nullptr;
+  unsigned char* cord = nullptr;
   int cl_cap = 0;
   int* cstart = nullptr;
   int* ccount = nullptr;
@@ -132,7 +133,10 @@ struct dem_ctx {
   int* rm_buf = nullptr;  // escaped list + status words of the removal kernel
   int rm_cap = 0;
   long long rm_stats[3] = {0, 0, 0};  // removals, swaps, records renamed or moved
-  int pass_variant = 0;  // pair kernel compiled for 4 (0), 3 (1) or 5 (2) blocks per SM
+  // pair kernel compiled for 4 (0), 3 (1) or 5 (2) blocks per SM (FP64), 6, 4
+  // or 8 (mixed: at 5, 90 registers, a launch over 3.3M contacts takes 315 us
+  // against 260 at 6)
+  int pass_variant = 0;
   // launch shape (dem_set_launch_shape): threads per block of the test
   // kernel, particles per thread of the test and fold kernels, the pair
   // kernel's grid in waves of resident blocks, and 4-step chunks as one
@@ -386,6 +390,7 @@ void free_lists(dem_ctx* c) {
   cudaFree(c->clist);
   cudaFree(c->irec);
   cudaFree(c->irec9);
+  cudaFree(c->cord);
   cudaFree(c->cstart);
   cudaFree(c->ccount);
   cudaFree(c->matched);
@@ -395,6 +400,7 @@ void free_lists(dem_ctx* c) {
   c->clist = nullptr;
   c->irec = nullptr;
   c->irec9 = nullptr;
+  c->cord = nullptr;
   c->cstart = nullptr;
   c->ccount = nullptr;
   c->matched = nullptr;
@@ -737,6 +743,7 @@ PassArgs<V4, W2> pass_args(dem_ctx* c, int side, bool update, double dt, const R
   A.amsum = c->amsum;
   A.rank = c->rows.rank;
   A.clist = c->clist;
+  A.cord = c->cord;
   A.cstart = c->cstart;
   A.ccount = c->ccount;
   A.irec = c->irec;
@@ -773,12 +780,15 @@ int alloc_contacts(dem_ctx* c, int cap) {
   cudaFree(c->clist);
   cudaFree(c->irec);
   cudaFree(c->irec9);
+  cudaFree(c->cord);
   c->clist = nullptr;
   c->irec = nullptr;
   c->irec9 = nullptr;
+  c->cord = nullptr;
   const bool mixed = c->precision == DEM_PREC_MIXED;
   const size_t m = (size_t)std::max(cap, 1);
   CK(cudaMalloc(&c->clist, sizeof(int2) * m));
+  CK(cudaMalloc(&c->cord, m));
   CK(cudaMalloc(&c->irec, (mixed ? sizeof(F8) : 2 * sizeof(double4)) * m));
   CK(cudaMalloc(&c->irec9, (mixed ? sizeof(float) : sizeof(double)) * m));
   c->cl_cap = cap;
@@ -902,6 +912,7 @@ void launch_pass_kernel(dem_ctx* c, int side, bool update, double dt, int epi, c
   T.cand = c->rows.cand;
   T.meta = c->rows.meta;
   T.clist = c->clist;
+  T.cord = c->cord;
   T.cstart = c->cstart;
   T.ccount = c->ccount;
   T.cl_cap = c->cl_cap;
@@ -965,8 +976,7 @@ void launch_pass_kernel(dem_ctx* c, int side, bool update, double dt, int epi, c
   }
   const int mb = c->pass_variant == 1 ? 3 : c->pass_variant == 2 ? 5 : 4;
   // the pair kernel loops over the list: pair_waves waves of the blocks its
-  // register budget lets an SM hold (at least mb per SM)
-  const unsigned pair_blocks = (unsigned)(148 * c->pair_waves * std::max(mb, 6));
+  // register budget lets an SM hold
   if (c->precision == DEM_PREC_MIXED) {
     auto A = pass_args<float4, float2>(c, side, update, dt, rm, tag, tgt);
     if (epi == EPI_STORE) A.amsum = c->force_out;
@@ -974,15 +984,16 @@ void launch_pass_kernel(dem_ctx* c, int side, bool update, double dt, int epi, c
       if ((k == 0 && part == 2) || (k == 1 && part == 1)) continue;
       timed(c, k ? "fold_mixed" : "pair_mixed", [&]() {
         mixed_pass(c->M, c->pp, epi, c->pass_variant, walls, c->has_cone, A, c->hcur, c->stream,
-                   k, pair_blocks, c->ppt, early && !c->prof);
+                   k, c->pair_waves, c->ppt, early && !c->prof);
       });  // (timed counts the launch)
     }
     return;
   }
   auto A = pass_args<double4, double2>(c, side, update, dt, rm, tag, tgt);
   if (epi == EPI_STORE) A.amsum = c->force_out;
-#define PAIR_CASE(PPV, MB) \
-  launch_early(c, early, "pair_fp64", k_pair_fp64<PPV, MB>, pair_blocks, 128, A)
+#define PAIR_CASE(PPV, MB)                                                                   \
+  launch_early(c, early, "pair_fp64", k_pair_fp64<PPV, MB>,           \
+               pair_grid(c->n, MB, c->pair_waves), 128, A, c->pair_waves)
   if (part == 2) {
   } else if (mb == 3) {
     if (c->pp) PAIR_CASE(true, 3);

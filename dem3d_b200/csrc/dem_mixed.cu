@@ -249,13 +249,12 @@ __device__ __forceinline__ void rec_write(float4* a, float4* b, float* c, size_t
 // semantics, each contact evaluated once, summation order), FP32 contact
 // arithmetic, FP64 integrator epilogue.
 
-constexpr int KSPEC = 2;  // record keys read before the record count is known
-
-// The pair kernel: one thread per contact, grid-stride over the list.
-// (Body for block `vblock` of a grid of `vgrid` blocks.)
+// The pair kernel: one thread per contact (pair_sweep).  (Body for block
+// `vblock` of a grid of `vgrid` blocks.)
 template <bool PP>
 __device__ __forceinline__ void pair_mixed_body(const PassArgs<float4, float2>& A,
-                                                const MixedView& V, int vblock, int vgrid) {
+                                                const MixedView& V, int vblock, int vgrid,
+                                                int nseg) {
   __shared__ int s_abort;
   if (threadIdx.x == 0) s_abort = A.cnt->abort;
   __syncthreads();
@@ -273,27 +272,36 @@ __device__ __forceinline__ void pair_mixed_body(const PassArgs<float4, float2>& 
   unsigned n_col = 0;
   int need = 0, need_in = 0;
   bool overflow = false, in_over = false;
-  const int stride = vgrid * blockDim.x;
-  for (int s = vblock * blockDim.x + threadIdx.x; s < total; s += stride) {
-    const int2 e = A.clist[s];
+  // A contact's pair record is nearly always at the contact's own number
+  // among i's (the table is written in that order and contacts last for many
+  // passes), so that slot is read together with the particles' data; the
+  // next contact's list entry is read a turn ahead, and its partner's data
+  // requested into L2 before this one's results are written.
+  const PairSweep w = pair_sweep(total, vblock, vgrid, nseg);
+  const int stride = w.stride, end = w.end;
+  int s = w.first + threadIdx.x;
+  int2 e = make_int2(0, 0);
+  int ord = 0;
+  if (s < end) {
+    e = A.clist[s];
+    ord = A.cord[s];
+  }
+  while (s < end) {
     const int p = e.x, q = e.y;
-    // the next contact of this thread: its pair's data requested into L2
-    // now, so that the next iteration's gathers overlap this one's work
-    if (s + stride < total) {
-      const int2 e2 = A.clist[s + stride];
-      prefetch_l2(A.X + e2.x);
-      prefetch_l2(A.X + e2.y);
-      prefetch_l2(A.v4 + e2.x);
-      prefetch_l2(A.v4 + e2.y);
-      prefetch_l2(Hr.key + e2.x);
-      prefetch_l2(A.in_cnt + e2.y);
-    }
     const int s_in = atomicAdd(&A.in_cnt[q], 1);  // q's "j" record (returns early)
-    const int ord = s - A.cstart[p];
+    int2 e2 = e;
+    int ord2 = 0;
+    if (s + stride < end) {
+      e2 = A.clist[s + stride];
+      ord2 = A.cord[s + stride];
+    }
+    if (ord == ORD_MAX) ord = s - A.cstart[p];
     const int hc = Hr.cnt[p];
-    int kspec[KSPEC];
-#pragma unroll
-    for (int r = 0; r < KSPEC; r++) kspec[r] = r < Hr.cap ? Hr.key[hslot(Hr, p, r)] : -1;
+    const bool room = ord < Hr.cap;
+    const size_t hg = hslot(Hr, p, room ? ord : 0);
+    const int kg = Hr.key[hg];
+    F3 ft0, ft0lo, vt0;
+    rec_read(V.ra, V.rb, V.rc, hg, ft0, ft0lo, vt0);
     const DevParams& P = sys_params(A.P, A.sysid, p);
     const double4 p4 = ld32(A.X + p), q4 = ld32(A.X + q);
     const float4 pv4 = A.v4[p], qv4 = A.v4[q];
@@ -310,27 +318,32 @@ __device__ __forceinline__ void pair_mixed_body(const PassArgs<float4, float2>& 
     const F3 vo = mk(pv4.x, pv4.y, pv4.z), wo = mk(pv4.w, pw2.x, pw2.y);
     const F3 vq = mk(qv4.x, qv4.y, qv4.z), wq = mk(qv4.w, qw2.x, qw2.y);
     // i's records, then j's
-    int r = -1;
-#pragma unroll
-    for (int rr = 0; rr < KSPEC; rr++)
-      if (r < 0 && rr < hc && kspec[rr] == q) r = rr;
-    for (int rr = KSPEC; r < 0 && rr < hc; rr++)
-      if (Hr.key[hslot(Hr, p, rr)] == q) r = rr;
-    F3 ft0 = mk(0.f, 0.f, 0.f), ft0lo = ft0, vt0 = ft0;
+    int r = room && ord < hc && kg == q ? ord : -1;
     bool contacting = r >= 0;
-    if (contacting) {
-      rec_read(V.ra, V.rb, V.rc, hslot(Hr, p, r), ft0, ft0lo, vt0);
-      if (r < 32) atomicOr(&A.matched[p], 1u << r);
-    } else {
-      const int r2 = find_record(Hr, q, p);
-      contacting = r2 >= 0;
-      if (contacting) rec_read(V.ra, V.rb, V.rc, hslot(Hr, q, r2), ft0, ft0lo, vt0);
+    if (!contacting) {
+      r = find_record(Hr, p, q);
+      contacting = r >= 0;
+      if (contacting) {
+        rec_read(V.ra, V.rb, V.rc, hslot(Hr, p, r), ft0, ft0lo, vt0);
+      } else {
+        const int r2 = find_record(Hr, q, p);
+        contacting = r2 >= 0;
+        if (contacting) rec_read(V.ra, V.rb, V.rc, hslot(Hr, q, r2), ft0, ft0lo, vt0);
+      }
     }
+    // (the fold reads the matched bits of history-updating passes only)
+    if (update && r >= 0 && r < 32) atomicOr(&A.matched[p], 1u << r);
     if (!contacting) n_col++;
     MOut out;
     mixed_pair(Rij, DijSq, Delta, m, Ra, vo, wo, Rb, vq, wq, half_dt, contacting, ft0, ft0lo,
                vt0, out);
     const F3 FTs = out.FT + out.FTlo;
+    if (s + stride < end) {
+      prefetch_l2(A.X + e2.y);
+      prefetch_l2(A.v4 + e2.y);
+      prefetch_l2(A.w2 + e2.y);
+      prefetch_l2(A.in_cnt + e2.y);
+    }
     // "j" half into q's incoming records
     if (s_in < A.in_cap) {
       const unsigned long long key = sweep_key(A.cell_cur[p], A.rank[p]);
@@ -359,6 +372,9 @@ __device__ __forceinline__ void pair_mixed_body(const PassArgs<float4, float2>& 
       }
       need = need > ord + 1 ? need : ord + 1;
     }
+    s += stride;
+    e = e2;
+    ord = ord2;
   }
   if (overflow) {
     atomicExch(&A.cnt->overflow, 1);
@@ -373,9 +389,9 @@ __device__ __forceinline__ void pair_mixed_body(const PassArgs<float4, float2>& 
 
 template <bool PP, int MINB>
 __global__ void __launch_bounds__(128, MINB) k_pair_mixed(PassArgs<float4, float2> A,
-                                                          MixedView V) {
+                                                          MixedView V, int nseg) {
   pass_kernel_entry();
-  pair_mixed_body<PP>(A, V, blockIdx.x, gridDim.x);
+  pair_mixed_body<PP>(A, V, blockIdx.x, gridDim.x, nseg);
 }
 
 // The fold kernel: p's block of the sweep, Force and Torque in sweep order
@@ -634,7 +650,7 @@ __global__ void __launch_bounds__(128, 4) k_chunk_mixed(const ChunkPassMx* __res
     const int nvb = (sp.t.n + 127) / 128;
     for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) test_body<PP, false>(sp.t, vb);
     if (!grid_sync(g)) return;
-    pair_mixed_body<PP>(sp.a, sp.v, blockIdx.x, gridDim.x);
+    pair_mixed_body<PP>(sp.a, sp.v, blockIdx.x, gridDim.x, 1);
     if (!grid_sync(g)) return;
     for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
       if (sp.epi == EPI_PREDICT) fold_mixed_body<PP, EPI_PREDICT, WALLS, CONE>(sp.a, sp.v, vb, stage);
@@ -838,11 +854,13 @@ MixedView mixed_view(const MixedBuffers& M, int cur) {
 
 void mixed_pass(MixedBuffers& M, bool pp, int epi, int variant, bool walls, bool cone,
                 const PassArgs<float4, float2>& A, int cur, cudaStream_t st, int part,
-                unsigned pair_blocks, int ppt, bool early) {
+                int pair_waves, int ppt, bool early) {
   if (A.n == 0) return;
   const MixedView V = mixed_view(M, cur);
   if (part == 0) {
-#define PCASE(PPV, MB) launch_pass(early, k_pair_mixed<PPV, MB>, pair_blocks, 128, st, A, V)
+#define PCASE(PPV, MB)                                                                    \
+  launch_pass(early, k_pair_mixed<PPV, MB>, pair_grid(A.n, MB, pair_waves), 128, st, A, V, \
+              pair_waves)
     if (variant == 1) {
       if (pp) PCASE(true, 4);
       else PCASE(false, 4);

@@ -50,8 +50,8 @@ bool mixed_regrow(MixedBuffers& M, int n, int stride, int newcap, int cur, const
 // the wall records of the first n particles into arrays for `stride` rows
 bool mixed_grow_walls(MixedBuffers& M, int n, int stride, int cur, cudaStream_t st);
 // One kernel of a force pass (FP32 contact arithmetic) on the context's
-// stream: part 0 = the pair kernel (pair_blocks blocks of 128 threads over
-// the contact list; variant: compiled for 4 (0), 3 (1) or 5 (2) resident
+// stream: part 0 = the pair kernel (pair_waves waves of blocks of 128 threads
+// over the contact list; variant: compiled for 6 (0), 4 (1) or 8 (2) resident
 // blocks per SM), 1 = the fold kernel with epilogue `epi` (walls: some
 // system has walls; cone: some wall is a cone; ppt > 1: the fold grid holds
 // 1/ppt of the blocks of 128 particles and strides over them; early: launched
@@ -59,7 +59,7 @@ bool mixed_grow_walls(MixedBuffers& M, int n, int stride, int cur, cudaStream_t 
 // contact list is shared with the FP64 path.
 void mixed_pass(MixedBuffers& M, bool pp, int epi, int variant, bool walls, bool cone,
                 const PassArgs<float4, float2>& A, int cur, cudaStream_t st, int part,
-                unsigned pair_blocks, int ppt, bool early);
+                int pair_waves, int ppt, bool early);
 // One persistent chunk (npass passes of prog, a device array) as a
 // cooperative launch of at most want_blocks blocks of 128 threads (fewer if
 // fewer fit on the device at once; the count in *blocks_out).  g.expected

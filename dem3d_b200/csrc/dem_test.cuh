@@ -463,6 +463,7 @@ struct TestArgs {
   const int* cand;
   const int* meta;
   int2* clist;
+  unsigned char* cord;
   int* cstart;
   int* ccount;
   int cl_cap;
@@ -690,7 +691,9 @@ __device__ __forceinline__ void test_body(const TestArgs& A, int vblock) {
       while (mask) {
         const int k = base + __ffsll((long long)mask) - 1;
         mask &= mask - 1ull;
-        A.clist[s++] = make_int2(p, ld_row<NC>(A.cand + (size_t)k * n + p));
+        A.clist[s] = make_int2(p, ld_row<NC>(A.cand + (size_t)k * n + p));
+        const int o = s - start;
+        A.cord[s++] = (unsigned char)(o < ORD_MAX ? o : ORD_MAX);
       }
     }
   }
