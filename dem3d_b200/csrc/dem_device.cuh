@@ -167,13 +167,12 @@ struct CellLists {
   int* dflag;     // [ncell] cell already in a dirty list
   int* rflag;     // [ncell] stamp: pass_id + 1 when the cell's rows are rebuilt in that pass
   int* dlist[2];  // [ncell] cells that gain or lose a particle on the way to assignment b
-  int* rlist;     // [ncell] (unused: the stamps replace a repair list)
   // the particles that left or entered a cell in the relink of the pass
-  // with stamp s: mlist[(s & 1) * mcap + k], k < Counters::n_mlist[s & 1]
-  // (more than mcap: not all recorded); dstamp[c] = s when that relink
-  // rewrote cell c's list
-  int* mlist;
-  int* dstamp;
+  // with stamp s, each with that cell: mlist[(s & 1) * mcap + k], k <
+  // Counters::n_mlist[s & 1] (more than mcap: not all recorded); rstamp[p] = s
+  // when a warp of that pass has taken p's row to rebuild it
+  int2* mlist;
+  int* rstamp;
   int mcap;
   // each cell's list copied in order into SLOT_CAP slots ([cell*SLOT_CAP +
   // k]) and its length (slot_n > SLOT_CAP: only the first SLOT_CAP are
@@ -186,9 +185,9 @@ struct CellLists {
   // stored in the reference's order
   const int* gid;
 };
-constexpr int SLOT_CAP = 32;
-// movers one relink records for the test kernel's row check (more: every
-// stamped row is rebuilt)
+constexpr int SLOT_CAP = 64;
+// movers one relink records for the row kernel (more: every stamped row is
+// rebuilt)
 constexpr int MLIST_CAP = 4096;
 
 // Candidate rows, column-major (cand[k*n + p]): the particles within

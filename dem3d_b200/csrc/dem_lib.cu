@@ -193,6 +193,7 @@ struct dem_ctx {
   bool has_cone = false; // some wall of some system is a cone
   double skin_factor = 0.05;  // candidate-row skin / CutOff
   int par = 0;         // L.cell[par] is the assignment the lists hold
+  bool rows_done = false;  // the relink's launch built the pass's rows too
   int prepared = -1;   // side whose copies + next assignment are ready (-1: none)
   int last_side = -1;  // side of the last pass (its copies are intact)
 
@@ -374,8 +375,9 @@ unsigned blocks_for(long long n, int b) { return (unsigned)((n + b - 1) / b); }
 void free_lists(dem_ctx* c) {
   CellLists& L = c->L;
   int** f[] = {&L.head,  &L.next,  &L.cell[0], &L.cell[1], &L.arr_head, &L.arr_next, &L.mflag,
-               &L.mnext, &L.dflag, &L.rflag,   &L.dlist[0], &L.dlist[1],  &L.rlist,
-               &L.slot,  &L.slot_n, &L.mlist, &L.dstamp};
+               &L.mnext, &L.dflag, &L.rflag,   &L.dlist[0], &L.dlist[1],
+               &L.slot,  &L.slot_n, &L.rstamp};
+  cudaFree(L.mlist);
   for (int** q : f) {
     cudaFree(*q);
     *q = nullptr;
@@ -594,6 +596,8 @@ int grow_capacity(dem_ctx* c, int newcap) {
   CK(fresh(L.arr_next, N, n));
   CK(fresh(L.mflag, N, n));
   CK(fresh(L.mnext, N, n));
+  CK(fresh(L.rstamp, N, 0));
+  CK(cudaMemsetAsync(L.rstamp, 0, sizeof(int) * N, c->stream));
   CK(fresh(c->rows.cand, N * (size_t)c->rows.kc, 0));
   CK(fresh(c->rows.meta, N, 0));
   CK(cudaMemsetAsync(c->rows.meta, 0, sizeof(int) * N, c->stream));
@@ -643,7 +647,11 @@ StateArrays make_state(double* base, size_t n) {
 // ---------------------------------------------------------------------------
 // K1: initial distribution (DistributeParticles3D) of the Particle positions
 
-constexpr int LIST_BLOCKS = 148;      // relink / repair kernels (grid-stride)
+constexpr int LIST_BLOCKS = 148;   // relink and list kernels (grid-stride)
+constexpr int ROWS_BLOCKS = 148 * 4;  // row kernel (grid-stride, 4 warps each)
+// systems whose relink and rows are one launch of one cluster: its 64 warps
+// rebuild this many rows at once in about a launch's time
+constexpr int MERGED_LISTS_MAX = 16384;
 
 // the slots of every cell from its list (after the lists were built or
 // changed outside the relink: initial distribution, imported lists, removal,
@@ -661,7 +669,6 @@ int init_cells(dem_ctx* c) {
   CK(cudaMemsetAsync(L.arr_head, 0xFF, sizeof(int) * (size_t)ncell, c->stream));
   CK(cudaMemsetAsync(L.dflag, 0, sizeof(int) * (size_t)ncell, c->stream));
   CK(cudaMemsetAsync(L.rflag, 0, sizeof(int) * (size_t)ncell, c->stream));
-  CK(cudaMemsetAsync(L.dstamp, 0, sizeof(int) * (size_t)ncell, c->stream));
   if (n > 0) CK(cudaMemsetAsync(L.mflag, 0, sizeof(int) * (size_t)n, c->stream));
   CK(cudaMemsetAsync(c->cell_cnt, 0, sizeof(int) * (size_t)ncell, c->stream));
   if (n > 0) {
@@ -888,18 +895,9 @@ void fluid_prepare(dem_ctx* c, int side) {
          (const Counters*)c->cnt);
 }
 
-// part: 0 = the whole pass, 1 = the test and pair kernels, 2 = the fold
-// kernel (a slab of a decomposition exchanges data in between)
-// early_ok: the operation ahead of this pass's test kernel in the stream is
-// the pass's relink (or a fluid kernel after it), so the test, pair and fold
-// kernels may be launched early; not after the status resets of a repeated
-// pass, nor between the exchanges of a slab
-void launch_pass_kernel(dem_ctx* c, int side, bool update, double dt, int epi, const RingMap& rm,
-                        int tag, int part = 0, bool early_ok = true) {
-  if (c->n == 0) return;
-  const bool early = early_ok && c->early_launch && !c->slab && part == 0;
-  const StateArrays& tgt = side ? c->Pr : c->P;
-  // the test kernel: the contact list of the pass
+// the row and the test kernel of the pass on `side` (after its relink: c->par
+// is the pass's assignment)
+TestArgs test_args(dem_ctx* c, int side, int tag) {
   TestArgs T;
   T.P = c->dp;
   T.sysid = c->sysid;
@@ -921,6 +919,21 @@ void launch_pass_kernel(dem_ctx* c, int side, bool update, double dt, int epi, c
   T.slab_c0 = c->slab ? c->hsys[0].slab_c0 : 0;
   T.slab_span = c->slab ? (unsigned)(c->hsys[0].slab_c1 - c->hsys[0].slab_c0) : 0xffffffffu;
   T.fine = c->slab ? 0 : 1;  // (a slab's stamps of its ghost layer come by exchange)
+  return T;
+}
+
+// part: 0 = the whole pass, 1 = the test and pair kernels, 2 = the fold
+// kernel (a slab of a decomposition exchanges data in between)
+// early_ok: the operation ahead of this pass's test kernel in the stream is
+// the pass's relink (or a fluid kernel after it), so the test, pair and fold
+// kernels may be launched early; not after the status resets of a repeated
+// pass, nor between the exchanges of a slab
+void launch_pass_kernel(dem_ctx* c, int side, bool update, double dt, int epi, const RingMap& rm,
+                        int tag, int part = 0, bool early_ok = true) {
+  if (c->n == 0) return;
+  const bool early = early_ok && c->early_launch && !c->slab && part == 0;
+  const StateArrays& tgt = side ? c->Pr : c->P;
+  const TestArgs T = test_args(c, side, tag);
   const bool walls = c->nw_max > 0;
   if (c->recording) {
     // a pass of a persistent chunk: appended, not launched
@@ -948,9 +961,16 @@ void launch_pass_kernel(dem_ctx* c, int side, bool update, double dt, int epi, c
     }
     return;
   }
-  // test kernel: test_block threads per block; with ppt > 1 the grid holds
-  // 1/ppt of the blocks and strides over them
+  // row kernel (unless the relink's launch built the rows too), then the test
+  // kernel: test_block threads per block; with ppt > 1 the grid holds 1/ppt of
+  // the blocks and strides over them
   if (part != 2) {
+    if (!c->rows_done) {
+      const unsigned rb = std::min<unsigned>((unsigned)ROWS_BLOCKS, blocks_for(c->n, 4));
+      if (c->pp) launch_early(c, early, "rows", k_rows<true>, rb, 128u, T);
+      else launch_early(c, early, "rows", k_rows<false>, rb, 128u, T);
+    }
+    c->rows_done = false;
     const int bs = c->test_block;
     const unsigned nvb = blocks_for(c->n, bs);
     const bool stride = c->ppt > 1;
@@ -1067,17 +1087,24 @@ int prepare_side(dem_ctx* c, int side) {
 
 // relink towards the prepared assignment (the candidate rows around the
 // relinked cells are rebuilt by the test kernel)
-void pass_lists(dem_ctx* c, int side, bool update, int tag) {
-  (void)side;
+void pass_lists(dem_ctx* c, int side, bool update, int tag, bool early) {
+  early = early && c->early_launch && !c->slab;
   const int b = c->par ^ 1;
   const int stop_tag = c->capturing && c->stop_on_escape && update ? tag : -1;
-  if (c->recording) {
-    c->rec_rl = RelinkArgs{c->dp, c->cellsys, c->L, b, c->n, update ? 1 : 0, stop_tag, c->cnt};
-  } else {
-    launch(c, "relink", k_relink, (unsigned)LIST_BLOCKS, 256, (const DevParams*)c->dp,
-           (const int*)c->cellsys, c->L, b, c->n, update ? 1 : 0, stop_tag, c->cnt);
-  }
+  const RelinkArgs R{c->dp, c->cellsys, c->L, b, c->n, update ? 1 : 0, stop_tag, c->cnt};
   c->par = b;
+  if (c->recording) {
+    c->rec_rl = R;
+    return;
+  }
+  if (!c->slab && c->n > 0 && c->n <= MERGED_LISTS_MAX) {
+    const TestArgs T = test_args(c, side, tag);
+    if (c->pp) launch_early(c, early, "lists", k_lists<true>, 8u, (unsigned)LIST_THREADS, R, T);
+    else launch_early(c, early, "lists", k_lists<false>, 8u, (unsigned)LIST_THREADS, R, T);
+    c->rows_done = true;
+    return;
+  }
+  launch_early(c, early, "relink", k_relink, (unsigned)LIST_BLOCKS, (unsigned)LIST_THREADS, R);
 }
 
 RingMap current_map(dem_ctx* c) {
@@ -1218,7 +1245,10 @@ int force_pass(dem_ctx* c, int side, bool update, double dt, int epi, const Ring
     int st = prepare_side(c, side);
     if (st) return st;
   }
-  pass_lists(c, side, update, tag);
+  // the relink follows the previous pass's fold kernel directly in a captured
+  // chunk without moving walls (their copies lie in between), but for its
+  // first pass: it may then be launched early, too
+  pass_lists(c, side, update, tag, c->capturing && tag > 0 && c->wm.empty());
   fluid_prepare(c, side);
   launch_pass_kernel(c, side, update, dt, epi, rm, tag);
   cudaError_t e = cudaGetLastError();
@@ -2508,14 +2538,13 @@ int dem_set_state(dem_ctx* c, int32_t n, const int32_t* comp, const double* radi
     CK(cudaMalloc(&L.rflag, sizeof(int) * NC));
     CK(cudaMalloc(&L.dlist[0], sizeof(int) * NC));
     CK(cudaMalloc(&L.dlist[1], sizeof(int) * NC));
-    CK(cudaMalloc(&L.rlist, sizeof(int) * NC));
     CK(cudaMalloc(&L.slot, sizeof(int) * NC * SLOT_CAP));
     CK(cudaMalloc(&L.slot_n, sizeof(int) * NC));
     CK(cudaMemsetAsync(L.slot_n, 0xFF, sizeof(int) * NC, c->stream));
     L.mcap = MLIST_CAP;
-    CK(cudaMalloc(&L.mlist, sizeof(int) * 2 * (size_t)MLIST_CAP));
-    CK(cudaMalloc(&L.dstamp, sizeof(int) * NC));
-    CK(cudaMemsetAsync(L.dstamp, 0, sizeof(int) * NC, c->stream));
+    CK(cudaMalloc(&L.mlist, sizeof(int2) * 2 * (size_t)MLIST_CAP));
+    CK(cudaMalloc(&L.rstamp, sizeof(int) * N));
+    CK(cudaMemsetAsync(L.rstamp, 0, sizeof(int) * N, c->stream));
     CK(cudaMalloc(&c->rows.cand, sizeof(int) * N * (size_t)c->kc));
     CK(cudaMalloc(&c->rows.meta, sizeof(int) * N));
     CK(cudaMemsetAsync(c->rows.meta, 0, sizeof(int) * N, c->stream));
@@ -3841,7 +3870,7 @@ int dem_slab_phase(dem_ctx* c, int32_t step, int32_t pass, int32_t phase) {
       }
       c->gepoch++;
       c->n_ghosts = 0;
-      pass_lists(c, side, update, pass);
+      pass_lists(c, side, update, pass, false);
       break;
     case DEM_SLAB_TEST_PAIR:
       launch_pass_kernel(c, side, update, dt, epi, c->slab_rm, pass, 1);

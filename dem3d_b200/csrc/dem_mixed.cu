@@ -640,15 +640,21 @@ __global__ void __launch_bounds__(128, 4) k_chunk_mixed(const ChunkPassMx* __res
                                                         int npass, GridSync g) {
   __shared__ ChunkPassMx sp;
   __shared__ __align__(16) double stage[EpiStage<EPI_PREDICT, true>::SIZE];  // (the larger of the two)
-  const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-  const int nthreads = gridDim.x * blockDim.x;
+  // (the relink's and the test's shared arrays lie in the fold's columns)
+  int(*const sh)[RELINK_ROOM] = reinterpret_cast<int(*)[RELINK_ROOM]>(stage);
+  TestWarp* const warps = reinterpret_cast<TestWarp*>(stage);
+  static_assert(sizeof(stage) >= 4 * sizeof(TestWarp) && sizeof(stage) >= 4 * RELINK_ROOM * 4,
+                "shared arrays of the phases");
+  const int gwarp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int nwarps = gridDim.x * (blockDim.x >> 5);
   for (int k = 0; k < npass; k++) {
     load_pass(sp, prog + k);
-    const RelinkArgs& R = sp.rl;
-    relink_body(R.PT, R.cellsys, R.L, R.par, R.n, R.update, R.stop_tag, R.cnt, tid, nthreads);
+    chunk_relink(sp, gwarp, nwarps, sh[threadIdx.x >> 5]);
+    if (!grid_sync(g)) return;
+    chunk_rows<PP>(sp, gwarp, nwarps);
     if (!grid_sync(g)) return;
     const int nvb = (sp.t.n + 127) / 128;
-    for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) test_body<PP, false>(sp.t, vb);
+    chunk_test<PP>(sp, warps);
     if (!grid_sync(g)) return;
     pair_mixed_body<PP>(sp.a, sp.v, blockIdx.x, gridDim.x, 1);
     if (!grid_sync(g)) return;

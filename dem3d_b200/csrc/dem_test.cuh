@@ -20,6 +20,10 @@ __device__ __forceinline__ double min_image_rn(double r, const Box& B, int k) {
     r = __dsub_rn(r, __dmul_rn(B.lbox[k], (double)(int)round(__dmul_rn(r, B.inv_lbox[k]))));
   return r;
 }
+// the image itself, for a component known to be beyond the shortcut's bound
+__device__ __forceinline__ double image_rn(double r, const Box& B, int k) {
+  return __dsub_rn(r, __dmul_rn(B.lbox[k], (double)(int)round(__dmul_rn(r, B.inv_lbox[k]))));
+}
 __device__ __forceinline__ double sumsq3_rn(const double a[3]) {
   double c = 0.0;
   c = __dadd_rn(c, __dmul_rn(a[0], a[0]));
@@ -54,21 +58,97 @@ __device__ __forceinline__ void copy_slots(const CellLists& L, int c, int first,
   L.slot_n[c] = k;
 }
 
+// The o-th (0 <= o < 14) of the cells whose particles' rows read cell c: c
+// itself (o = 13) and c + o' for the 13 offsets with kx + Nx*(ky + Ny*kz) < 0;
+// -1: off the grid.
+__device__ __forceinline__ int reading_cell(const DevParams& P, int c, int o) {
+  const int nx = P.nx, ny = P.ny, nz = P.nz;
+  int cx, cy, cz;
+  cell_coords(P, c, cx, cy, cz);
+  const int jx = cx + o % 3 - 1, jy = cy + (o / 3) % 3 - 1, jz = cz + o / 9 - 1;
+  const bool ok = (P.pbc[0] || (jx >= 0 && jx < nx)) && (P.pbc[1] || (jy >= 0 && jy < ny)) &&
+                  (P.pbc[2] || (jz >= 0 && jz < nz));
+  if (!ok) return -1;
+  return P.coff + axis_wrap(jx, nx, P.pbc[0]) +
+         nx * (axis_wrap(jy, ny, P.pbc[1]) + ny * axis_wrap(jz, nz, P.pbc[2]));
+}
+
+// The rewrite of a cell whose list does not fit the slots, by one thread: the
+// old list is walked link by link (a leaver's successor was saved when it
+// moved, mnext: its own link may be rewritten by the warp of the cell it
+// entered), the leavers dropped, the arrivals prepended in decreasing index.
+template <class Rec, class Gid>
+__device__ __forceinline__ bool relink_links(const CellLists& L, const int* cell_new, int c,
+                                             int n, Rec&& record, Gid&& G) {
+  int prev = -1, first = -1, guard = 0;
+  int q = L.head[c];
+  while (q != -1) {
+    if (++guard > n) return false;
+    const bool stays = cell_new[q] == c;
+    const int nq = stays ? L.next[q] : L.mnext[q];
+    if (!stays) {
+      record(q);
+    } else {
+      if (prev == -1) first = q;
+      else L.next[prev] = q;
+      prev = q;
+    }
+    q = nq;
+  }
+  if (prev != -1) L.next[prev] = -1;
+  int sh = -1, tail = -1, a = L.arr_head[c];
+  guard = 0;
+  while (a != -1) {
+    if (++guard > n) return false;
+    const int an = L.arr_next[a];  // (guard: arrivals so far)
+    L.mflag[a] = 0;
+    record(a);
+    if (sh == -1) {
+      sh = tail = a;
+      L.next[a] = -1;
+    } else if (G(a) > G(sh)) {
+      L.next[a] = sh;
+      sh = a;
+    } else {
+      int q2 = sh;
+      for (int g2 = 0; L.next[q2] != -1 && G(L.next[q2]) > G(a) && g2 < guard; g2++)
+        q2 = L.next[q2];
+      L.next[a] = L.next[q2];
+      L.next[q2] = a;
+      if (L.next[a] == -1) tail = a;
+    }
+    a = an;
+  }
+  if (sh != -1) {
+    L.next[tail] = first;
+    first = sh;
+  }
+  L.head[c] = first;
+  copy_slots(L, c, first, n);
+  return true;
+}
+
 // Relink (RedistributeParticles3D's list updates, src/MCells.f90:607-643):
-// one thread per dirty cell of list `par` drops the particles that left it
+// one warp per dirty cell of list `par` drops the particles that left it
 // (TransferParticle's unlink, :747-774) and prepends its arrivals in
 // decreasing index (AddParticle, :684-698, applied in increasing index
-// order), then marks its 27-cell neighbourhood for candidate-row repair.
-// The walk over the old list follows a leaver's successor saved when it
-// moved (mnext), so no thread reads a link that another thread rewrites.
+// order), records the movers with the cell, and stamps the 14 cells whose
+// rows read it.  The lanes hold the old list (from the cell's slots) and the
+// arrivals side by side, so a cell costs four round trips to memory and not
+// one per element; the kernel is bound by those round trips (14 us per launch
+// at 1M spheres with one thread per cell and its list in local memory).
 // Thread 0 also closes the previous pass's bookkeeping and decides whether
 // this pass rebuilds every candidate row.
-// (The body of k_relink; tid / nthreads: this thread's index in the grid and
-// the grid's thread count, so that a persistent kernel can run it too.)
+// (The body of k_relink; warp / nwarps: this warp's index among the warps
+// that share the work, `sh` RELINK_ROOM ints of shared memory of its own.)
+constexpr int RELINK_ROOM = SLOT_CAP + 32;
 __device__ __forceinline__ void relink_body(const DevParams* __restrict__ PT,
                                             const int* __restrict__ cellsys, const CellLists& L,
                                             int par, int n, int update, int stop_tag,
-                                            Counters* cnt, int tid, int nthreads) {
+                                            Counters* cnt, int warp, int nwarps, int* sh) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const bool first_thread = warp == 0 && lane == 0;
   // (the status words, the dirty-cell count and the pass number requested
   // together)
   const int abort0 = cnt->abort;
@@ -81,13 +161,13 @@ __device__ __forceinline__ void relink_body(const DevParams* __restrict__ PT,
   // count is final here (written by the previous kernel), so every block
   // takes the same branch
   if (stop_tag >= 0 && escaped != 0ull) {
-    if (tid == 0) {
+    if (first_thread) {
       cnt->escape_stop = 1;
       set_abort(cnt, stop_tag);
     }
     return;
   }
-  if (tid == 0) {
+  if (first_thread) {
     const DevParams& P = PT[0];  // the integrator settings are shared
     cnt->n_repair = 0;
     cnt->n_mlist[(stamp & 1) ^ 1] = 0;  // for the next pass's relink
@@ -116,152 +196,107 @@ __device__ __forceinline__ void relink_body(const DevParams* __restrict__ PT,
     cnt->disp_acc = full ? 0.0 : acc;
     if (full) cnt->force_full = 0;
   }
-  const int* __restrict__ cell_new = L.cell[par];
-  // a particle that leaves or enters a cell, for the test kernel's row check
-  auto record = [&](int x) {
-    const int k = atomicAdd(&cnt->n_mlist[stamp & 1], 1);
-    if (k < L.mcap) L.mlist[(size_t)(stamp & 1) * L.mcap + k] = x;
-  };
-  for (int i = tid; i < m; i += nthreads) {
+  const int* cell_new = L.cell[par];
+  // the reference's index (gid when the storage is in cell order)
+  auto G = [&](int x) { return L.gid ? L.gid[x] : x; };
+  for (int i = warp; i < m; i += nwarps) {
     const int c = L.dlist[par][i];
+    const int len = L.slot_n[c];
+    const int ah = L.arr_head[c];
+    const int* sl = L.slot + (size_t)c * SLOT_CAP;
+    const int e0 = lane < len && len <= SLOT_CAP ? sl[lane] : -1;
+    const int e1 = lane + 32 < len && len <= SLOT_CAP ? sl[lane + 32] : -1;
     const DevParams& P = sys_params(PT, cellsys, c);
     if (!in_slab(P, c)) {
       // a cell another slab advances (a particle of this slab left for it):
       // its list here is not kept; only the transition is forgotten
-      for (int a = L.arr_head[c], g2 = 0; a != -1 && g2 < n; a = L.arr_next[a], g2++)
-        L.mflag[a] = 0;
-      L.arr_head[c] = -1;
-      L.dflag[c] = 0;
+      if (lane == 0) {
+        for (int a = ah, g2 = 0; a != -1 && g2 < n; a = L.arr_next[a], g2++) L.mflag[a] = 0;
+        L.arr_head[c] = -1;
+        L.dflag[c] = 0;
+      }
       continue;
     }
-    // 1. unlink the leavers.  The old list is in the cell's slots when it
-    // fits there (independent loads); else it is walked link by link (a
-    // leaver's successor saved when it moved: its own link may be rewritten
-    // by the thread of the cell it entered)
-    int prev = -1, first = -1;
-    int guard = 0;
-    const int len = L.slot_n[c];
-    const bool from_slots = len >= 0 && len <= SLOT_CAP;
-    int old[SLOT_CAP];
-    unsigned stay = 0u;  // bit k: old element k stays
-    if (from_slots) {
-      const int* sl = L.slot + (size_t)c * SLOT_CAP;
-#pragma unroll 4
-      for (int k = 0; k < len; k++) old[k] = sl[k];
-#pragma unroll 4
-      for (int k = 0; k < len; k++)
-        if (cell_new[old[k]] == c) stay |= 1u << k;
-      for (int k = 0; k < len; k++) {
-        if (!((stay >> k) & 1u)) {
-          record(old[k]);
-          continue;
-        }
-        if (prev == -1) first = old[k];
-        else L.next[prev] = old[k];
-        prev = old[k];
+    // a particle that leaves or enters the cell, for the row kernel
+    auto record = [&](int x) {
+      const int k = atomicAdd(&cnt->n_mlist[stamp & 1], 1);
+      if (k < L.mcap) L.mlist[(size_t)(stamp & 1) * L.mcap + k] = make_int2(x, c);
+    };
+    // the arrivals, one per lane (every lane walks their list)
+    int arr = -1, na = 0;
+    for (int a = ah; a != -1 && na <= 32; a = L.arr_next[a]) {
+      if (lane == na) arr = a;
+      na++;
+    }
+    if (len >= 0 && len <= SLOT_CAP && na <= 32) {
+      const bool s0 = e0 >= 0 && cell_new[e0] == c;
+      const bool s1 = e1 >= 0 && cell_new[e1] == c;
+      const unsigned b0 = __ballot_sync(FULL, s0), b1 = __ballot_sync(FULL, s1);
+      if (e0 >= 0 && !s0) record(e0);
+      if (e1 >= 0 && !s1) record(e1);
+      if (arr >= 0) {
+        L.mflag[arr] = 0;
+        record(arr);
       }
+      // the new list: the arrivals in decreasing index, then the stayers in
+      // their old order
+      int at = 0;
+      const int ga = arr >= 0 ? G(arr) : -1;
+      for (int j = 0; j < na; j++) at += __shfl_sync(FULL, ga, j) > ga ? 1 : 0;
+      const unsigned lt = (1u << lane) - 1u;
+      if (arr >= 0) sh[at] = arr;
+      if (s0) sh[na + __popc(b0 & lt)] = e0;
+      if (s1) sh[na + __popc(b0) + __popc(b1 & lt)] = e1;
+      const int len2 = na + __popc(b0) + __popc(b1);
+      __syncwarp();
+      for (int k = lane; k < len2; k += 32) {
+        const int x = sh[k];
+        L.next[x] = k + 1 < len2 ? sh[k + 1] : -1;
+        if (k < SLOT_CAP) L.slot[(size_t)c * SLOT_CAP + k] = x;
+      }
+      if (lane == 0) {
+        L.head[c] = len2 > 0 ? sh[0] : -1;
+        L.slot_n[c] = len2;
+      }
+      __syncwarp();  // (sh is used again)
     } else {
-      int q = L.head[c];
-      while (q != -1) {
-        if (++guard > n) {
+      int ok = 1;
+      if (lane == 0) ok = relink_links(L, cell_new, c, n, record, G) ? 1 : 0;
+      if (!__shfl_sync(FULL, ok, 0)) {
+        if (lane == 0) {
           atomicExch(&cnt->list_error, 1);
           atomicExch(&cnt->abort, 1);
-          return;
         }
-        const bool stays = cell_new[q] == c;
-        const int nq = stays ? L.next[q] : L.mnext[q];
-        if (!stays) record(q);
-        if (stays) {
-          if (prev == -1) first = q;
-          else L.next[prev] = q;
-          prev = q;
-        }
-        q = nq;
-      }
-    }
-    if (prev != -1) L.next[prev] = -1;
-    // 2. prepend the arrivals, highest index first (the reference's index:
-    // gid when the storage is in cell order)
-    auto G = [&](int x) { return L.gid ? L.gid[x] : x; };
-    int sh = -1, tail = -1, a = L.arr_head[c];
-    guard = 0;
-    while (a != -1) {
-      if (++guard > n) {
-        atomicExch(&cnt->list_error, 1);
-        atomicExch(&cnt->abort, 1);
         return;
       }
-      const int an = L.arr_next[a];  // (guard: arrivals so far)
-      L.mflag[a] = 0;
-      record(a);
-      if (sh == -1) {
-        sh = tail = a;
-        L.next[a] = -1;
-      } else if (G(a) > G(sh)) {
-        L.next[a] = sh;
-        sh = a;
-      } else {
-        int q2 = sh;
-        for (int g2 = 0; L.next[q2] != -1 && G(L.next[q2]) > G(a) && g2 < guard; g2++)
-          q2 = L.next[q2];
-        L.next[a] = L.next[q2];
-        L.next[q2] = a;
-        if (L.next[a] == -1) tail = a;
-      }
-      a = an;
     }
-    L.arr_head[c] = -1;
-    if (sh != -1) {
-      L.next[tail] = first;
-      first = sh;
+    if (lane == 0) {
+      L.arr_head[c] = -1;
+      L.dflag[c] = 0;
     }
-    L.head[c] = first;
-    L.dflag[c] = 0;
-    L.dstamp[c] = stamp;
-    if (from_slots) {
-      // the new list's slots: the arrivals (this thread linked them), then
-      // the stayers in their old order
-      int k = 0;
-      int x = sh;
-      for (int t = 0; t < guard; t++) {
-        if (k < SLOT_CAP) L.slot[(size_t)c * SLOT_CAP + k] = x;
-        k++;
-        x = L.next[x];
-      }
-      for (int j = 0; j < len; j++)
-        if ((stay >> j) & 1u) {
-          if (k < SLOT_CAP) L.slot[(size_t)c * SLOT_CAP + k] = old[j];
-          k++;
-        }
-      L.slot_n[c] = k;
-    } else {
-      copy_slots(L, c, first, n);
-    }
-    // 3. the rows that read c are rebuilt in this pass (by the test
-    // kernel): a row of a particle in cell b holds the rest of b's list and
-    // the half-shell cells b + o, kx + Nx*(ky + Ny*kz) > 0, so c is read by
-    // the rows of c itself and of c + o' for the 13 offsets o' with
+    // the rows that read c: a row of a particle in cell b holds the rest of
+    // b's list and the half-shell cells b + o, kx + Nx*(ky + Ny*kz) > 0, so c
+    // is read by the rows of c itself and of c + o' for the 13 offsets o' with
     // kx + Nx*(ky + Ny*kz) < 0; those 14 cells are stamped with the pass
-    const int nx = P.nx, ny = P.ny, nz = P.nz;
-    const int cl = c - P.coff;
-    const int cx = cl % nx, cy = (cl / nx) % ny, cz = cl / (nx * ny);
-#pragma unroll
-    for (int o = 0; o < 14; o++) {
-      const int jx = cx + o % 3 - 1, jy = cy + (o / 3) % 3 - 1, jz = cz + o / 9 - 1;
-      const bool ok = (P.pbc[0] || (jx >= 0 && jx < nx)) && (P.pbc[1] || (jy >= 0 && jy < ny)) &&
-                      (P.pbc[2] || (jz >= 0 && jz < nz));
-      if (ok)
-        L.rflag[P.coff + axis_wrap(jx, nx, P.pbc[0]) +
-                nx * (axis_wrap(jy, ny, P.pbc[1]) + ny * axis_wrap(jz, nz, P.pbc[2]))] = stamp;
-    }
+    const int b = lane < 14 ? reading_cell(P, c, lane) : -1;
+    if (b >= 0) L.rflag[b] = stamp;
   }
 }
+
+// Arguments of a relink
+struct RelinkArgs {
+  const DevParams* PT;
+  const int* cellsys;
+  CellLists L;
+  int par, n, update, stop_tag;
+  Counters* cnt;
+};
 
 // ---------------------------------------------------------------------------
 // K2: candidate rows
 
-// The row of particle p (cell c), built by one warp.  Lane L < 27 owns the
-// neighbour cell at offset (L%3-1, L/3%3-1, L/9-1); lane 13 (own cell) walks
+// The row of particle p (cell c) when a list it reads does not fit the slots,
+// built by one warp.  Lane L < 27 owns the neighbour cell at offset (L%3-1, L/3%3-1, L/9-1); lane 13 (own cell) walks
 // the part of the list after p, lane 27 the part before p (p's rank).  The
 // row holds the partners the sweep meets with p as "i": the own cell after p,
 // then the half-shell cells (offset index kx + Nx*(ky + Ny*kz) > 0,
@@ -269,10 +304,10 @@ __device__ __forceinline__ void relink_body(const DevParams* __restrict__ PT,
 // descending (kz, ky, kx) -- NeighbourParticles' list (src/MCells.f90:
 // 793-829) from p on.
 template <bool PP>
-__device__ __forceinline__ void build_row(const DevParams& P, int n, int p, int c,
-                                          const double4* __restrict__ X,
-                                          const int* __restrict__ comp, const CellLists& L,
-                                          const Rows& R, Counters* cnt, int tag) {
+__device__ __noinline__ void build_row_links(const DevParams& P, int n, int p, int c,
+                                             const double4* __restrict__ X,
+                                             const int* __restrict__ comp, const CellLists& L,
+                                             const Rows& R, Counters* cnt, int tag) {
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int nx = P.nx, ny = P.ny, nz = P.nz;
@@ -325,40 +360,17 @@ __device__ __forceinline__ void build_row(const DevParams& P, int n, int p, int 
     md = __dadd_rn(md, skin);
     return __dsub_rn(__dmul_rn(md, md), DijSq) > 0.0;
   };
-  // the lane's cell read from its slots when its whole list is there
-  // (independent loads), else by walking its links
-  const int len = cw >= 0 ? L.slot_n[cw] : -1;
-  const bool arr = len >= 0 && len <= SLOT_CAP;
-  const int* sl = L.slot + (size_t)(cw >= 0 ? cw : 0) * SLOT_CAP;
-  // pass 1: count the candidates; lane 13 (own cell after p) and lane 27
-  // (p's rank: the list before p) first find p in its cell.  Slots: the hits
-  // are a bit mask for pass 2; links: the first 8 elements and their test
-  // results stay in registers for pass 2.
-  int count = 0, walked = 0;
+  // pass 1: count the candidates; lane 13 (own cell after p) starts behind p,
+  // lane 27 counts the list before p (p's rank).  The first 8 elements and
+  // their test results stay in registers for pass 2.
   unsigned hits = 0u;
+  int count = 0, walked = 0;
   int cache[8];
   bool bad = false;
   int q = -1;
 #pragma unroll
   for (int i = 0; i < 8; i++) cache[i] = -1;
-  if (arr) {
-    int k0 = 0;
-    if (lane == 13 || lane == 27) {
-      int r = 0;
-      while (r < len && sl[r] != p) r++;
-      if (r == len) bad = true;
-      if (lane == 27) count = r;
-      k0 = r + 1;
-    }
-    if (walk && !bad) {
-#pragma unroll 4
-      for (int k = k0; k < len; k++)
-        if (is_cand(sl[k])) {
-          hits |= 1u << k;
-          count++;
-        }
-    }
-  } else if (cw >= 0) {
+  if (cw >= 0) {
     q = lane == 13 ? L.next[p] : L.head[cw];
     if (walk) {
 #pragma unroll
@@ -375,8 +387,8 @@ __device__ __forceinline__ void build_row(const DevParams& P, int n, int p, int 
       }
     }
   }
-  const int resume = q;  // (links) first element not cached (-1: none)
-  if (!arr && cw >= 0) {
+  const int resume = q;  // first element not cached (-1: none)
+  if (cw >= 0) {
     int guard = 0;
     if (walk) {
       while (q != -1) {
@@ -422,25 +434,16 @@ __device__ __forceinline__ void build_row(const DevParams& P, int n, int p, int 
     }
     return;
   }
-  // pass 2: write (slots: the hits; links: the cached part, then the rest)
+  // pass 2: write the cached part, then the rest
   if (walk) {
     int k = off;
-    if (arr) {
-      unsigned h = hits;
-      while (h) {
-        const int j = __ffs(h) - 1;
-        h &= h - 1u;
-        R.cand[(size_t)(k++) * n + p] = sl[j];
-      }
-    } else {
 #pragma unroll
-      for (int i = 0; i < 8; i++)
-        if (i < walked && ((hits >> i) & 1u)) R.cand[(size_t)(k++) * n + p] = cache[i];
-      int q2 = resume;
-      while (q2 != -1) {
-        if (is_cand(q2)) R.cand[(size_t)(k++) * n + p] = q2;
-        q2 = L.next[q2];
-      }
+    for (int i = 0; i < 8; i++)
+      if (i < walked && ((hits >> i) & 1u)) R.cand[(size_t)(k++) * n + p] = cache[i];
+    int q2 = resume;
+    while (q2 != -1) {
+      if (is_cand(q2)) R.cand[(size_t)(k++) * n + p] = q2;
+      q2 = L.next[q2];
     }
   }
   if (lane == 0) {
@@ -450,7 +453,194 @@ __device__ __forceinline__ void build_row(const DevParams& P, int n, int p, int 
 }
 
 
-// Arguments of the test kernel (the same for both precisions).
+// Whether q belongs into p's row: the pair closer than MinDij + skin (+ slack)
+template <bool PP>
+__device__ __forceinline__ bool within_skin(const DevParams& P, const double4& p4, int cp,
+                                            const double4& q4, int cq, double slack) {
+  double Rij[3] = {__dsub_rn(q4.x, p4.x), __dsub_rn(q4.y, p4.y), __dsub_rn(q4.z, p4.z)};
+#pragma unroll
+  for (int k = 0; k < 3; k++) Rij[k] = min_image_rn(Rij[k], P.box, k);
+  const double DijSq = sumsq3_rn(Rij);
+  double md;
+  if (PP) md = __dadd_rn(p4.w, q4.w);
+  else md = __dsqrt_rn(min_dij_sq_rn<PP>(P, cp, p4.w, cq, q4.w));
+  md = __dadd_rn(md, __dadd_rn(P.vl_skin, slack));
+  return !(__dsub_rn(__dmul_rn(md, md), DijSq) <= 0.0);
+}
+
+// The row of particle p (cell c), built by one warp: the partners the sweep
+// meets with p as "i" -- the own cell's list after p, then the half-shell
+// cells (offset index kx + Nx*(ky + Ny*kz) > 0, AddAllNeighbours3D
+// src/MCells.f90:456) in FirstNeighbour order, i.e. descending (kz, ky, kx),
+// which is NeighbourParticles' list (src/MCells.f90:793-829) from p on.  Lane
+// l < 14 holds the l-th of those lists; laid end to end they are tested 32
+// elements at a time, two loads deep, and the hits appended in order, so a
+// row costs the same few round trips whether its cells hold two particles or
+// thirty.
+template <bool PP>
+__device__ __noinline__ void build_row(const DevParams& P, int n, int p, int c,
+                                       const double4* __restrict__ X,
+                                       const int* __restrict__ comp, const CellLists& L,
+                                       const Rows& R, Counters* cnt, int tag) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const double4 p4 = ld32(X + p);
+  const int cp = PP ? 0 : comp[p];
+  int cx, cy, cz;
+  cell_coords(P, c, cx, cy, cz);
+  int cw = -1, len = 0;
+  if (lane == 0) {
+    cw = c;
+  } else if (lane < 14) {
+    const int o = 27 - lane;  // 26 .. 14: offsets in descending (kz, ky, kx)
+    const int jx = cx + o % 3 - 1, jy = cy + (o / 3) % 3 - 1, jz = cz + o / 9 - 1;
+    const bool ok = (P.pbc[0] || (jx >= 0 && jx < P.nx)) &&
+                    (P.pbc[1] || (jy >= 0 && jy < P.ny)) && (P.pbc[2] || (jz >= 0 && jz < P.nz));
+    if (ok)
+      cw = P.coff + axis_wrap(jx, P.nx, P.pbc[0]) +
+           P.nx * (axis_wrap(jy, P.ny, P.pbc[1]) + P.ny * axis_wrap(jz, P.nz, P.pbc[2]));
+  }
+  if (cw >= 0) len = L.slot_n[cw];
+  const int* own = L.slot + (size_t)c * SLOT_CAP;
+  // (p's place in its list; entries past the list's end are old ones)
+  const int w0 = own[lane], w1 = own[lane + 32];
+  if (__any_sync(FULL, len < 0 || len > SLOT_CAP)) {
+    build_row_links<PP>(P, n, p, c, X, comp, L, R, cnt, tag);
+    return;
+  }
+  const int len0 = __shfl_sync(FULL, len, 0);
+  const unsigned f0 = __ballot_sync(FULL, lane < len0 && w0 == p);
+  const unsigned f1 = __ballot_sync(FULL, lane + 32 < len0 && w1 == p);
+  if (!(f0 | f1)) {
+    if (lane == 0) {
+      atomicExch(&cnt->list_error, 1);
+      set_abort(cnt, tag);
+    }
+    return;
+  }
+  const int rank = f0 ? __ffs(f0) - 1 : 31 + __ffs(f1);
+  int skip = 0;  // entries of the lane's list that the row does not read
+  if (lane == 0) {
+    skip = rank + 1;
+    len -= skip;
+  }
+  int incl = len;  // (0 on lanes >= 14)
+#pragma unroll
+  for (int o = 1; o < 16; o <<= 1) {
+    const int y = __shfl_up_sync(FULL, incl, o);
+    if (lane >= o) incl += y;
+  }
+  const int T = __shfl_sync(FULL, incl, 13);
+  const int excl = lane < 14 ? incl - len : INT_MAX;
+  // the slot of element f of the lists laid end to end
+  auto slot_of = [&](int f) -> size_t {
+    int j = 0;
+#pragma unroll
+    for (int step = 8; step > 0; step >>= 1) {
+      const int ex = __shfl_sync(FULL, excl, j + step);
+      if (ex <= f) j += step;
+    }
+    const int cj = __shfl_sync(FULL, cw, j), sj = __shfl_sync(FULL, skip, j),
+              ej = __shfl_sync(FULL, excl, j);
+    return (size_t)cj * SLOT_CAP + (sj + f - ej);
+  };
+  int m = 0;
+  for (int f = 0; f < T; f += 64) {
+    const size_t i0 = slot_of(f + lane), i1 = slot_of(f + 32 + lane);
+    const bool a0 = f + lane < T, a1 = f + 32 + lane < T;
+    const int q0 = a0 ? L.slot[i0] : p, q1 = a1 ? L.slot[i1] : p;
+    const double4 x0 = ld32(X + q0), x1 = ld32(X + q1);
+    const bool h0 = a0 && within_skin<PP>(P, p4, cp, x0, PP ? 0 : comp[q0], 0.0);
+    const bool h1 = a1 && within_skin<PP>(P, p4, cp, x1, PP ? 0 : comp[q1], 0.0);
+    const unsigned b0 = __ballot_sync(FULL, h0), b1 = __ballot_sync(FULL, h1);
+    const unsigned lt = (1u << lane) - 1u;
+    const int k0 = m + __popc(b0 & lt), k1 = m + __popc(b0) + __popc(b1 & lt);
+    if (h0 && k0 < R.kc) R.cand[(size_t)k0 * n + p] = q0;
+    if (h1 && k1 < R.kc) R.cand[(size_t)k1 * n + p] = q1;
+    m += __popc(b0) + __popc(b1);
+  }
+  if (lane != 0) return;
+  if (m > R.kc) {
+    atomicMax(&cnt->need_kc, m);
+    atomicExch(&cnt->row_overflow, 1);
+    set_abort(cnt, tag);
+    R.meta[p] = 0;
+    return;
+  }
+  R.meta[p] = m;
+  R.rank[p] = rank;
+}
+
+// The same row by one thread, for a full rebuild: 32 neighbouring rows read
+// the same cells through L1, so a warp builds them in about the round trips
+// that it needs for one row on its own (1M rows: 1.5 ms a warp per row).
+// false: a list does not fit the slots, nothing is written.
+template <bool PP>
+__device__ __noinline__ bool build_row_thread(const DevParams& P, int n, int p, int c,
+                                              const double4* __restrict__ X,
+                                              const int* __restrict__ comp, const CellLists& L,
+                                              const Rows& R, Counters* cnt, int tag) {
+  const double4 p4 = ld32(X + p);
+  const int cp = PP ? 0 : comp[p];
+  int cx, cy, cz;
+  cell_coords(P, c, cx, cy, cz);
+  int m = 0, rank = -1;
+#pragma unroll 1
+  for (int l = 0; l < 14; l++) {
+    int cw = c;
+    if (l > 0) {
+      const int o = 27 - l;
+      const int jx = cx + o % 3 - 1, jy = cy + (o / 3) % 3 - 1, jz = cz + o / 9 - 1;
+      const bool ok = (P.pbc[0] || (jx >= 0 && jx < P.nx)) &&
+                      (P.pbc[1] || (jy >= 0 && jy < P.ny)) &&
+                      (P.pbc[2] || (jz >= 0 && jz < P.nz));
+      if (!ok) continue;
+      cw = P.coff + axis_wrap(jx, P.nx, P.pbc[0]) +
+           P.nx * (axis_wrap(jy, P.ny, P.pbc[1]) + P.ny * axis_wrap(jz, P.nz, P.pbc[2]));
+    }
+    const int4* sl = (const int4*)(L.slot + (size_t)cw * SLOT_CAP);
+    int4 s = sl[0];  // (the first entries with the length)
+    const int len = L.slot_n[cw];
+    if (len < 0 || len > SLOT_CAP) return false;
+    for (int k0 = 0; k0 < len; k0 += 4) {
+      if (k0 > 0) s = sl[k0 >> 2];
+      const int q[4] = {s.x, s.y, s.z, s.w};
+      double4 x[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        if (k0 + u < len) x[u] = ld32(X + q[u]);
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        if (k0 + u >= len) continue;
+        if (l == 0 && rank < 0) {  // the own list up to p: not read
+          if (q[u] == p) rank = k0 + u;
+          continue;
+        }
+        if (within_skin<PP>(P, p4, cp, x[u], PP ? 0 : comp[q[u]], 0.0)) {
+          if (m < R.kc) R.cand[(size_t)m * n + p] = q[u];
+          m++;
+        }
+      }
+    }
+    if (rank < 0) {  // p is not in its cell's list
+      atomicExch(&cnt->list_error, 1);
+      set_abort(cnt, tag);
+      return true;
+    }
+  }
+  if (m > R.kc) {
+    atomicMax(&cnt->need_kc, m);
+    atomicExch(&cnt->row_overflow, 1);
+    set_abort(cnt, tag);
+    R.meta[p] = 0;
+    return true;
+  }
+  R.meta[p] = m;
+  R.rank[p] = rank;
+  return true;
+}
+
+// Arguments of the row and the test kernel (the same for both precisions).
 struct TestArgs {
   const DevParams* P;
   const int* sysid;
@@ -473,229 +663,319 @@ struct TestArgs {
   // (a slab of a decomposition, or every cell)
   int slab_c0;
   unsigned slab_span;
-  // 1: a stamped row is rebuilt only when a particle that changed cell is
-  // near it (row_stays); 0: every stamped row is rebuilt
+  // 1: of the rows that read a relinked cell, only those near a particle that
+  // changed cell are rebuilt; 0: every row of a stamped cell
   int fine;
 };
 
-// Whether the row of particle pl (cell cl), stamped because a cell it reads
-// was relinked, can stay as it is; called by the whole warp together.  A
-// relink keeps the stayers of a list in their order and puts the arrivals
-// first, so the row changes only if a particle that left or entered one of
-// those cells is within MinDij + skin of pl; one farther than that can come
-// no closer than MinDij + 0.2 skin before the next full rebuild (every
-// particle moves at most 0.4 skin in between), so a stale entry for it in
-// the row is tested and rejected, and its absence changes no contact.  The
-// lanes check the pass's movers 32 at a time (a margin errs towards
-// rebuilding); when none is near, the row stays, and if pl's own cell was
-// relinked its rank (its place in the list) is rewritten from the slots.
+// The candidate rows this pass rebuilds (the body of k_rows; warp / nwarps:
+// this warp's index among the warps that share the work):
+//  - every row on a full rebuild, a thread per row;
+//  - else the rows a relinked cell's movers change.  A relink keeps the
+//    stayers of a list in their order and puts the arrivals first, so a row
+//    that reads the cell changes only if a particle that left or entered it
+//    is within MinDij + skin of the row's owner; one farther than that can
+//    come no closer than MinDij + 0.2 skin before the next full rebuild
+//    (every particle moves at most 0.4 skin in between), so a stale entry for
+//    it in the row is tested and rejected, and its absence changes no
+//    contact.  A warp takes one record (mover, cell) and one of the 14 cells
+//    whose rows read that cell, its lanes check the owners there (a margin
+//    errs towards rebuilding), and it builds the rows that are near and that
+//    no other warp has claimed in this pass.  The rank (the place in the list)
+//    of every particle of a relinked cell is rewritten.
+//  - else, when more movers were recorded than the list holds, or in a slab
+//    of a decomposition (the stamps of its ghost layer come by exchange),
+//    every row of a stamped cell.
+// The rows were rebuilt inside the test kernel before, each by the warp of
+// its owner: one after another within a warp, whose block waited (box of
+// 1M bidisperse spheres, 84 movers a pass: 300 us per test launch).
 template <bool PP>
-__device__ __forceinline__ bool row_stays(const TestArgs& A, int pl, int cl, const double4& p4,
-                                          int cp, int stamp, int n, int lane) {
+__device__ __forceinline__ void rows_body(const TestArgs& A, int warp, int nwarps) {
   const unsigned FULL = 0xffffffffu;
-  const int b = stamp & 1;
-  const int nm = A.cnt->n_mlist[b];
-  if (nm > A.L.mcap) return false;
-  const DevParams& P = sys_params(A.P, A.sysid, pl);
-  const double skin = P.vl_skin;
-  const int* ml = A.L.mlist + (size_t)b * A.L.mcap;
-  bool near = false;
-  for (int k = lane; k < nm && !near; k += 32) {
-    const int q = ml[k];
-    if ((unsigned)q >= (unsigned)n) {
-      near = true;
-      break;
+  const int lane = threadIdx.x & 31;
+  Counters* const cnt = A.cnt;
+  const int abort0 = cnt->abort;
+  const bool full = cnt->full_due != 0;
+  const int stamp = cnt->pass_id + 1;
+  const int nm = cnt->n_mlist[stamp & 1];
+  if (abort0) return;
+  const int n = A.n;
+  const CellLists& L = A.L;
+  auto build = [&](int p, int c) {
+    build_row<PP>(sys_params(A.P, A.sysid, p), n, p, c, A.X, A.comp, L, A.R, cnt, A.tag);
+  };
+  if (full || !A.fine || nm > L.mcap) {
+    for (int v = warp; v < (n + 31) / 32; v += nwarps) {
+      const int p = v * 32 + lane;
+      const int c = p < n ? A.cell_cur[p] : -1;
+      bool need = p < n && (unsigned)(c - A.slab_c0) < A.slab_span;
+      if (need)
+        need = full ? !build_row_thread<PP>(sys_params(A.P, A.sysid, p), n, p, c, A.X, A.comp, L,
+                                            A.R, cnt, A.tag)
+                    : L.rflag[c] == stamp;
+      unsigned todo = __ballot_sync(FULL, need);
+      while (todo) {
+        const int l = __ffs(todo) - 1;
+        todo &= todo - 1u;
+        build(__shfl_sync(FULL, p, l), __shfl_sync(FULL, c, l));
+      }
     }
-    const double4 q4 = ld32(A.X + q);
-    double Rij[3] = {__dsub_rn(q4.x, p4.x), __dsub_rn(q4.y, p4.y), __dsub_rn(q4.z, p4.z)};
-#pragma unroll
-    for (int d = 0; d < 3; d++) Rij[d] = min_image_rn(Rij[d], P.box, d);
-    const double DijSq = sumsq3_rn(Rij);
-    double md;
-    if (PP) md = __dadd_rn(p4.w, q4.w);
-    else md = __dsqrt_rn(min_dij_sq_rn<PP>(P, cp, p4.w, A.comp[q], q4.w));
-    md = __dadd_rn(__dadd_rn(md, skin), __dadd_rn(1.0e-9, __dmul_rn(1.0e-9, md)));
-    if (!(__dsub_rn(__dmul_rn(md, md), DijSq) < 0.0)) near = true;
+    return;
   }
-  if (__any_sync(FULL, near)) return false;
-  if (A.L.dstamp[cl] == stamp) {
-    const int len = A.L.slot_n[cl];
-    if (len < 0 || len > SLOT_CAP) return false;
-    const bool hit = lane < len && A.L.slot[(size_t)cl * SLOT_CAP + lane] == pl;
-    const unsigned h = __ballot_sync(FULL, hit);
-    if (!h) return false;
-    if (lane == 0) A.R.rank[pl] = __ffs(h) - 1;
+  for (int item = warp; item < nm * 14; item += nwarps) {
+    const int2 r = L.mlist[(size_t)(stamp & 1) * L.mcap + item / 14];
+    const int o = item % 14;
+    if ((unsigned)r.x >= (unsigned)n) continue;
+    const DevParams& P = sys_params(A.P, A.sysid, r.x);
+    const int b = reading_cell(P, r.y, o);
+    if (b < 0) continue;
+    const int len = L.slot_n[b];
+    const double4 q4 = ld32(A.X + r.x);
+    const int cq = PP ? 0 : A.comp[r.x];
+    const int* sl = L.slot + (size_t)b * SLOT_CAP;
+    const bool slots = len >= 0 && len <= SLOT_CAP;
+    int at = L.head[b];  // (a list that does not fit the slots: its next 32)
+    for (int k0 = 0; slots ? k0 < len : (at != -1 && k0 < n); k0 += 32) {
+      int x = -1;
+      if (slots) {
+        if (k0 + lane < len) x = sl[k0 + lane];
+      } else {
+        for (int k = 0; k < 32 && at != -1; k++) {
+          if (lane == k) x = at;
+          at = L.next[at];
+        }
+      }
+      bool need = false;
+      if (x >= 0) {
+        if (o == 13) A.R.rank[x] = k0 + lane;  // (the relinked cell itself)
+        const double4 x4 = ld32(A.X + x);
+        const double slack = 1.0e-9 * (1.0 + x4.w + q4.w);
+        need = within_skin<PP>(P, x4, PP ? 0 : A.comp[x], q4, cq, slack) &&
+               atomicExch(&L.rstamp[x], stamp) != stamp;
+      }
+      unsigned todo = __ballot_sync(FULL, need);
+      while (todo) {
+        const int l = __ffs(todo) - 1;
+        todo &= todo - 1u;
+        build(__shfl_sync(FULL, x, l), b);
+      }
+    }
   }
-  return true;
 }
 
-// First, the candidate rows of the warp's particles that this pass rebuilds
-// (every row on a full rebuild, else the rows of the particles whose cell the
-// relink stamped with this pass) are built, one particle at a time by the
-// whole warp (build_row).  Then every particle tests its row, and the block
-// takes room for its contacts in the list with one atomic (two block
-// barriers, which every thread of the block meets).  (The pass's contact
-// count and the list length it needs come from the pair kernel, or from
-// here when the list overflows.)
+// Every particle tests its row; the contacts of a particle are written
+// together and in row order, and the block takes room for its contacts in
+// the list with one atomic (two block barriers, which every thread of the
+// block meets).  (The pass's contact count and the list length it needs come
+// from the pair kernel, or from here when the list overflows.)
+//
+// Rows are short and uneven (2.9 candidates on average, 8 in the longest of
+// 32, at 1M spheres), so a warp lays its 32 rows end to end in shared memory
+// and its lanes test one candidate each, 128 at a time: 3 turns instead of
+// two groups of four per thread, all positions of a turn in flight together.
+// The ballots of the turns give every contact's place.  A warp whose rows
+// hold more than WIN candidates goes through them in windows, once to count
+// and once more to write.
 // (The body of k_test for block `vblock`, so that a persistent kernel can
 // run it too.  NC: candidates read through the non-coherent path, which
-// needs the rows unchanged for the whole launch except by the warp that
-// reads them; a kernel that runs several passes reads them coherently.)
+// needs the rows unchanged for the whole launch; a kernel that runs several
+// passes reads them coherently.)
 template <bool NC>
 __device__ __forceinline__ int ld_row(const int* a) {
   return NC ? __ldg(a) : *a;
 }
+constexpr int WIN = 256;
+struct alignas(16) TestWarp {  // shared memory of one warp
+  double4 x[32];               // the rows' owners
+  int q[WIN];                  // candidates of the window
+  unsigned short own[WIN];     // (component << 8) | lane of the owner
+  unsigned mask[WIN / 32 + 1];  // contacts among them
+  int pre[WIN / 32 + 1];       // contacts before each 32
+};
 
 template <bool PP, bool NC = true>
-__device__ __forceinline__ void test_body(const TestArgs& A, int vblock) {
+__device__ __forceinline__ void test_body(const TestArgs& A, int vblock, TestWarp* warps) {
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5;
+  TestWarp& W = warps[warp];
   const int p0 = vblock * blockDim.x + threadIdx.x;
-  const bool valid0 = p0 < A.n;
-  const int p = valid0 ? p0 : 0;
+  const int p = p0 < A.n ? p0 : 0;
   const int n = A.n;
-  // the abort word, the pass's rebuild decision, the particle's cell, own
-  // data, row length and first candidates are requested together (the first
-  // candidates before the row length is known: every row holds at least 4
-  // entries' room); nothing is written once the abort word is seen (the
-  // block still meets its barrier), and a warp whose rows were rebuilt reads
-  // them again
+  // the abort word, the particle's own data, row length and first candidates
+  // are requested together (every row holds at least 4 entries' room);
+  // nothing is written once the abort word is seen (the block still meets its
+  // barriers)
   const bool live = A.cnt->abort == 0;
-  const bool full = A.cnt->full_due != 0;
-  const int stamp = A.cnt->pass_id + 1;
-  const int cp0 = A.cell_cur[p];
-  // (a slab of a decomposition tests only its own particles)
-  const bool valid = valid0 && (unsigned)(cp0 - A.slab_c0) < A.slab_span;
-  const double4 p4 = ld32(A.X + p);
-  const int cp = PP ? 0 : A.comp[p];
+  const int meta = A.meta[p];
   int q0[4];
 #pragma unroll
   for (int u = 0; u < 4; u++) q0[u] = ld_row<NC>(A.cand + (size_t)u * n + p);
-  int meta = A.meta[p];
-  {
-    bool stale = live && valid && (full || A.L.rflag[cp0] == stamp);
-    if (!full && A.fine) {
-      // the stamped rows checked against the pass's movers, one at a time
-      // by the whole warp
-      unsigned chk = __ballot_sync(FULL, stale);
-      while (chk) {
-        const int l = __ffs(chk) - 1;
-        chk &= chk - 1u;
-        const int pl = __shfl_sync(FULL, p, l);
-        const int cl = __shfl_sync(FULL, cp0, l);
-        const int cpl = __shfl_sync(FULL, cp, l);
-        const double4 pl4 = make_double4(__shfl_sync(FULL, p4.x, l), __shfl_sync(FULL, p4.y, l),
-                                         __shfl_sync(FULL, p4.z, l), __shfl_sync(FULL, p4.w, l));
-        const bool keep = row_stays<PP>(A, pl, cl, pl4, cpl, stamp, n, lane);
-        if (lane == l && keep) stale = false;
-      }
-    }
-    unsigned todo = __ballot_sync(FULL, stale);
-    if (todo) {
-      while (todo) {
-        const int l = __ffs(todo) - 1;
-        todo &= todo - 1u;
-        const int pl = __shfl_sync(FULL, p, l);
-        const int cl = __shfl_sync(FULL, cp0, l);
-        build_row<PP>(sys_params(A.P, A.sysid, pl), n, pl, cl, A.X, A.comp, A.L, A.R, A.cnt,
-                      A.tag);
-      }
-      __syncwarp();  // the rows written by the warp are visible to their owners
-#pragma unroll
-      for (int u = 0; u < 4; u++) q0[u] = A.cand[(size_t)u * n + p];
-      meta = A.meta[p];
-    }
-  }
-  const DevParams& P = sys_params(A.P, A.sysid, p);
+  const double4 p4 = ld32(A.X + p);
+  const int cp = PP ? 0 : A.comp[p];
+  // (a slab of a decomposition tests only its own particles)
+  bool valid = p0 < n;
+  if (A.slab_span != 0xffffffffu && valid)
+    valid = (unsigned)(A.cell_cur[p] - A.slab_c0) < A.slab_span;
   const int m = live && valid ? (meta & META_MASK) : 0;
-  // contact bit masks of the row, 64 candidates per window (windows past
-  // the first only for rows longer than 64)
-  unsigned long long mask0 = 0ull;
-  unsigned long long more[(KC_MAX + 1) / 64 - 1];
-  int total = 0;
-  // the next group's candidates are requested with this group's positions:
-  // one round trip per group of 4 after the first
-  int qn[4];
-#pragma unroll
-  for (int u = 0; u < 4; u++) qn[u] = q0[u];
-  for (int base = 0; base < m; base += 64) {
-    unsigned long long mask = 0ull;
-    const int end = m < base + 64 ? m : base + 64;
-#pragma unroll 1
-    for (int b = base; b < end; b += 4) {
-      int q[4];
-#pragma unroll
-      for (int u = 0; u < 4; u++) q[u] = b + u < end ? qn[u] : -1;
-#pragma unroll
-      for (int u = 0; u < 4; u++)
-        qn[u] = b + 4 + u < m ? ld_row<NC>(A.cand + (size_t)(b + 4 + u) * n + p) : -1;
-      double4 xq[4];
-#pragma unroll
-      for (int u = 0; u < 4; u++)
-        if (q[u] >= 0) xq[u] = ld32(A.X + q[u]);
-#pragma unroll
-      for (int u = 0; u < 4; u++) {
-        if (q[u] < 0) continue;
-        double Rij[3] = {__dsub_rn(xq[u].x, p4.x), __dsub_rn(xq[u].y, p4.y),
-                         __dsub_rn(xq[u].z, p4.z)};
-#pragma unroll
-        for (int k = 0; k < 3; k++) Rij[k] = min_image_rn(Rij[k], P.box, k);
-        const double DijSq = sumsq3_rn(Rij);
-        const int cq = PP ? 0 : A.comp[q[u]];
-        if (__dsub_rn(min_dij_sq_rn<PP>(P, cp, p4.w, cq, xq[u].w), DijSq) > 0.0)
-          mask |= 1ull << (b + u - base);
-      }
-    }
-    total += __popcll(mask);
-    if (base == 0) mask0 = mask;
-    else more[base / 64 - 1] = mask;
-  }
-  // one allocation per block (the warps' sums through shared memory, one
-  // atomic on the pass's list length); a particle's contacts are contiguous
-  int incl = total;
+  W.x[lane] = p4;
+  int off = m;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(FULL, incl, o);
-    if (lane >= o) incl += y;
+    const int y = __shfl_up_sync(FULL, off, o);
+    if (lane >= o) off += y;
   }
-  __shared__ int s_wsum[8];  // blocks of at most 256 threads
-  __shared__ int s_base;
-  const int warp = threadIdx.x >> 5;
-  if (lane == 31) s_wsum[warp] = incl;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int acc = 0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); w++) {
-      const int t = s_wsum[w];
-      s_wsum[w] = acc;
-      acc += t;
+  const int T = __shfl_sync(FULL, off, 31);
+  off -= m;
+  // one system: its box in registers (no image beyond an infinite bound)
+  const DevParams& P0 = A.P[0];
+  const bool one = A.sysid == nullptr;
+  const double inf = __longlong_as_double(0x7ff0000000000000ll);
+  const double hx = P0.box.pbc[0] ? P0.box.half_lim[0] : inf;
+  const double hy = P0.box.pbc[1] ? P0.box.half_lim[1] : inf;
+  const double hz = P0.box.pbc[2] ? P0.box.half_lim[2] : inf;
+  // candidates [w0, w0 + WIN) of the warp into W.q / W.own, their contact
+  // ballots into W.mask, the running count into W.pre
+  auto window = [&](int w0) {
+    const int lo = w0 > off ? w0 - off : 0;
+    const int hi = off + m < w0 + WIN ? m : w0 + WIN - off;
+    const unsigned short own = (unsigned short)((cp << 8) | lane);
+    for (int k = lo; k < hi; k++) {
+      const int f = off + k - w0;
+      int q;
+      if (k < 4) {
+        q = q0[0];
+        if (k == 1) q = q0[1];
+        if (k == 2) q = q0[2];
+        if (k == 3) q = q0[3];
+      } else {
+        q = ld_row<NC>(A.cand + (size_t)k * n + p);
+      }
+      W.q[f] = q;
+      W.own[f] = own;
     }
-    s_base = acc > 0 ? atomicAdd(&A.cnt->n_contacts, acc) : 0;
-  }
-  __syncthreads();
-  const int start = s_base + s_wsum[warp] + incl - total;
-  if (live && valid) {
-    A.cstart[p] = start;
-    A.ccount[p] = total;
-  }
-  if (!live) return;
-  if (start + total > A.cl_cap) {
-    // the list is grown and the pass launched again
-    atomicMax(&A.cnt->need_cl, start + total);
-    atomicExch(&A.cnt->cl_overflow, 1);
-    set_abort(A.cnt, A.tag);
-  } else if (total > 0) {
-    int s = start;
-    for (int base = 0; base < m; base += 64) {
-      unsigned long long mask = base == 0 ? mask0 : more[base / 64 - 1];
-      while (mask) {
-        const int k = base + __ffsll((long long)mask) - 1;
-        mask &= mask - 1ull;
-        A.clist[s] = make_int2(p, ld_row<NC>(A.cand + (size_t)k * n + p));
-        const int o = s - start;
-        A.cord[s++] = (unsigned char)(o < ORD_MAX ? o : ORD_MAX);
+    __syncwarp();
+    const int Tw = T - w0 < WIN ? T - w0 : WIN;
+    int run = 0;
+    for (int f0 = 0; f0 < Tw; f0 += 128) {
+      double4 xq[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const int f = f0 + 32 * u + lane;
+        if (f < Tw) xq[u] = ld32(A.X + W.q[f]);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const int f = f0 + 32 * u + lane;
+        bool hit = false;
+        if (f < Tw) {
+          const int own_f = W.own[f];
+          const double4 a = W.x[own_f & 31];
+          double Rij[3] = {__dsub_rn(xq[u].x, a.x), __dsub_rn(xq[u].y, a.y),
+                           __dsub_rn(xq[u].z, a.z)};
+          const DevParams* P = &P0;
+          if (one) {
+            if (!(fabs(Rij[0]) < hx)) Rij[0] = image_rn(Rij[0], P0.box, 0);
+            if (!(fabs(Rij[1]) < hy)) Rij[1] = image_rn(Rij[1], P0.box, 1);
+            if (!(fabs(Rij[2]) < hz)) Rij[2] = image_rn(Rij[2], P0.box, 2);
+          } else {
+            P = A.P + A.sysid[p0 - lane + (own_f & 31)];
+#pragma unroll
+            for (int k = 0; k < 3; k++) Rij[k] = min_image_rn(Rij[k], P->box, k);
+          }
+          const int cq = PP || P->nc == 1 ? 0 : A.comp[W.q[f]];
+          const double md = min_dij_sq_rn<PP>(*P, PP ? 0 : own_f >> 8, a.w, cq, xq[u].w);
+          hit = __dsub_rn(md, sumsq3_rn(Rij)) > 0.0;
+        }
+        if (f0 + 32 * u < Tw) {
+          const unsigned b = __ballot_sync(FULL, hit);
+          if (lane == 0) {
+            W.mask[(f0 >> 5) + u] = b;
+            W.pre[(f0 >> 5) + u] = run;
+          }
+          run += __popc(b);
+        }
       }
     }
+    if (lane == 0) {
+      W.mask[(Tw + 31) >> 5] = 0u;
+      W.pre[(Tw + 31) >> 5] = run;
+    }
+    __syncwarp();
+  };
+  // contacts among the window's first f candidates
+  auto before = [&](int f) {
+    return W.pre[f >> 5] + __popc(W.mask[f >> 5] & ((1u << (f & 31)) - 1u));
+  };
+  __shared__ int s_wsum[8];  // blocks of at most 256 threads
+  __shared__ int s_base;
+  int total = 0, start = 0, done = 0;  // done: contacts written from earlier windows
+  // first the contacts are counted, then written
+#pragma unroll 1
+  for (int ph = 0; ph < 2; ph++) {
+#pragma unroll 1
+    for (int w0 = 0; w0 < T; w0 += WIN) {
+      if (ph == 0 || T > WIN) window(w0);
+      const int Tw = T - w0 < WIN ? T - w0 : WIN;
+      // the lane's part of the window
+      const int lo = off < w0 ? 0 : off - w0 < Tw ? off - w0 : Tw;
+      const int hi = off + m < w0 ? 0 : off + m - w0 < Tw ? off + m - w0 : Tw;
+      const int b_lo = before(lo), mine = before(hi) - b_lo;
+      if (ph == 0) {
+        total += mine;
+        __syncwarp();
+        continue;
+      }
+      const int base = start + done - b_lo;  // place of the row's contact k: base + before
+      const int first = done - b_lo;         // its number among the owner's: first + before
+      done += mine;
+      for (int f = lane; f < ((Tw + 31) & ~31); f += 32) {
+        const unsigned b = W.mask[f >> 5];
+        const int o = f < Tw ? W.own[f] & 31 : 0;
+        const int bo = __shfl_sync(FULL, base, o), fo = __shfl_sync(FULL, first, o);
+        if ((b >> lane) & 1u) {
+          const int k = W.pre[f >> 5] + __popc(b & ((1u << lane) - 1u));
+          A.clist[bo + k] = make_int2(p0 - lane + o, W.q[f]);
+          const int ord = fo + k;
+          A.cord[bo + k] = (unsigned char)(ord < ORD_MAX ? ord : ORD_MAX);
+        }
+      }
+      __syncwarp();
+    }
+    if (ph == 1) break;
+    // one allocation per block (the warps' sums through shared memory, one
+    // atomic on the pass's list length); a particle's contacts are contiguous
+    int incl = total;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(FULL, incl, o);
+      if (lane >= o) incl += y;
+    }
+    if (lane == 31) s_wsum[warp] = incl;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      int acc = 0;
+      for (int w = 0; w < (int)(blockDim.x >> 5); w++) {
+        const int t = s_wsum[w];
+        s_wsum[w] = acc;
+        acc += t;
+      }
+      s_base = acc > 0 ? atomicAdd(&A.cnt->n_contacts, acc) : 0;
+    }
+    __syncthreads();
+    start = s_base + s_wsum[warp] + incl - total;
+    if (live && valid) {
+      A.cstart[p] = start;
+      A.ccount[p] = total;
+    }
+    const bool over = live && start + total > A.cl_cap;
+    if (over) {
+      // the list is grown and the pass launched again
+      atomicMax(&A.cnt->need_cl, start + total);
+      atomicExch(&A.cnt->cl_overflow, 1);
+      set_abort(A.cnt, A.tag);
+    }
+    if (__any_sync(FULL, over)) return;
   }
 }
 
@@ -703,15 +983,6 @@ __device__ __forceinline__ void test_body(const TestArgs& A, int vblock) {
 // Persistent launches: a 4-step chunk (8 force passes) as one cooperative
 // launch whose blocks step through every pass's phases (relink, test, pair,
 // fold), separated by grid-wide barriers.
-
-// Arguments of a relink (k_relink's parameters)
-struct RelinkArgs {
-  const DevParams* PT;
-  const int* cellsys;
-  CellLists L;
-  int par, n, update, stop_tag;
-  Counters* cnt;
-};
 
 // A grid-wide barrier over `expected` blocks (gridDim.x of a cooperative
 // launch, so that every block is resident): an arrival counter and a
@@ -789,6 +1060,27 @@ struct alignas(16) ChunkPass {
   View v;
   int epi;
 };
+
+// The list phases of a chunk as calls, so that each has its own register
+// allocation within the kernel's budget (inlined together they spill 1-2 kB a
+// thread).
+template <class CP>
+__device__ __noinline__ void chunk_relink(const CP& p, int warp, int nwarps, int* sh) {
+  const RelinkArgs& R = p.rl;
+  relink_body(R.PT, R.cellsys, R.L, R.par, R.n, R.update, R.stop_tag, R.cnt, warp, nwarps, sh);
+}
+template <bool PP, class CP>
+__device__ __noinline__ void chunk_rows(const CP& p, int warp, int nwarps) {
+  rows_body<PP>(p.t, warp, nwarps);
+}
+template <bool PP, class CP>
+__device__ __noinline__ void chunk_test(const CP& p, TestWarp* warps) {
+  const int nvb = (p.t.n + 127) / 128;
+  for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
+    test_body<PP, false>(p.t, vb, warps);
+    __syncthreads();
+  }
+}
 
 // the pass `src` into the block's shared copy `dst`
 template <class CP>
