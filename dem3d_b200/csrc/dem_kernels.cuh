@@ -1094,11 +1094,25 @@ __global__ void __launch_bounds__(128, WALLS ? 4 : 5) k_fold_fp64(PassArgs<doubl
 // Rows are read coherently (written by earlier passes of the same launch).
 using ChunkPass64 = ChunkPass<double4, double2, NoView>;
 
-template <bool PP, bool WALLS>
-__global__ void __launch_bounds__(128, 4) k_chunk_fp64(const ChunkPass64* __restrict__ prog,
-                                                       int npass, GridSync g) {
+// the fold phase of this block
+template <bool PP, int EPI, bool WALLS>
+__device__ __forceinline__ void fold_blocks_fp64(const ChunkPass64& sp, double* stage) {
+  const int nvb = (sp.t.n + 127) / 128;
+  for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
+    fold_fp64_body<PP, EPI, WALLS>(sp.a, vb, stage);
+    __syncthreads();
+  }
+}
+// CLUSTER: the launch is one cluster instead (ClusterRun), for systems so
+// small that a pass is a chain of latencies: no launch boundaries, a hardware
+// barrier between the phases, npass passes of a program of 8 that repeats, and
+// the whole register file of an SM for each block.
+template <bool PP, bool WALLS, bool CLUSTER>
+__global__ void __launch_bounds__(128, CLUSTER ? 1 : 3)
+    k_chunk_fp64(const ChunkPass64* __restrict__ prog, int npass, GridSync g, ClusterRun cr) {
   __shared__ ChunkPass64 sp;
-  __shared__ __align__(16) double stage[EpiStage<EPI_PREDICT, false>::SIZE];  // (the larger of the two)
+  // (the larger of the two epilogues')
+  __shared__ __align__(16) double stage[EpiStage<EPI_PREDICT, false>::SIZE];
   // (the relink's and the test's shared arrays lie in the fold's columns)
   int(*const sh)[RELINK_ROOM] = reinterpret_cast<int(*)[RELINK_ROOM]>(stage);
   TestWarp* const warps = reinterpret_cast<TestWarp*>(stage);
@@ -1106,23 +1120,25 @@ __global__ void __launch_bounds__(128, 4) k_chunk_fp64(const ChunkPass64* __rest
                 "shared arrays of the phases");
   const int gwarp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int nwarps = gridDim.x * (blockDim.x >> 5);
+  auto sync = [&]() -> bool {
+    if (!CLUSTER) return grid_sync(g);
+    cluster_sync();
+    return true;
+  };
   for (int k = 0; k < npass; k++) {
-    load_pass(sp, prog + k);
+    load_pass(sp, prog + (CLUSTER ? k & 7 : k));
+    if (CLUSTER) cluster_pass(sp, cr, k);
     chunk_relink(sp, gwarp, nwarps, sh[threadIdx.x >> 5]);
-    if (!grid_sync(g)) return;
+    if (!sync()) return;
     chunk_rows<PP>(sp, gwarp, nwarps);
-    if (!grid_sync(g)) return;
-    const int nvb = (sp.t.n + 127) / 128;
+    if (!sync()) return;
     chunk_test<PP>(sp, warps);
-    if (!grid_sync(g)) return;
+    if (!sync()) return;
     pair_fp64_body<PP>(sp.a, blockIdx.x, gridDim.x, 1);
-    if (!grid_sync(g)) return;
-    for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
-      if (sp.epi == EPI_PREDICT) fold_fp64_body<PP, EPI_PREDICT, WALLS>(sp.a, vb, stage);
-      else fold_fp64_body<PP, EPI_CORRECT, WALLS>(sp.a, vb, stage);
-      __syncthreads();
-    }
-    if (!grid_sync(g)) return;  // (also: every block is done with sp)
+    if (!sync()) return;
+    if (sp.epi == EPI_PREDICT) fold_blocks_fp64<PP, EPI_PREDICT, WALLS>(sp, stage);
+    else fold_blocks_fp64<PP, EPI_CORRECT, WALLS>(sp, stage);
+    if (!sync()) return;  // (also: every block is done with sp)
   }
 }
 

@@ -25,6 +25,10 @@ using namespace dem;
 
 namespace {
 
+// steps of one cluster launch (run_chunk), and wall slots for them
+constexpr int CLUSTER_STEPS = 32;
+constexpr int WALL_SLOTS = CLUSTER_STEPS;
+
 struct KernelStat {
   std::string name;
   long long launches = 0;
@@ -88,7 +92,8 @@ struct dem_ctx {
   // captured chunk the walls of step k come from pinned slot k, which the
   // host fills before every replay
   std::vector<dem_wall_motion> wm;
-  dem_wall* wall_slots = nullptr;  // pinned, [5][NWM]: 4 chunk slots + staging
+  dem_wall* wall_slots = nullptr;  // pinned, [WALL_SLOTS + 1][NWM]: the slots + staging
+  dem_wall* wall_dev = nullptr;    // the slots of a cluster launch in device memory
   bool capturing = false;
   bool walls_moved = false;  // MoveWalls has run at least once (at `time`)
   // UpdateParticleList after every step of dem_run (single-system contexts);
@@ -649,6 +654,8 @@ StateArrays make_state(double* base, size_t n) {
 
 constexpr int LIST_BLOCKS = 148;   // relink and list kernels (grid-stride)
 constexpr int ROWS_BLOCKS = 148 * 4;  // row kernel (grid-stride, 4 warps each)
+// systems whose steps are one launch of one cluster: a thread per sphere
+constexpr int CLUSTER_MAX = 2048;
 // systems whose relink and rows are one launch of one cluster: its 64 warps
 // rebuild this many rows at once in about a launch's time
 constexpr int MERGED_LISTS_MAX = 16384;
@@ -1606,12 +1613,13 @@ int apply_walls(dem_ctx* c, int k) {
   dem_wall* dst = reinterpret_cast<dem_wall*>(reinterpret_cast<char*>(c->dp) +
                                               offsetof(DevParams, walls));  // system 0
   c->walls_moved = true;
+  if (c->recording) return DEM_OK;  // (the launch copies the walls of each step)
   if (c->capturing) {
     CK(cudaMemcpyAsync(dst, c->wall_slots + (size_t)k * NWM, nb, cudaMemcpyHostToDevice,
                        c->stream));
     return DEM_OK;
   }
-  dem_wall* w = c->wall_slots + (size_t)4 * NWM;  // staging, not a chunk slot
+  dem_wall* w = c->wall_slots + (size_t)WALL_SLOTS * NWM;  // staging, not a chunk slot
   CK(cudaStreamSynchronize(c->stream));  // the previous upload has been read
   for (size_t j = 0; j < c->wm.size(); j++) w[j] = c->hsys[0].walls[j];
   move_walls_host(c, c->time, w);
@@ -1734,6 +1742,16 @@ int capture_steps(dem_ctx* c, int steps, cudaGraphExec_t* out) {
 bool chunk_persistent(const dem_ctx* c) {
   return c->launch_mode == 1 && c->wm.empty() && !c->fluid && !c->prof;
 }
+// A small system's steps run as one launch of one cluster (k_chunk_*,
+// CLUSTER): a pass is then a chain of latencies, to which the boundaries of
+// its four launches add.  One cluster is 2,048 threads: up to that many
+// spheres it is ahead (hopper of 600 in motion: 54.1 -> 44.3 us per step,
+// 2,000 on a floor: 53.6 -> 51.4, 300: 47.8 -> 42.2), past it the spheres
+// take turns (4,000: 57 -> 71).
+bool chunk_cluster(const dem_ctx* c) {
+  return c->launch_mode == 0 && c->nsys == 1 && !c->fluid && !c->prof && !c->slab && c->n > 0 &&
+         c->n <= CLUSTER_MAX;
+}
 
 // Record `steps` MoveParticles steps as the passes of one persistent chunk
 // into prog[phase] (the host bookkeeping is left as it was, as by
@@ -1783,39 +1801,55 @@ cudaError_t coop_launch64(K k, const ChunkPass64* prog, int npass, GridSync g, i
   const int nb = std::min(want, per * sms);
   if (nb <= 0) return cudaErrorLaunchOutOfResources;
   g.expected += (unsigned)nb;  // (on entry: the blocks a test adds to every barrier)
-  void* args[] = {(void*)&prog, (void*)&npass, (void*)&g};
+  ClusterRun cr{};
+  void* args[] = {(void*)&prog, (void*)&npass, (void*)&g, (void*)&cr};
   if (blocks_out) *blocks_out = nb;
   return cudaLaunchCooperativeKernel((const void*)k, dim3(nb), dim3(128), args, 0, st);
 }
 
-// Launch the recorded chunk of rotation phase `phase`.
-int launch_chunk(dem_ctx* c, int phase) {
-  if (!c->bar) {
+// Launch the recorded chunk of rotation phase `phase`; steps > 0: as one
+// cluster, for that many steps from `first` on.
+int launch_chunk(dem_ctx* c, int phase, int first = 0, int steps = 0) {
+  ClusterRun cr{};
+  if (steps > 0) {
+    cr.stop = c->stop_on_escape ? 1 : 0;
+    if (!c->wm.empty()) {
+      fill_wall_slots(c, first, steps);  // the previous launch has completed
+      if (!c->wall_dev) CK(cudaMalloc(&c->wall_dev, sizeof(dem_wall) * NWM * WALL_SLOTS));
+      CK(cudaMemcpyAsync(c->wall_dev, c->wall_slots, sizeof(dem_wall) * NWM * (size_t)steps,
+                         cudaMemcpyHostToDevice, c->stream));
+      cr.walls = c->wall_dev;
+      cr.table = c->dp;
+      cr.nw = (int)c->wm.size();
+    }
+  } else if (!c->bar) {
     CK(cudaMalloc(&c->bar, 2 * sizeof(unsigned)));
     CK(cudaMemsetAsync(c->bar, 0, 2 * sizeof(unsigned), c->stream));
   }
-  GridSync g{c->bar, c->bar + 1, c->cnt, c->bar_limit_ns, (unsigned)c->bar_extra};
+  GridSync g{c->bar, c->bar ? c->bar + 1 : nullptr, c->cnt, c->bar_limit_ns,
+             (unsigned)c->bar_extra};
   const int want = std::max(1, (int)blocks_for(c->n, 128));
   const bool walls = c->nw_max > 0;
   cudaError_t e;
+  const int np = steps > 0 ? 2 * steps : c->prog_n[phase];
   if (c->precision == DEM_PREC_MIXED) {
     e = mixed_chunk(c->pp, walls, c->has_cone,
-                    (const ChunkPass<float4, float2, MixedView>*)c->prog[phase], c->prog_n[phase],
-                    g, want, c->stream, &c->chunk_blocks);
+                    (const ChunkPass<float4, float2, MixedView>*)c->prog[phase], np, g, want,
+                    c->stream, &c->chunk_blocks, steps > 0 ? &cr : nullptr);
   } else {
     const ChunkPass64* prog = (const ChunkPass64*)c->prog[phase];
-    const int np = c->prog_n[phase];
+#define CCASE(PPV, W)                                                                      \
+  e = steps > 0 ? launch_cluster(k_chunk_fp64<PPV, W, true>, prog, np, cr, c->stream)       \
+                : coop_launch64(k_chunk_fp64<PPV, W, false>, prog, np, g, want, c->stream, \
+                                &c->chunk_blocks)
     if (walls) {
-      e = c->pp ? coop_launch64(k_chunk_fp64<true, true>, prog, np, g, want, c->stream,
-                                &c->chunk_blocks)
-                : coop_launch64(k_chunk_fp64<false, true>, prog, np, g, want, c->stream,
-                                &c->chunk_blocks);
+      if (c->pp) CCASE(true, true);
+      else CCASE(false, true);
     } else {
-      e = c->pp ? coop_launch64(k_chunk_fp64<true, false>, prog, np, g, want, c->stream,
-                                &c->chunk_blocks)
-                : coop_launch64(k_chunk_fp64<false, false>, prog, np, g, want, c->stream,
-                                &c->chunk_blocks);
+      if (c->pp) CCASE(true, false);
+      else CCASE(false, false);
     }
+#undef CCASE
   }
   if (e != cudaSuccess) return cuda_fail(c, e, "persistent chunk launch");
   c->launches += 1;
@@ -2130,6 +2164,151 @@ int restore_order(dem_ctx* c, bool settle) {
 }
 
 
+// How dem_run issues several steps at once
+constexpr int CHUNK_GRAPH = 0;       // 4 steps replayed from a graph
+constexpr int CHUNK_PERSISTENT = 1;  // 4 steps as one cooperative launch
+constexpr int CHUNK_CLUSTER = 2;     // up to CLUSTER_STEPS steps as one cluster
+
+// The G steps from `step` on in one go; *done_out: the steps that ran (fewer
+// after a failed pass, whose step is then finished here), *stopped: particles
+// had left the box before the step after them, *fresh: the host mirror of the
+// counters is the last step's.
+int run_chunk(dem_ctx* c, int step, int G, int mode, int* done_out, bool* stopped, bool* fresh) {
+  const int HEADROOM = 2;
+  const double dt = c->params.time_step;
+  *stopped = false;
+  int st = read_counters(c);
+  if (st) return st;
+  if (c->hcnt->need_capacity + HEADROOM > c->hcap) {
+    st = grow_history(c, c->hcnt->need_capacity + HEADROOM);
+    if (st) return st;
+  }
+  if (c->hcnt->need_in + HEADROOM > c->in_cap) {
+    st = grow_incoming(c, c->hcnt->need_in + HEADROOM);
+    if (st) return st;
+  }
+  if (c->hcnt->need_cl + c->hcnt->need_cl / 16 > c->cl_cap) {
+    st = grow_contacts(c, c->hcnt->need_cl + c->hcnt->need_cl / 8);
+    if (st) return st;
+  }
+  // a graph starts from prepared Particle copies
+  if (c->prepared != 0) {
+    st = prepare_side(c, 0);
+    if (st) return st;
+  }
+  // one graph (or recorded persistent chunk) per rotation phase (ring
+  // spare slot, history parity, list parity)
+  int phase = (c->nprev > 0 ? c->ringmap[c->nprev] : 0) * 4 + c->hcur * 2 + c->par;
+  if (mode != CHUNK_GRAPH) {
+    if (!c->prog[phase]) {
+      st = record_chunk(c, 4, phase);
+      if (st) return st;
+    }
+    st = mode == CHUNK_CLUSTER ? launch_chunk(c, phase, step, G) : launch_chunk(c, phase);
+    if (st) return st;
+  } else {
+    if (!c->graph_valid) {
+      for (auto& g : c->graph) g = nullptr;
+      c->graph_valid = true;
+    }
+    if (!c->graph[phase]) {
+      st = capture_steps(c, G, &c->graph[phase]);
+      if (st) return st;
+    }
+    fill_wall_slots(c, step, G);  // the previous replay has completed
+    CK(cudaGraphLaunch(c->graph[phase], c->stream));
+    c->launches += c->graph_kernels;
+  }
+  st = read_counters(c);
+  if (st) return st;
+  if (c->hcnt->barrier_timeout) {
+    // the chunk stopped part-way: the barrier words and flags are reset,
+    // the state is left as it is and must be set again
+    CK(cudaMemsetAsync(c->bar, 0, 2 * sizeof(unsigned), c->stream));
+    CK(cudaMemsetAsync(&c->cnt->barrier_timeout, 0, sizeof(int), c->stream));
+    CK(cudaMemsetAsync(&c->cnt->abort, 0, 2 * sizeof(int), c->stream));  // abort, abort_tag
+    CK(cudaStreamSynchronize(c->stream));
+    c->cells_ready = false;
+    drop_graphs(c);
+    return fail(c, DEM_ERR_STATE,
+                "persistent chunk: a grid-wide barrier timed out; the state is part-way "
+                "through the chunk (set it again)");
+  }
+  int done = G, failed_pass = -1;
+  bool escape_stop = false;
+  if (c->hcnt->abort) {
+    const int tag = c->hcnt->abort_tag - 1;  // 2*(step in chunk) + pass
+    if (c->hcnt->nonfinite) return fail(c, DEM_ERR_STATE, "a particle position is not finite");
+    if (c->hcnt->list_error) return fail(c, DEM_ERR_STATE, "cell lists inconsistent");
+    if (tag < 0 || tag >= 2 * G) return fail(c, DEM_ERR_STATE, "bad abort tag");
+    done = tag / 2;
+    escape_stop = c->hcnt->escape_stop != 0;
+    // an escape stop happens before the step starts: nothing to finish
+    failed_pass = escape_stop ? -1 : tag % 2;
+  }
+  for (int k = 0; k < done; k++) {
+    abm_rotate(c);
+    c->hcur ^= 1;
+  }
+  if (done > 0) {
+    c->prepared = 0;
+    c->last_side = 1;
+  }
+  step += done;
+  c->time = (double)(step - 1) * dt;
+  if (escape_stop) {
+    // the replay's later wall copies ran: back to the walls of step-1
+    st = apply_walls(c, 0);
+    if (st) return st;
+    CK(cudaMemsetAsync(&c->cnt->abort, 0, 2 * sizeof(int), c->stream));  // abort, abort_tag
+    CK(cudaMemsetAsync(&c->cnt->escape_stop, 0, sizeof(int), c->stream));
+    *done_out = done;
+    *stopped = true;
+    return DEM_OK;
+  }
+  if (failed_pass >= 0) {
+    // the replay's later wall uploads ran: back to the walls of step-1
+    st = apply_walls(c, 0);
+    if (st) return st;
+    // the failed step: its first pass ran up to the failure (relink done),
+    // or its first pass completed and its second one failed
+    c->par ^= 1;
+    if (failed_pass == 0) {
+      RingMap rm = current_map(c);
+      st = finish_pass(c, 0, true, dt, EPI_PREDICT, rm, 0);
+      if (st) return st;
+      c->last_side = 0;
+      c->prepared = 1;
+      c->hcur ^= 1;
+      abm_rotate(c);
+      c->time = (double)step * dt;
+      st = apply_walls(c, 0);
+      if (st) return st;
+      rm = current_map(c);
+      st = force_pass(c, 1, false, dt, EPI_CORRECT, rm, true, 1);
+      if (st) return st;
+    } else {
+      c->last_side = 0;
+      c->prepared = 1;
+      c->hcur ^= 1;
+      abm_rotate(c);
+      c->time = (double)step * dt;
+      st = apply_walls(c, 0);
+      if (st) return st;
+      c->par ^= 1;
+      RingMap rm = current_map(c);
+      st = finish_pass(c, 1, false, dt, EPI_CORRECT, rm, 1);
+      if (st) return st;
+      c->last_side = 1;
+      c->prepared = 0;
+    }
+    done++;
+  }
+  *done_out = done;
+  *fresh = failed_pass < 0;
+  return DEM_OK;
+}
+
 }  // namespace
 
 // ===========================================================================
@@ -2440,6 +2619,7 @@ void dem_destroy(dem_ctx* c) {
   cudaFree(c->drag);
   cudaFree(c->amsum);
   if (c->wall_slots) cudaFreeHost(c->wall_slots);
+  cudaFree(c->wall_dev);
   cudaFree(c->cellsys);
   cudaFree(c->cnt);
   if (c->hcnt) cudaFreeHost(c->hcnt);
@@ -3050,6 +3230,15 @@ int dem_move_particles(dem_ctx* c, int32_t step) {
   if (!c) return DEM_ERR_INVALID;
   int st = validate_ready(c);
   if (st) return st;
+  if (chunk_cluster(c)) {
+    // one launch and one look at the counters instead of ten and three
+    c->stop_on_escape = false;
+    int done = 0;
+    bool stopped = false, fresh = false;
+    st = run_chunk(c, step, 1, CHUNK_CLUSTER, &done, &stopped, &fresh);
+    if (st) return st;
+    return fresh ? DEM_OK : read_counters(c);
+  }
   st = move_particles_impl(c, step, true, 0);
   if (st) return st;
   CK(cudaGetLastError());
@@ -3104,21 +3293,19 @@ int dem_run(dem_ctx* c, int32_t first_step, int32_t last_step) {
   }
   int step = s0;
   const int G = 4;
-  const int HEADROOM = 2;
-  const double dt = c->params.time_step;
   int poured_step = s0 - 1;
   while (step <= last_step) {
     int remaining = last_step - step + 1;
     // PouringAttempt(Step) (src/DEM.f90:95, 115-123); a chunk holds no other
-    // pouring step, so those steps run one at a time
-    bool pour_inside = false;
+    // pouring step: the steps before one run one at a time, or as a shorter
+    // cluster launch
+    int pour_next = INT_MAX;  // steps until the next attempt
     if (pour_active(c)) {
       if (step % c->pour.interval == 0 && poured_step != step) {
         st = pour_particle_impl(c, nullptr);
         if (st) return st;
       }
-      for (int k = 1; k < G; k++)
-        if ((step + k) % c->pour.interval == 0) pour_inside = true;
+      pour_next = c->pour.interval - step % c->pour.interval;
     }
     poured_step = step;
     // the storage back into cell order every reorder_every steps
@@ -3127,7 +3314,16 @@ int dem_run(dem_ctx* c, int32_t first_step, int32_t last_step) {
       if (st) return st;
       c->since_reorder = 0;
     }
-    if (remaining < G || c->prof || pour_inside) {
+    const int mode = chunk_cluster(c) ? CHUNK_CLUSTER
+                     : chunk_persistent(c) ? CHUNK_PERSISTENT
+                                           : CHUNK_GRAPH;
+    int chunk = G;
+    if (mode == CHUNK_CLUSTER) {
+      chunk = std::min(std::min(remaining, pour_next), CLUSTER_STEPS);
+      if (c->reorder_every > 0)
+        chunk = std::min(chunk, std::max(1, c->reorder_every - (int)c->since_reorder));
+    }
+    if (remaining < chunk || c->prof || pour_next < chunk) {
       st = move_particles_impl(c, step, true, 0);
       if (st) return st;
       st = remove_escaped();
@@ -3136,135 +3332,18 @@ int dem_run(dem_ctx* c, int32_t first_step, int32_t last_step) {
       c->since_reorder++;
       continue;
     }
-    st = read_counters(c);
+    int done = 0;
+    bool stopped = false, fresh = false;
+    st = run_chunk(c, step, chunk, mode, &done, &stopped, &fresh);
     if (st) return st;
-    if (c->hcnt->need_capacity + HEADROOM > c->hcap) {
-      st = grow_history(c, c->hcnt->need_capacity + HEADROOM);
-      if (st) return st;
-    }
-    if (c->hcnt->need_in + HEADROOM > c->in_cap) {
-      st = grow_incoming(c, c->hcnt->need_in + HEADROOM);
-      if (st) return st;
-    }
-    if (c->hcnt->need_cl + c->hcnt->need_cl / 16 > c->cl_cap) {
-      st = grow_contacts(c, c->hcnt->need_cl + c->hcnt->need_cl / 8);
-      if (st) return st;
-    }
-    // a graph starts from prepared Particle copies
-    if (c->prepared != 0) {
-      st = prepare_side(c, 0);
-      if (st) return st;
-    }
-    // one graph (or recorded persistent chunk) per rotation phase (ring
-    // spare slot, history parity, list parity)
-    int phase = (c->nprev > 0 ? c->ringmap[c->nprev] : 0) * 4 + c->hcur * 2 + c->par;
-    if (chunk_persistent(c)) {
-      if (!c->prog[phase]) {
-        st = record_chunk(c, G, phase);
-        if (st) return st;
-      }
-      st = launch_chunk(c, phase);
-      if (st) return st;
-    } else {
-      if (!c->graph_valid) {
-        for (auto& g : c->graph) g = nullptr;
-        c->graph_valid = true;
-      }
-      if (!c->graph[phase]) {
-        st = capture_steps(c, G, &c->graph[phase]);
-        if (st) return st;
-      }
-      fill_wall_slots(c, step, G);  // the previous replay has completed
-      CK(cudaGraphLaunch(c->graph[phase], c->stream));
-      c->launches += c->graph_kernels;
-    }
-    st = read_counters(c);
-    if (st) return st;
-    if (c->hcnt->barrier_timeout) {
-      // the chunk stopped part-way: the barrier words and flags are reset,
-      // the state is left as it is and must be set again
-      CK(cudaMemsetAsync(c->bar, 0, 2 * sizeof(unsigned), c->stream));
-      CK(cudaMemsetAsync(&c->cnt->barrier_timeout, 0, sizeof(int), c->stream));
-      CK(cudaMemsetAsync(&c->cnt->abort, 0, 2 * sizeof(int), c->stream));  // abort, abort_tag
-      CK(cudaStreamSynchronize(c->stream));
-      c->cells_ready = false;
-      drop_graphs(c);
-      return fail(c, DEM_ERR_STATE,
-                  "persistent chunk: a grid-wide barrier timed out; the state is part-way "
-                  "through the chunk (set it again)");
-    }
-    int done = G, failed_pass = -1;
-    bool escape_stop = false;
-    if (c->hcnt->abort) {
-      const int tag = c->hcnt->abort_tag - 1;  // 2*(step in chunk) + pass
-      if (c->hcnt->nonfinite) return fail(c, DEM_ERR_STATE, "a particle position is not finite");
-      if (c->hcnt->list_error) return fail(c, DEM_ERR_STATE, "cell lists inconsistent");
-      if (tag < 0 || tag >= 2 * G) return fail(c, DEM_ERR_STATE, "bad abort tag");
-      done = tag / 2;
-      escape_stop = c->hcnt->escape_stop != 0;
-      // an escape stop happens before the step starts: nothing to finish
-      failed_pass = escape_stop ? -1 : tag % 2;
-    }
-    for (int k = 0; k < done; k++) {
-      abm_rotate(c);
-      c->hcur ^= 1;
-    }
-    if (done > 0) {
-      c->prepared = 0;
-      c->last_side = 1;
-    }
     step += done;
     c->since_reorder += done;
-    c->time = (double)(step - 1) * dt;
-    if (escape_stop) {
-      // the replay's later wall copies ran: back to the walls of step-1
-      st = apply_walls(c, 0);
-      if (st) return st;
-      CK(cudaMemsetAsync(&c->cnt->abort, 0, 2 * sizeof(int), c->stream));  // abort, abort_tag
-      CK(cudaMemsetAsync(&c->cnt->escape_stop, 0, sizeof(int), c->stream));
+    if (stopped) {
       st = update_particle_list_impl(c, nullptr);
       if (st) return st;
       continue;
     }
-    if (failed_pass >= 0) {
-      // the replay's later wall uploads ran: back to the walls of step-1
-      st = apply_walls(c, 0);
-      if (st) return st;
-      // the failed step: its first pass ran up to the failure (relink done),
-      // or its first pass completed and its second one failed
-      c->par ^= 1;
-      if (failed_pass == 0) {
-        RingMap rm = current_map(c);
-        st = finish_pass(c, 0, true, dt, EPI_PREDICT, rm, 0);
-        if (st) return st;
-        c->last_side = 0;
-        c->prepared = 1;
-        c->hcur ^= 1;
-        abm_rotate(c);
-        c->time = (double)step * dt;
-        st = apply_walls(c, 0);
-        if (st) return st;
-        rm = current_map(c);
-        st = force_pass(c, 1, false, dt, EPI_CORRECT, rm, true, 1);
-        if (st) return st;
-      } else {
-        c->last_side = 0;
-        c->prepared = 1;
-        c->hcur ^= 1;
-        abm_rotate(c);
-        c->time = (double)step * dt;
-        st = apply_walls(c, 0);
-        if (st) return st;
-        c->par ^= 1;
-        RingMap rm = current_map(c);
-        st = finish_pass(c, 1, false, dt, EPI_CORRECT, rm, 1);
-        if (st) return st;
-        c->last_side = 1;
-        c->prepared = 0;
-      }
-      step++;
-    }
-    st = remove_escaped(failed_pass < 0);  // escapes of the chunk's last step
+    st = remove_escaped(fresh);  // escapes of the chunk's last step
     if (st) return st;
   }
   CK(cudaGetLastError());
@@ -3425,7 +3504,7 @@ int dem_set_wall_motion(dem_ctx* c, const dem_wall_motion* motion) {
           !std::isfinite(m.phase_angle[k]) || m.two_pi_frequency[k] < 0.0)
         return fail(c, DEM_ERR_INVALID, "wall motion must be finite with frequency >= 0");
     }
-  if (!c->wall_slots) CK(cudaMallocHost(&c->wall_slots, sizeof(dem_wall) * NWM * 5));
+  if (!c->wall_slots) CK(cudaMallocHost(&c->wall_slots, sizeof(dem_wall) * NWM * (WALL_SLOTS + 1)));
   c->wm.assign(motion, motion + nw);
   return DEM_OK;
 }

@@ -635,11 +635,25 @@ __global__ void __launch_bounds__(128, 5)
 // exactly as in k_pair_mixed / k_fold_mixed.
 using ChunkPassMx = ChunkPass<float4, float2, MixedView>;
 
-template <bool PP, bool WALLS, bool CONE>
-__global__ void __launch_bounds__(128, 4) k_chunk_mixed(const ChunkPassMx* __restrict__ prog,
-                                                        int npass, GridSync g) {
+// the fold phase of this block
+template <bool PP, int EPI, bool WALLS, bool CONE>
+__device__ __forceinline__ void fold_blocks_mixed(const ChunkPassMx& sp, double* stage) {
+  const int nvb = (sp.t.n + 127) / 128;
+  for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
+    fold_mixed_body<PP, EPI, WALLS, CONE>(sp.a, sp.v, vb, stage);
+    __syncthreads();
+  }
+}
+// CLUSTER: the launch is one cluster instead (ClusterRun), for systems so
+// small that a pass is a chain of latencies: no launch boundaries, a hardware
+// barrier between the phases, npass passes of a program of 8 that repeats, and
+// the whole register file of an SM for each block.
+template <bool PP, bool WALLS, bool CONE, bool CLUSTER>
+__global__ void __launch_bounds__(128, CLUSTER ? 1 : 3)
+    k_chunk_mixed(const ChunkPassMx* __restrict__ prog, int npass, GridSync g, ClusterRun cr) {
   __shared__ ChunkPassMx sp;
-  __shared__ __align__(16) double stage[EpiStage<EPI_PREDICT, true>::SIZE];  // (the larger of the two)
+  // (the larger of the two epilogues')
+  __shared__ __align__(16) double stage[EpiStage<EPI_PREDICT, true>::SIZE];
   // (the relink's and the test's shared arrays lie in the fold's columns)
   int(*const sh)[RELINK_ROOM] = reinterpret_cast<int(*)[RELINK_ROOM]>(stage);
   TestWarp* const warps = reinterpret_cast<TestWarp*>(stage);
@@ -647,23 +661,25 @@ __global__ void __launch_bounds__(128, 4) k_chunk_mixed(const ChunkPassMx* __res
                 "shared arrays of the phases");
   const int gwarp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int nwarps = gridDim.x * (blockDim.x >> 5);
+  auto sync = [&]() -> bool {
+    if (!CLUSTER) return grid_sync(g);
+    cluster_sync();
+    return true;
+  };
   for (int k = 0; k < npass; k++) {
-    load_pass(sp, prog + k);
+    load_pass(sp, prog + (CLUSTER ? k & 7 : k));
+    if (CLUSTER) cluster_pass(sp, cr, k);
     chunk_relink(sp, gwarp, nwarps, sh[threadIdx.x >> 5]);
-    if (!grid_sync(g)) return;
+    if (!sync()) return;
     chunk_rows<PP>(sp, gwarp, nwarps);
-    if (!grid_sync(g)) return;
-    const int nvb = (sp.t.n + 127) / 128;
+    if (!sync()) return;
     chunk_test<PP>(sp, warps);
-    if (!grid_sync(g)) return;
+    if (!sync()) return;
     pair_mixed_body<PP>(sp.a, sp.v, blockIdx.x, gridDim.x, 1);
-    if (!grid_sync(g)) return;
-    for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
-      if (sp.epi == EPI_PREDICT) fold_mixed_body<PP, EPI_PREDICT, WALLS, CONE>(sp.a, sp.v, vb, stage);
-      else fold_mixed_body<PP, EPI_CORRECT, WALLS, CONE>(sp.a, sp.v, vb, stage);
-      __syncthreads();
-    }
-    if (!grid_sync(g)) return;  // (also: every block is done with sp)
+    if (!sync()) return;
+    if (sp.epi == EPI_PREDICT) fold_blocks_mixed<PP, EPI_PREDICT, WALLS, CONE>(sp, stage);
+    else fold_blocks_mixed<PP, EPI_CORRECT, WALLS, CONE>(sp, stage);
+    if (!sync()) return;  // (also: every block is done with sp)
   }
 }
 
@@ -744,7 +760,8 @@ cudaError_t launch_chunk(K k, const ChunkPassMx* prog, int npass, GridSync g, in
   const int nb = coop_blocks(k, want);
   if (nb <= 0) return cudaErrorLaunchOutOfResources;
   g.expected += (unsigned)nb;  // (on entry: the blocks a test adds to every barrier)
-  void* args[] = {(void*)&prog, (void*)&npass, (void*)&g};
+  ClusterRun cr{};
+  void* args[] = {(void*)&prog, (void*)&npass, (void*)&g, (void*)&cr};
   if (blocks_out) *blocks_out = nb;
   return cudaLaunchCooperativeKernel((const void*)k, dim3(nb), dim3(128), args, 0, st);
 }
@@ -912,9 +929,12 @@ void mixed_pass(MixedBuffers& M, bool pp, int epi, int variant, bool walls, bool
 
 cudaError_t mixed_chunk(bool pp, bool walls, bool cone,
                         const ChunkPass<float4, float2, MixedView>* prog, int npass, GridSync g,
-                        int want_blocks, cudaStream_t st, int* blocks_out) {
-#define CCASE(PPV, W, CN) \
-  return launch_chunk(k_chunk_mixed<PPV, W, CN>, prog, npass, g, want_blocks, st, blocks_out)
+                        int want_blocks, cudaStream_t st, int* blocks_out,
+                        const ClusterRun* cluster) {
+#define CCASE(PPV, W, CN)                                                                      \
+  return cluster ? launch_cluster(k_chunk_mixed<PPV, W, CN, true>, prog, npass, *cluster, st)  \
+                 : launch_chunk(k_chunk_mixed<PPV, W, CN, false>, prog, npass, g, want_blocks, \
+                                st, blocks_out)
   if (!walls) {
     if (pp) CCASE(true, false, false);
     CCASE(false, false, false);

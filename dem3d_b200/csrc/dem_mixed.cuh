@@ -66,7 +66,8 @@ void mixed_pass(MixedBuffers& M, bool pp, int epi, int variant, bool walls, bool
 // holds the blocks a test adds to every barrier (0 normally).
 cudaError_t mixed_chunk(bool pp, bool walls, bool cone,
                         const ChunkPass<float4, float2, MixedView>* prog, int npass, GridSync g,
-                        int want_blocks, cudaStream_t st, int* blocks_out);
+                        int want_blocks, cudaStream_t st, int* blocks_out,
+                        const ClusterRun* cluster);
 void mixed_import_history(MixedBuffers& M, const History& H, int n, int nw, int cur,
                           cudaStream_t st);
 void mixed_export_history(MixedBuffers& M, const History& H, int n, int nw, int cur,

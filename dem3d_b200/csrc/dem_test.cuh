@@ -998,6 +998,21 @@ struct GridSync {
   unsigned expected;
 };
 
+// A launch of one cluster (small systems): the hardware cluster barrier, the
+// walls of each step of the launch (copied into the system's table after the
+// step's predictor; NULL: walls at rest) and whether escapes stop the launch.
+struct ClusterRun {
+  const dem_wall* walls;
+  DevParams* table;
+  int nw, stop;
+};
+// release / acquire at cluster scope: what every thread of the cluster wrote
+// before is visible to every thread after
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n"
+               "barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 __device__ __forceinline__ unsigned long long global_ns() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -1048,6 +1063,38 @@ __device__ __forceinline__ bool grid_sync(const GridSync& g) {
 
 struct NoView {};
 
+// Host side: `k` (a chunk kernel) as one cluster of 16 blocks, or of 8 where
+// the device does not take 16.
+template <class K, class CP>
+inline cudaError_t launch_cluster(K k, const CP* prog, int npass, ClusterRun cr,
+                                  cudaStream_t st) {
+  cudaError_t e =
+      cudaFuncSetAttribute((const void*)k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e != cudaSuccess) return e;
+  for (unsigned size = 16; size >= 8; size /= 2) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(size);
+    cfg.blockDim = dim3(128);
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = size;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int fit = 0;
+    if (size > 8) {
+      e = cudaOccupancyMaxActiveClusters(&fit, (const void*)k, &cfg);
+      if (e != cudaSuccess || fit < 1) {
+        (void)cudaGetLastError();
+        continue;
+      }
+    }
+    return cudaLaunchKernelEx(&cfg, k, prog, npass, GridSync{}, cr);
+  }
+  return cudaErrorLaunchOutOfResources;
+}
+
 // One force pass of a chunk: its relink, test and pass arguments, the
 // integrator epilogue (EPI_PREDICT / EPI_CORRECT) and, for the mixed path,
 // the FP32 record arrays it reads and writes.  16-byte aligned: blocks copy
@@ -1080,6 +1127,25 @@ __device__ __noinline__ void chunk_test(const CP& p, TestWarp* warps) {
     test_body<PP, false>(p.t, vb, warps);
     __syncthreads();
   }
+}
+
+// The start of pass k of a cluster launch: its own tag (the pass number in the
+// launch; the program repeats every 8 passes), the escape stop before a
+// step's first pass, and the walls of the step before its second one.
+template <class CP>
+__device__ __forceinline__ void cluster_pass(CP& p, const ClusterRun& c, int k) {
+  if (threadIdx.x == 0) {
+    p.t.tag = k;
+    p.a.tag = k;
+    p.rl.stop_tag = c.stop && (k & 1) == 0 ? k : -1;
+  }
+  if (c.walls && (k & 1) && blockIdx.x == 0) {
+    const int words = c.nw * (int)(sizeof(dem_wall) / sizeof(double));
+    const double* src = (const double*)(c.walls + (size_t)(k >> 1) * NWM);
+    double* dst = (double*)c.table->walls;  // (one system)
+    for (int i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];
+  }
+  __syncthreads();
 }
 
 // the pass `src` into the block's shared copy `dst`

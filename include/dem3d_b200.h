@@ -371,8 +371,9 @@ int dem_get_row_stats(dem_ctx* ctx, int64_t* candidates, int32_t* row_capacity);
 /* Tuning (no counterpart in the reference).  skin_factor: candidate-row skin
  * as a fraction of CutOff (0.05 by default; larger = longer rows, fewer full
  * row rebuilds); pass_variant: the contact kernel's block budget, compiled
- * for 4 (0, default), 3 (1) or 5 (2) resident blocks of 128 threads per SM
- * (fewer registers per thread, more warps to hide memory latency).  Neither
+ * for 4 (0, default), 3 (1) or 5 (2) resident blocks of 128 threads per SM,
+ * in mixed precision 6, 4 or 8 (fewer registers per thread, more warps to
+ * hide memory latency).  Neither
  * changes any result: the rows stay complete and in sweep order, and the
  * arithmetic is the same code. */
 int dem_set_tuning(dem_ctx* ctx, double skin_factor, int32_t pass_variant);
@@ -381,8 +382,10 @@ int dem_get_tuning(dem_ctx* ctx, double* skin_factor, int32_t* pass_variant);
  * same bodies run over the same particles and contacts, and every sum keeps
  * its order).
  *  - launch_mode: how dem_run issues its 4-step chunks.  0 (default): a
- *    CUDA graph of the chunk's kernels (relink, test, pair, fold per force
- *    pass: 8 launches per step).  1: one persistent cooperative launch per
+ *    CUDA graph of the chunk's kernels (relink, rows, test, pair, fold per
+ *    force pass: 10 launches per step; 8 up to 16,384 particles); one system
+ *    of up to 2,048 particles without fluid drag runs its steps (also that of
+ *    dem_move_particles) as one launch of one thread-block cluster.  1: one persistent cooperative launch per
  *    chunk, as many blocks of 128 threads as fit on the GPU at once, which
  *    step through the 8 passes' phases with grid-wide barriers between them
  *    (every wait bounded: see dem_set_persistent_barrier).  Chunks with

@@ -7,6 +7,7 @@ import numpy as np
 import pytest
 
 from dem3d_b200 import configs
+from dem3d_b200 import params as P
 from dem3d_b200.system import DEMSystem
 from tests.oracle_lib import oracle_system
 
@@ -52,3 +53,36 @@ def test_rows_follow_the_oracle(name):
     assert g.ncol() == o.ncol() > 0
     g.close()
     o.close()
+
+
+@pytest.mark.parametrize("n,precision", [(1, 0), (127, 0), (2047, 0), (2048, 1), (2049, 0)])
+def test_cluster_steps_equal_single_calls(n, precision):
+    """The largest systems whose steps are one cluster launch and the smallest
+    past them: runs of 33 and 1 steps (a full launch and a remainder), with a
+    moving floor, against one call per step; FP64 against the oracle too."""
+    def make(factory):
+        w = configs.settling(n=n, layer_side=12, sigma_v=3.0, euler_intervals=2,
+                             max_ncell=1 << 30)
+        w.params.precision = precision
+        s = factory(w.params)
+        s.set_state(w.pos, w.vel, w.omega, comp=w.comp)
+        z = w.params.walls[0].position[2]
+        s.set_wall_motion([P.wall_motion((0.0, 0.0, z), (0.0, 0.0, 0.05), (0.0, 0.0, 20.0),
+                                         (0.0, 0.0, 0.25))])
+        s.initialize_cell_distribution()
+        return s
+    a, b = make(DEMSystem), make(DEMSystem)
+    a.run(1, 36)
+    a.run(37, 37)
+    b.run(1, 3)
+    for k in range(4, 38):
+        b.move_particles(k)
+    other = [b] if precision else [b, make(oracle_system)]
+    if not precision:
+        other[1].run(1, 37)
+    for o in other:
+        x, y = a.get_state(), o.get_state()
+        for k in x:
+            np.testing.assert_array_equal(x[k], y[k], err_msg=k)
+        assert a.ncol() == o.ncol()
+        np.testing.assert_array_equal(a.walls()["position"], o.walls()["position"])
