@@ -637,9 +637,11 @@ __global__ void __launch_bounds__(LIST_THREADS) k_relink(RelinkArgs R) {
               blockIdx.x * (LIST_THREADS / 32) + w, gridDim.x * (LIST_THREADS / 32), sh[w]);
 }
 
-// The candidate rows of the pass (rows_body), a warp per row.
+// The candidate rows of the pass (rows_body), a warp per row.  (Constant
+// parameters: the row builders are calls that take them by address, and a
+// parameter that may change is copied to every thread's stack for that.)
 template <bool PP>
-__global__ void __launch_bounds__(128) k_rows(TestArgs A) {
+__global__ void __launch_bounds__(128) k_rows(const __grid_constant__ TestArgs A) {
   pass_kernel_entry();
   rows_body<PP>(A, blockIdx.x * 4 + (threadIdx.x >> 5), gridDim.x * 4);
 }
@@ -650,7 +652,7 @@ __global__ void __launch_bounds__(128) k_rows(TestArgs A) {
 // 12.5k spheres 70.9 -> 67.8 us per step, 2,000 spheres 59.4 -> 53.9).
 template <bool PP>
 __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(LIST_THREADS)
-    k_lists(RelinkArgs R, TestArgs A) {
+    k_lists(const __grid_constant__ RelinkArgs R, const __grid_constant__ TestArgs A) {
   pass_kernel_entry();
   __shared__ int sh[LIST_THREADS / 32][RELINK_ROOM];
   const int w = threadIdx.x >> 5;
@@ -686,9 +688,12 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(LIST_THREADS)
 
 // BS threads per block.  STRIDE: grid-stride over blocks of BS particles (a
 // grid smaller than the particle count gives each thread several particles);
-// else one block of particles per block.
+// else one block of particles per block.  (Register budget: 7 blocks of 128
+// threads per SM, 72 registers; at 8 it spills, 64 against 60 us per launch
+// at 1M spheres.  Half of the issue slots and 60% of the L1's throughput are
+// in use: the gathers of the candidates' positions.)
 template <bool PP, int BS, bool STRIDE>
-__global__ void __launch_bounds__(BS, 8 * 128 / BS) k_test(TestArgs A) {
+__global__ void __launch_bounds__(BS, 7 * 128 / BS) k_test(TestArgs A) {
   pass_kernel_entry();
   __shared__ TestWarp warps[BS / 32];
   if (!STRIDE) {
@@ -841,7 +846,7 @@ __global__ void __launch_bounds__(128, MINB) k_pair_fp64(PassArgs<double4, doubl
 // The fold kernel (FP64): p's block of the sweep, its Force and Torque in
 // sweep order, a = F/m, alpha = T/I, then the integrator epilogue.  WALLS:
 // some system has walls.
-template <bool PP, int EPI, bool WALLS>
+template <bool PP, int EPI, bool WALLS, bool WAIT = false>
 __device__ __forceinline__ void fold_fp64_body(const PassArgs<double4, double2>& A, int vblock,
                                                double* stage) {
   __shared__ double s_w[WALLS ? NWM : 1][128];  // |FN| of each wall contact
@@ -853,13 +858,17 @@ __device__ __forceinline__ void fold_fp64_body(const PassArgs<double4, double2>&
   stage_epilogue<EPI, false>(A, vblock * blockDim.x, stage);
   const int c = A.cell_cur[p];
   const int rank = A.rank[p];
-  const int ni = A.in_cnt[p];
-  const unsigned matched = A.matched[p];
   const int nc = A.ccount[p];
   const int st0 = A.cstart[p];
   const double4 p4 = ld32(A.X + p);
   const double4 pv4 = ld32(A.v4 + p);
   const double2 pw2 = A.w2[p];
+  // (none of these are written by the pair kernel, and when this kernel is
+  // scheduled the kernels before that one have completed: see
+  // pass_kernel_entry)
+  if (WAIT) pass_kernel_entry();
+  const int ni = A.in_cnt[p];
+  const unsigned matched = A.matched[p];
   // one decision for the warp (with walls, for the block: it meets block
   // barriers later)
   int stop = 0;
@@ -1069,12 +1078,12 @@ __device__ __forceinline__ void fold_fp64_body(const PassArgs<double4, double2>&
 // read in 32-byte pieces.)
 template <bool PP, int EPI, bool WALLS, bool STRIDE>
 __global__ void __launch_bounds__(128, WALLS ? 4 : 5) k_fold_fp64(PassArgs<double4, double2> A) {
-  pass_kernel_entry();
   __shared__ __align__(16) double stage[EpiStage<EPI, false>::SIZE];
   if (!STRIDE) {
-    fold_fp64_body<PP, EPI, WALLS>(A, blockIdx.x, stage);
+    fold_fp64_body<PP, EPI, WALLS, true>(A, blockIdx.x, stage);
     return;
   }
+  pass_kernel_entry();
   const int nvb = (A.n + 127) / 128;
   for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
     fold_fp64_body<PP, EPI, WALLS>(A, vb, stage);

@@ -25,8 +25,7 @@ __device__ __forceinline__ double image_rn(double r, const Box& B, int k) {
   return __dsub_rn(r, __dmul_rn(B.lbox[k], (double)(int)round(__dmul_rn(r, B.inv_lbox[k]))));
 }
 __device__ __forceinline__ double sumsq3_rn(const double a[3]) {
-  double c = 0.0;
-  c = __dadd_rn(c, __dmul_rn(a[0], a[0]));
+  double c = __dmul_rn(a[0], a[0]);  // (0.0 + a square: the square itself)
   c = __dadd_rn(c, __dmul_rn(a[1], a[1]));
   c = __dadd_rn(c, __dmul_rn(a[2], a[2]));
   return c;
@@ -576,10 +575,11 @@ __device__ __noinline__ void build_row(const DevParams& P, int n, int p, int c,
 // that it needs for one row on its own (1M rows: 1.5 ms a warp per row).
 // false: a list does not fit the slots, nothing is written.
 template <bool PP>
-__device__ __noinline__ bool build_row_thread(const DevParams& P, int n, int p, int c,
-                                              const double4* __restrict__ X,
-                                              const int* __restrict__ comp, const CellLists& L,
-                                              const Rows& R, Counters* cnt, int tag) {
+__device__ __forceinline__ bool build_row_thread(const DevParams& P, int n, int p, int c,
+                                                 const double4* __restrict__ X,
+                                                 const int* __restrict__ comp,
+                                                 const CellLists& L, const Rows& R,
+                                                 Counters* cnt, int tag) {
   const double4 p4 = ld32(X + p);
   const int cp = PP ? 0 : comp[p];
   int cx, cy, cz;
@@ -840,19 +840,25 @@ __device__ __forceinline__ void test_body(const TestArgs& A, int vblock, TestWar
     const int lo = w0 > off ? w0 - off : 0;
     const int hi = off + m < w0 + WIN ? m : w0 + WIN - off;
     const unsigned short own = (unsigned short)((cp << 8) | lane);
-    for (int k = lo; k < hi; k++) {
-      const int f = off + k - w0;
-      int q;
-      if (k < 4) {
-        q = q0[0];
-        if (k == 1) q = q0[1];
-        if (k == 2) q = q0[2];
-        if (k == 3) q = q0[3];
-      } else {
-        q = ld_row<NC>(A.cand + (size_t)k * n + p);
+    int* const wq = W.q + (off - w0);
+    unsigned short* const wo = W.own + (off - w0);
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      if (k >= lo && k < hi) {
+        wq[k] = q0[k];
+        wo[k] = own;
       }
-      W.q[f] = q;
-      W.own[f] = own;
+    for (int k0 = lo > 4 ? lo : 4; k0 < hi; k0 += 4) {
+      int q[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        if (k0 + u < hi) q[u] = ld_row<NC>(A.cand + (size_t)(k0 + u) * n + p);
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        if (k0 + u < hi) {
+          wq[k0 + u] = q[u];
+          wo[k0 + u] = own;
+        }
     }
     __syncwarp();
     const int Tw = T - w0 < WIN ? T - w0 : WIN;
