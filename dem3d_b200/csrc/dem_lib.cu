@@ -2172,12 +2172,12 @@ constexpr int CHUNK_CLUSTER = 2;     // up to CLUSTER_STEPS steps as one cluster
 // The G steps from `step` on in one go; *done_out: the steps that ran (fewer
 // after a failed pass, whose step is then finished here), *stopped: particles
 // had left the box before the step after them, *fresh: the host mirror of the
-// counters is the last step's.
+// counters is the last step's (on entry: it is the latest already).
 int run_chunk(dem_ctx* c, int step, int G, int mode, int* done_out, bool* stopped, bool* fresh) {
   const int HEADROOM = 2;
   const double dt = c->params.time_step;
   *stopped = false;
-  int st = read_counters(c);
+  int st = *fresh ? DEM_OK : read_counters(c);
   if (st) return st;
   if (c->hcnt->need_capacity + HEADROOM > c->hcap) {
     st = grow_history(c, c->hcnt->need_capacity + HEADROOM);
@@ -3294,8 +3294,12 @@ int dem_run(dem_ctx* c, int32_t first_step, int32_t last_step) {
   int step = s0;
   const int G = 4;
   int poured_step = s0 - 1;
+  // the host mirror of the counters is the last chunk's, so that the next one
+  // need not wait for them again
+  bool fresh = false;
   while (step <= last_step) {
     int remaining = last_step - step + 1;
+    const int n_before = c->n;
     // PouringAttempt(Step) (src/DEM.f90:95, 115-123); a chunk holds no other
     // pouring step: the steps before one run one at a time, or as a shorter
     // cluster launch
@@ -3304,6 +3308,7 @@ int dem_run(dem_ctx* c, int32_t first_step, int32_t last_step) {
       if (step % c->pour.interval == 0 && poured_step != step) {
         st = pour_particle_impl(c, nullptr);
         if (st) return st;
+        fresh = false;
       }
       pour_next = c->pour.interval - step % c->pour.interval;
     }
@@ -3313,6 +3318,7 @@ int dem_run(dem_ctx* c, int32_t first_step, int32_t last_step) {
       st = reorder_by_cell(c);
       if (st) return st;
       c->since_reorder = 0;
+      fresh = false;
     }
     const int mode = chunk_cluster(c) ? CHUNK_CLUSTER
                      : chunk_persistent(c) ? CHUNK_PERSISTENT
@@ -3328,12 +3334,13 @@ int dem_run(dem_ctx* c, int32_t first_step, int32_t last_step) {
       if (st) return st;
       st = remove_escaped();
       if (st) return st;
+      fresh = false;
       step++;
       c->since_reorder++;
       continue;
     }
     int done = 0;
-    bool stopped = false, fresh = false;
+    bool stopped = false;
     st = run_chunk(c, step, chunk, mode, &done, &stopped, &fresh);
     if (st) return st;
     step += done;
@@ -3341,9 +3348,11 @@ int dem_run(dem_ctx* c, int32_t first_step, int32_t last_step) {
     if (stopped) {
       st = update_particle_list_impl(c, nullptr);
       if (st) return st;
+      fresh = false;
       continue;
     }
     st = remove_escaped(fresh);  // escapes of the chunk's last step
+    if (c->n != n_before) fresh = false;
     if (st) return st;
   }
   CK(cudaGetLastError());
