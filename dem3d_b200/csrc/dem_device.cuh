@@ -118,7 +118,10 @@ struct Counters {
 struct History {
   int* cnt;       // [n] records held by particle
   int* key;       // [cap*n] partner
-  double2* val;   // [cap*n*3] (ft.x,ft.y) (ft.z,vt.x) (vt.y,vt.z)
+  // record k: val[2k], val[2k + 1] = (ft.x,ft.y) (ft.z,vt.x), one 32-byte
+  // piece, and val2[k] = (vt.y,vt.z)
+  double2* val;
+  double2* val2;
   int* wflag;     // [n*nw] wall record present
   double2* wval;  // [n*nw*3]
   int cap;

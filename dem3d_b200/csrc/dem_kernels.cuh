@@ -283,19 +283,19 @@ struct Material<true> {
 
 __device__ __forceinline__ void hist_read(const History& H, int owner, int r, double ft[3],
                                           double vt[3]) {
-  const double2* v = H.val + hslot(H, owner, r) * 3;
-  double2 a = v[0], b = v[1], c = v[2];
-  ft[0] = a.x; ft[1] = a.y; ft[2] = b.x;
-  vt[0] = b.y; vt[1] = c.x; vt[2] = c.y;
+  const size_t k = hslot(H, owner, r);
+  const double4 a = ld32((const double4*)H.val + k);
+  const double2 c = H.val2[k];
+  ft[0] = a.x; ft[1] = a.y; ft[2] = a.z;
+  vt[0] = a.w; vt[1] = c.x; vt[2] = c.y;
 }
 
 __device__ __forceinline__ void hist_write(const History& H, int owner, int r, int partner,
                                            const double ft[3], const double vt[3]) {
-  H.key[hslot(H, owner, r)] = partner;
-  double2* v = H.val + hslot(H, owner, r) * 3;
-  v[0] = make_double2(ft[0], ft[1]);
-  v[1] = make_double2(ft[2], vt[0]);
-  v[2] = make_double2(vt[1], vt[2]);
+  const size_t k = hslot(H, owner, r);
+  H.key[k] = partner;
+  st32((double4*)H.val + k, make_double4(ft[0], ft[1], ft[2], vt[0]));
+  H.val2[k] = make_double2(vt[1], vt[2]);
 }
 
 // ring store of MoveParticlesEuler (src/MDEM.f90:266-271): (v,a,alpha) -> slot
@@ -397,7 +397,8 @@ __global__ void k_hist_regrow(int n, History src, History dst) {
   dst.cnt[i] = c;
   for (int r = 0; r < c; r++) {
     dst.key[hslot(dst, i, r)] = src.key[hslot(src, i, r)];
-    for (int k = 0; k < 3; k++) dst.val[hslot(dst, i, r) * 3 + k] = src.val[hslot(src, i, r) * 3 + k];
+    for (int k = 0; k < 2; k++) dst.val[hslot(dst, i, r) * 2 + k] = src.val[hslot(src, i, r) * 2 + k];
+    dst.val2[hslot(dst, i, r)] = src.val2[hslot(src, i, r)];
   }
 }
 
@@ -409,8 +410,7 @@ __global__ void k_hist_regrow(int n, History src, History dst) {
 // FP32 record values of the mixed mode move with them (sa.. -> da.., or
 // null in FP64 mode).
 __global__ void k_hist_canon(int n, History src, History dst, const float4* __restrict__ sa,
-                             const float4* __restrict__ sb, const float* __restrict__ sc,
-                             float4* __restrict__ da, float4* __restrict__ db,
+                             const float* __restrict__ sc, float4* __restrict__ da,
                              float* __restrict__ dc, int* status) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -429,12 +429,13 @@ __global__ void k_hist_canon(int n, History src, History dst, const float4* __re
     const size_t to = hslot(dst, o, s);
     dst.key[to] = move ? i : q;
     if (sa) {
-      da[to] = sa[from];
-      db[to] = sb[from];
+      da[2 * to] = sa[2 * from];
+      da[2 * to + 1] = sa[2 * from + 1];
       dc[to] = sc[from];
     } else {
 #pragma unroll
-      for (int k = 0; k < 3; k++) dst.val[to * 3 + k] = src.val[from * 3 + k];
+      for (int k = 0; k < 2; k++) dst.val[to * 2 + k] = src.val[from * 2 + k];
+      dst.val2[to] = src.val2[from];
     }
   }
 }

@@ -450,6 +450,7 @@ void free_state(dem_ctx* c) {
     cudaFree(c->H[b].cnt);
     cudaFree(c->H[b].key);
     cudaFree(c->H[b].val);
+    cudaFree(c->H[b].val2);
     cudaFree(c->H[b].wflag);
     cudaFree(c->H[b].wval);
     c->H[b] = History{};
@@ -487,7 +488,8 @@ int alloc_history(dem_ctx* c, History& H, int cap) {
   H.n = (int)n;
   CK(cudaMalloc(&H.cnt, n * sizeof(int)));
   CK(cudaMalloc(&H.key, n * cap * sizeof(int)));
-  CK(cudaMalloc(&H.val, n * cap * 3 * sizeof(double2)));
+  CK(cudaMalloc(&H.val, n * cap * 2 * sizeof(double2)));
+  CK(cudaMalloc(&H.val2, n * cap * sizeof(double2)));
   CK(cudaMalloc(&H.wflag, n * nw * sizeof(int)));
   CK(cudaMalloc(&H.wval, n * nw * 3 * sizeof(double2)));
   CK(cudaMemsetAsync(H.cnt, 0, n * sizeof(int), c->stream));
@@ -522,6 +524,7 @@ int grow_history(dem_ctx* c, int need) {
     cudaFree(c->H[b].cnt);
     cudaFree(c->H[b].key);
     cudaFree(c->H[b].val);
+    cudaFree(c->H[b].val2);
     cudaFree(c->H[b].wflag);
     cudaFree(c->H[b].wval);
     c->H[b] = nh[b];
@@ -1286,10 +1289,9 @@ int canonical_history(dem_ctx* c) {
     CK(cudaMemsetAsync(status, 0, 2 * sizeof(int), c->stream));
     CK(cudaMemsetAsync(D.cnt, 0, sizeof(int) * (size_t)n, c->stream));
     launch(c, "hist_canon", k_hist_canon, blocks_for(n, 256), 256, n, S, D,
-           (const float4*)(mixed ? c->M.ha[cur] : nullptr),
-           (const float4*)(mixed ? c->M.hb[cur] : nullptr),
-           (const float*)(mixed ? c->M.hc[cur] : nullptr), mixed ? c->M.ha[nxt] : nullptr,
-           mixed ? c->M.hb[nxt] : nullptr, mixed ? c->M.hc[nxt] : nullptr, status);
+           (const float4*)(mixed ? c->M.h[cur] : nullptr),
+           (const float*)(mixed ? c->M.hc[cur] : nullptr), mixed ? c->M.h[nxt] : nullptr,
+           mixed ? c->M.hc[nxt] : nullptr, status);
     int hs[2] = {0, 0};
     CK(cudaMemcpyAsync(hs, status, sizeof(hs), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
@@ -1362,8 +1364,7 @@ int update_particle_list_impl(dem_ctx* c, int64_t* removed) {
       A.par = c->par;
       A.H = c->H[c->hcur];
       const bool mixed = c->precision == DEM_PREC_MIXED;
-      A.ha = mixed ? c->M.ha[c->hcur] : nullptr;
-      A.hb = mixed ? c->M.hb[c->hcur] : nullptr;
+      A.ha = mixed ? c->M.h[c->hcur] : nullptr;
       A.hc = mixed ? c->M.hc[c->hcur] : nullptr;
       A.wa = mixed ? c->M.wa[c->hcur] : nullptr;
       A.wb = mixed ? c->M.wb[c->hcur] : nullptr;
@@ -1894,11 +1895,11 @@ void slab_hist_cols(const dem_ctx* c, SlabCols& C, int b, bool walls, int rows) 
   if (rows > 0) {
     slab_col(C, H.key, 4, rows, N * 4);
     if (mixed) {
-      slab_col(C, c->M.ha[b], 16, rows, N * 16);
-      slab_col(C, c->M.hb[b], 16, rows, N * 16);
+      slab_col(C, c->M.h[b], 32, rows, N * 32);
       slab_col(C, c->M.hc[b], 4, rows, N * 4);
     } else {
-      slab_col(C, H.val, 48, rows, N * 48);
+      slab_col(C, H.val, 32, rows, N * 32);
+      slab_col(C, H.val2, 16, rows, N * 16);
     }
   }
   if (!walls) return;
@@ -2943,7 +2944,7 @@ int dem_set_contacts(dem_ctx* c, int64_t m, const int32_t* imin, const int32_t* 
   const size_t S = (size_t)c->H[c->hcur].n;  // slot stride of the tables
   cnt.assign(S, 0);
   std::vector<int> key(S * cap, -1);
-  std::vector<double2> val(S * cap * 3);
+  std::vector<double2> val(S * cap * 2), val2(S * cap);
   // records kept sorted by partner as the reference lists are
   std::vector<int64_t> idx(m);
   for (int64_t r = 0; r < m; r++) idx[r] = r;
@@ -2954,10 +2955,10 @@ int dem_set_contacts(dem_ctx* c, int64_t m, const int32_t* imin, const int32_t* 
     int64_t r = idx[q];
     int o = imin[r], k = cnt[o]++;
     key[(size_t)k * S + o] = imax[r];  // slot major
-    double2* v = &val[((size_t)k * S + o) * 3];
+    double2* v = &val[((size_t)k * S + o) * 2];
     v[0] = make_double2(ft[3 * r], ft[3 * r + 1]);
     v[1] = make_double2(ft[3 * r + 2], vt[3 * r]);
-    v[2] = make_double2(vt[3 * r + 1], vt[3 * r + 2]);
+    val2[(size_t)k * S + o] = make_double2(vt[3 * r + 1], vt[3 * r + 2]);
   }
   std::vector<int> wf(N * nw, 0);
   std::vector<double2> wv(N * nw * 3);
@@ -2974,6 +2975,7 @@ int dem_set_contacts(dem_ctx* c, int64_t m, const int32_t* imin, const int32_t* 
   CK(cudaMemcpy(H.cnt, cnt.data(), sizeof(int) * S, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(H.key, key.data(), sizeof(int) * key.size(), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(H.val, val.data(), sizeof(double2) * val.size(), cudaMemcpyHostToDevice));
+  CK(cudaMemcpy(H.val2, val2.data(), sizeof(double2) * val2.size(), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(H.wflag, wf.data(), sizeof(int) * wf.size(), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(H.wval, wv.data(), sizeof(double2) * wv.size(), cudaMemcpyHostToDevice));
   if (c->precision == DEM_PREC_MIXED) mixed_import_history(c->M, H, n, c->params.n_walls, c->hcur, c->stream);
@@ -2984,7 +2986,7 @@ int dem_set_contacts(dem_ctx* c, int64_t m, const int32_t* imin, const int32_t* 
 namespace {
 struct HostHist {
   std::vector<int> cnt, key, wf;
-  std::vector<double2> val, wv;
+  std::vector<double2> val, val2, wv;
 };
 int download_history(dem_ctx* c, HostHist& h) {
   int nw = std::max(c->params.n_walls, 1);
@@ -2998,12 +3000,14 @@ int download_history(dem_ctx* c, HostHist& h) {
   CK(cudaStreamSynchronize(c->stream));
   h.cnt.resize(N);
   h.key.resize(N * H.cap);
-  h.val.resize(N * H.cap * 3);
+  h.val.resize(N * H.cap * 2);
+  h.val2.resize(N * H.cap);
   h.wf.resize(N * nw);
   h.wv.resize(N * nw * 3);
   CK(cudaMemcpy(h.cnt.data(), H.cnt, sizeof(int) * N, cudaMemcpyDeviceToHost));
   CK(cudaMemcpy(h.key.data(), H.key, sizeof(int) * h.key.size(), cudaMemcpyDeviceToHost));
   CK(cudaMemcpy(h.val.data(), H.val, sizeof(double2) * h.val.size(), cudaMemcpyDeviceToHost));
+  CK(cudaMemcpy(h.val2.data(), H.val2, sizeof(double2) * h.val2.size(), cudaMemcpyDeviceToHost));
   CK(cudaMemcpy(h.wf.data(), H.wflag, sizeof(int) * h.wf.size(), cudaMemcpyDeviceToHost));
   CK(cudaMemcpy(h.wv.data(), H.wval, sizeof(double2) * h.wv.size(), cudaMemcpyDeviceToHost));
   return DEM_OK;
@@ -3054,9 +3058,9 @@ int dem_get_contacts(dem_ctx* c, int64_t cap, int32_t* imin, int32_t* imax, doub
   for (const Rec& q : recs) {
     imin[a] = q.lo;
     imax[a] = q.hi;
-    const double2* v = &h.val[q.slot * 3];
+    const double2 *v = &h.val[q.slot * 2], v2 = h.val2[q.slot];
     ft[3 * a] = v[0].x; ft[3 * a + 1] = v[0].y; ft[3 * a + 2] = v[1].x;
-    vt[3 * a] = v[1].y; vt[3 * a + 1] = v[2].x; vt[3 * a + 2] = v[2].y;
+    vt[3 * a] = v[1].y; vt[3 * a + 1] = v2.x; vt[3 * a + 2] = v2.y;
     a++;
   }
   for (int i = 0; i < c->n; i++)

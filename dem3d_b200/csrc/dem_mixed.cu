@@ -244,6 +244,19 @@ __device__ __forceinline__ void rec_write(float4* a, float4* b, float* c, size_t
   c[i] = lo.z;
 }
 
+// a pair record: one 32-byte piece and the last remainder
+__device__ __forceinline__ void pair_rec_read(const F8* a, const float* c, size_t i, F3& ft, F3& lo,
+                                              F3& vt) {
+  const F8 x = ld32(a + i);
+  ft = mk(x.v[0], x.v[1], x.v[2]);
+  vt = mk(x.v[3], x.v[4], x.v[5]);
+  lo = mk(x.v[6], x.v[7], c[i]);
+}
+__device__ __forceinline__ void pair_rec_write(F8* a, float* c, size_t i, F3 ft, F3 lo, F3 vt) {
+  st32(a + i, F8{{ft.x, ft.y, ft.z, vt.x, vt.y, vt.z, lo.x, lo.y}});
+  c[i] = lo.z;
+}
+
 // The mixed-precision force pass: the FP64 pass's structure (the same test
 // kernel and contact list, exact FP64 overlap test, orientation, history
 // semantics, each contact evaluated once, summation order), FP32 contact
@@ -301,7 +314,7 @@ __device__ __forceinline__ void pair_mixed_body(const PassArgs<float4, float2>& 
     const size_t hg = hslot(Hr, p, room ? ord : 0);
     const int kg = Hr.key[hg];
     F3 ft0, ft0lo, vt0;
-    rec_read(V.ra, V.rb, V.rc, hg, ft0, ft0lo, vt0);
+    pair_rec_read(V.r8, V.rc, hg, ft0, ft0lo, vt0);
     const DevParams& P = sys_params(A.P, A.sysid, p);
     const double4 p4 = ld32(A.X + p), q4 = ld32(A.X + q);
     const float4 pv4 = A.v4[p], qv4 = A.v4[q];
@@ -324,11 +337,11 @@ __device__ __forceinline__ void pair_mixed_body(const PassArgs<float4, float2>& 
       r = find_record(Hr, p, q);
       contacting = r >= 0;
       if (contacting) {
-        rec_read(V.ra, V.rb, V.rc, hslot(Hr, p, r), ft0, ft0lo, vt0);
+        pair_rec_read(V.r8, V.rc, hslot(Hr, p, r), ft0, ft0lo, vt0);
       } else {
         const int r2 = find_record(Hr, q, p);
         contacting = r2 >= 0;
-        if (contacting) rec_read(V.ra, V.rb, V.rc, hslot(Hr, q, r2), ft0, ft0lo, vt0);
+        if (contacting) pair_rec_read(V.r8, V.rc, hslot(Hr, q, r2), ft0, ft0lo, vt0);
       }
     }
     // (the fold reads the matched bits of history-updating passes only)
@@ -366,7 +379,7 @@ __device__ __forceinline__ void pair_mixed_body(const PassArgs<float4, float2>& 
       if (ord < Hw.cap) {
         const size_t i = hslot(Hw, p, ord);
         Hw.key[i] = q;
-        rec_write(V.wa, V.wb, V.wc, i, out.FT, out.FTlo, out.VT);
+        pair_rec_write(V.w8, V.wc, i, out.FT, out.FTlo, out.VT);
       } else {
         overflow = true;
       }
@@ -536,10 +549,10 @@ __device__ __forceinline__ void fold_mixed_body(const PassArgs<float4, float2>& 
         if (q2 >= A.n || !partner_adjacent(A, P, c, q2)) {
           if (hw_n < Hw.cap) {
             F3 ft, lo, vt;
-            rec_read(V.ra, V.rb, V.rc, i, ft, lo, vt);
+            pair_rec_read(V.r8, V.rc, i, ft, lo, vt);
             const size_t o = hslot(Hw, p, hw_n);
             Hw.key[o] = q2;
-            rec_write(V.wa, V.wb, V.wc, o, ft, lo, vt);
+            pair_rec_write(V.w8, V.wc, o, ft, lo, vt);
           } else {
             overflow = true;
           }
@@ -688,15 +701,15 @@ __global__ void __launch_bounds__(128, CLUSTER ? 1 : 3)
 }
 
 // FP64 records <-> FP32 records
-__global__ void k_hist_to_mixed(int n, History H, float4* a, float4* b, float* c, int nw,
-                                float4* wa, float4* wb, float* wc) {
+__global__ void k_hist_to_mixed(int n, History H, float4* a, float* c, int nw, float4* wa,
+                                float4* wb, float* wc) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   for (int r = 0; r < H.cnt[i]; r++) {
     const size_t k = hslot(H, i, r);
-    double2 x = H.val[3 * k], y = H.val[3 * k + 1], z = H.val[3 * k + 2];
-    a[k] = make_float4((float)x.x, (float)x.y, (float)y.x, (float)y.y);
-    b[k] = make_float4((float)z.x, (float)z.y, 0.f, 0.f);
+    double2 x = H.val[2 * k], y = H.val[2 * k + 1], z = H.val2[k];
+    a[2 * k] = make_float4((float)x.x, (float)x.y, (float)y.x, (float)y.y);
+    a[2 * k + 1] = make_float4((float)z.x, (float)z.y, 0.f, 0.f);
     c[k] = 0.f;
   }
   for (int w = 0; w < nw; w++) {
@@ -708,17 +721,16 @@ __global__ void k_hist_to_mixed(int n, History H, float4* a, float4* b, float* c
   }
 }
 
-__global__ void k_hist_from_mixed(int n, History H, const float4* a, const float4* b,
-                                  const float* c, int nw, const float4* wa, const float4* wb,
-                                  const float* wc) {
+__global__ void k_hist_from_mixed(int n, History H, const float4* a, const float* c, int nw,
+                                  const float4* wa, const float4* wb, const float* wc) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   for (int r = 0; r < H.cnt[i]; r++) {
     const size_t k = hslot(H, i, r);
-    float4 x = a[k], y = b[k];
-    H.val[3 * k] = make_double2((double)x.x + y.z, (double)x.y + y.w);
-    H.val[3 * k + 1] = make_double2((double)x.z + c[k], (double)x.w);
-    H.val[3 * k + 2] = make_double2((double)y.x, (double)y.y);
+    float4 x = a[2 * k], y = a[2 * k + 1];
+    H.val[2 * k] = make_double2((double)x.x + y.z, (double)x.y + y.w);
+    H.val[2 * k + 1] = make_double2((double)x.z + c[k], (double)x.w);
+    H.val2[k] = make_double2((double)y.x, (double)y.y);
   }
   for (int w = 0; w < nw; w++) {
     size_t k = (size_t)i * nw + w;
@@ -730,16 +742,15 @@ __global__ void k_hist_from_mixed(int n, History H, const float4* a, const float
 }
 
 __global__ void k_mixed_regrow(int n, int ns, int nd, const int* cnt, const float4* a,
-                               const float4* b, const float* c, float4* na, float4* nb,
-                               float* nc) {
+                               const float* c, float4* na, float* nc) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   for (int r = 0; r < cnt[i]; r++) {
     // slot-major: record r of particle i at r*stride + i, the old tables laid
     // out for ns rows, the new ones for nd
     const size_t s = (size_t)r * ns + i, d = (size_t)r * nd + i;
-    na[d] = a[s];
-    nb[d] = b[s];
+    na[2 * d] = a[2 * s];
+    na[2 * d + 1] = a[2 * s + 1];
     nc[d] = c[s];
   }
 }
@@ -783,8 +794,7 @@ bool mixed_alloc(MixedBuffers& M, int n, int nw, int cap) {
   M.cap = cap;
   bool ok = true;
   for (int b = 0; b < 2 && ok; b++) {
-    ok = cudaMalloc(&M.ha[b], N * cap * sizeof(float4)) == cudaSuccess &&
-         cudaMalloc(&M.hb[b], N * cap * sizeof(float4)) == cudaSuccess &&
+    ok = cudaMalloc(&M.h[b], N * cap * 2 * sizeof(float4)) == cudaSuccess &&
          cudaMalloc(&M.hc[b], N * cap * sizeof(float)) == cudaSuccess &&
          cudaMalloc(&M.wa[b], W * sizeof(float4)) == cudaSuccess &&
          cudaMalloc(&M.wb[b], W * sizeof(float4)) == cudaSuccess &&
@@ -796,8 +806,7 @@ bool mixed_alloc(MixedBuffers& M, int n, int nw, int cap) {
 
 void mixed_free(MixedBuffers& M) {
   for (int b = 0; b < 2; b++) {
-    cudaFree(M.ha[b]);
-    cudaFree(M.hb[b]);
+    cudaFree(M.h[b]);
     cudaFree(M.hc[b]);
     cudaFree(M.wa[b]);
     cudaFree(M.wb[b]);
@@ -809,25 +818,21 @@ void mixed_free(MixedBuffers& M) {
 bool mixed_regrow(MixedBuffers& M, int n, int stride, int newcap, int cur, const History& old,
                   cudaStream_t st) {
   size_t N = (size_t)(stride > 0 ? stride : 1);
-  float4 *na[2], *nb[2];
+  float4* na[2];
   float* nc[2];
   for (int b = 0; b < 2; b++) {
-    if (cudaMalloc(&na[b], N * newcap * sizeof(float4)) != cudaSuccess ||
-        cudaMalloc(&nb[b], N * newcap * sizeof(float4)) != cudaSuccess ||
+    if (cudaMalloc(&na[b], N * newcap * 2 * sizeof(float4)) != cudaSuccess ||
         cudaMalloc(&nc[b], N * newcap * sizeof(float)) != cudaSuccess)
       return false;
   }
   if (n > 0)
-    k_mixed_regrow<<<blocks(n, 256), 256, 0, st>>>(n, old.n, (int)N, old.cnt, M.ha[cur],
-                                                    M.hb[cur], M.hc[cur], na[cur], nb[cur],
-                                                    nc[cur]);
+    k_mixed_regrow<<<blocks(n, 256), 256, 0, st>>>(n, old.n, (int)N, old.cnt, M.h[cur], M.hc[cur],
+                                                    na[cur], nc[cur]);
   cudaStreamSynchronize(st);
   for (int b = 0; b < 2; b++) {
-    cudaFree(M.ha[b]);
-    cudaFree(M.hb[b]);
+    cudaFree(M.h[b]);
     cudaFree(M.hc[b]);
-    M.ha[b] = na[b];
-    M.hb[b] = nb[b];
+    M.h[b] = na[b];
     M.hc[b] = nc[b];
   }
   M.cap = newcap;
@@ -864,11 +869,9 @@ bool mixed_grow_walls(MixedBuffers& M, int n, int stride, int cur, cudaStream_t 
 
 MixedView mixed_view(const MixedBuffers& M, int cur) {
   MixedView V;
-  V.ra = M.ha[cur];
-  V.rb = M.hb[cur];
+  V.r8 = (const F8*)M.h[cur];
   V.rc = M.hc[cur];
-  V.wa = M.ha[cur ^ 1];
-  V.wb = M.hb[cur ^ 1];
+  V.w8 = (F8*)M.h[cur ^ 1];
   V.wc = M.hc[cur ^ 1];
   V.rwa = M.wa[cur];
   V.rwb = M.wb[cur];
@@ -955,14 +958,14 @@ cudaError_t mixed_chunk(bool pp, bool walls, bool cone,
 void mixed_import_history(MixedBuffers& M, const History& H, int n, int nw, int cur,
                           cudaStream_t st) {
   if (n == 0) return;
-  k_hist_to_mixed<<<blocks(n, 256), 256, 0, st>>>(n, H, M.ha[cur], M.hb[cur], M.hc[cur], nw,
+  k_hist_to_mixed<<<blocks(n, 256), 256, 0, st>>>(n, H, M.h[cur], M.hc[cur], nw,
                                                   M.wa[cur], M.wb[cur], M.wc[cur]);
 }
 
 void mixed_export_history(MixedBuffers& M, const History& H, int n, int nw, int cur,
                           cudaStream_t st) {
   if (n == 0) return;
-  k_hist_from_mixed<<<blocks(n, 256), 256, 0, st>>>(n, H, M.ha[cur], M.hb[cur], M.hc[cur], nw,
+  k_hist_from_mixed<<<blocks(n, 256), 256, 0, st>>>(n, H, M.h[cur], M.hc[cur], nw,
                                                     M.wa[cur], M.wb[cur], M.wc[cur]);
 }
 

@@ -9,28 +9,25 @@ struct MixedBuffers {
   bool ready = false;
   int n = 0, nw = 0, cap = 0;
   // FP32 pair records (ft, vt, Kahan remainder of ft), double-buffered like
-  // the key/count tables of History: a = (ft.xyz, vt.x), b = (vt.yz, lo.xy),
-  // c = lo.z
-  float4* ha[2] = {nullptr, nullptr};
-  float4* hb[2] = {nullptr, nullptr};
+  // the key/count tables of History: record i is h[2i] = (ft.xyz, vt.x),
+  // h[2i + 1] = (vt.yz, lo.xy), one 32-byte piece, and hc[i] = lo.z
+  float4* h[2] = {nullptr, nullptr};
   float* hc[2] = {nullptr, nullptr};
-  // wall records, same packing, [n*nw]
+  // wall records [n*nw]: a = (ft.xyz, vt.x), b = (vt.yz, lo.xy), c = lo.z
   float4* wa[2] = {nullptr, nullptr};
   float4* wb[2] = {nullptr, nullptr};
   float* wc[2] = {nullptr, nullptr};
 };
 
 // The FP32 record arrays one pass reads (r*) and writes (w*): pair records
-// (a, b, c of MixedBuffers) and wall records (wa, wb, wc)
+// (h, hc of MixedBuffers) and wall records (wa, wb, wc)
 struct MixedView {
-  // history values [n*cap]: a = (ft.xyz, vt.x) b = (vt.yz, lo.xy) c = lo.z
-  const float4* ra;
-  const float4* rb;
+  // history values [n*cap]
+  const F8* r8;
   const float* rc;
-  float4* wa;
-  float4* wb;
+  F8* w8;
   float* wc;
-  // wall history values [n*nw], same packing
+  // wall history values [n*nw]
   const float4* rwa;
   const float4* rwb;
   const float* rwc;

@@ -41,7 +41,7 @@ struct RemovalArgs {
   int par;          // L.cell[par] = CellIndex
   History H;        // the live records
   // FP32 record values of the mixed mode (null in FP64 mode)
-  float4 *ha, *hb;
+  float4* ha;
   float* hc;
   float4 *wa, *wb;
   float* wc;
@@ -73,12 +73,13 @@ __global__ void k_escape_list(const DevParams* __restrict__ PT, int n, StateArra
 __device__ __forceinline__ void rm_copy_record(const RemovalArgs& A, size_t from, size_t to) {
   A.H.key[to] = A.H.key[from];
   if (A.ha) {
-    A.ha[to] = A.ha[from];
-    A.hb[to] = A.hb[from];
+    A.ha[2 * to] = A.ha[2 * from];
+    A.ha[2 * to + 1] = A.ha[2 * from + 1];
     A.hc[to] = A.hc[from];
   } else {
 #pragma unroll
-    for (int k = 0; k < 3; k++) A.H.val[to * 3 + k] = A.H.val[from * 3 + k];
+    for (int k = 0; k < 2; k++) A.H.val[to * 2 + k] = A.H.val[from * 2 + k];
+    A.H.val2[to] = A.H.val2[from];
   }
 }
 
