@@ -689,12 +689,13 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(LIST_THREADS)
 
 // BS threads per block.  STRIDE: grid-stride over blocks of BS particles (a
 // grid smaller than the particle count gives each thread several particles);
-// else one block of particles per block.  (Register budget: 7 blocks of 128
-// threads per SM, 72 registers; at 8 it spills, 64 against 60 us per launch
-// at 1M spheres.  Half of the issue slots and 60% of the L1's throughput are
-// in use: the gathers of the candidates' positions.)
+// else one block of particles per block.  (Register budget: 8 blocks of 128
+// threads per SM, 64 registers: 48 us per launch at 1M spheres; 9 and 10
+// blocks 49 and 50.  It is bound by instruction issue and by the L1's
+// throughput for the gathers of the candidates' positions; with rows of 0.3
+// candidates it takes 31 us, the latency of its blocks' allocations.)
 template <bool PP, int BS, bool STRIDE>
-__global__ void __launch_bounds__(BS, 7 * 128 / BS) k_test(TestArgs A) {
+__global__ void __launch_bounds__(BS, 8 * 128 / BS) k_test(TestArgs A) {
   pass_kernel_entry();
   __shared__ TestWarp warps[BS / 32];
   if (!STRIDE) {

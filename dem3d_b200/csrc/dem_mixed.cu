@@ -623,13 +623,16 @@ __device__ __forceinline__ void fold_mixed_body(const PassArgs<float4, float2>& 
 // (STRIDE: grid-stride over blocks of 128 particles.  The kernel is bound by
 // the latency of the contact results it gathers and by instruction issue,
 // not by its streams: the staged columns alone move at 6.2 TB/s.  Register
-// budget: 5 blocks of 128 per SM, 96 registers, no spills without cones; at 6
-// blocks the packing with 6.6 contacts per sphere loses (210 against 196 us
-// per launch at 1M spheres) what the one with 0.6 gains (119 against 126).
-// Before the columns were staged, the records read in 32-byte pieces two at
-// a time and the block barriers dropped: 212 and 142 us.)
+// budget: 5 blocks of 128 per SM, 96 registers, no spills without cones; the
+// corrector without walls, which needs fewer, 7 blocks, 72 registers (1M
+// spheres, mean of the two kernels: 127 -> 119 us per launch with 0.8
+// contacts each, 198 -> 189 with 6.6; with walls it would spill, 61 -> 65 us).
+// The predictor at 6 blocks loses on the dense packing (210 against 196) what
+// it gains on the thin one; one record in flight instead of two: 134 against
+// 127.  Before the columns were staged, the records read in 32-byte pieces
+// and the block barriers dropped: 142 and 212 us.)
 template <bool PP, int EPI, bool WALLS, bool CONE, bool STRIDE>
-__global__ void __launch_bounds__(128, 5)
+__global__ void __launch_bounds__(128, EPI == EPI_CORRECT && !WALLS ? 7 : 5)
     k_fold_mixed(PassArgs<float4, float2> A, MixedView V) {
   __shared__ __align__(16) double stage[EpiStage<EPI, true>::SIZE];
   if (!STRIDE) {

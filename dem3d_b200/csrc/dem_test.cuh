@@ -771,9 +771,10 @@ __device__ __forceinline__ void rows_body(const TestArgs& A, int warp, int nwarp
 //
 // Rows are short and uneven (2.9 candidates on average, 8 in the longest of
 // 32, at 1M spheres), so a warp lays its 32 rows end to end in shared memory
-// and its lanes test one candidate each, 128 at a time: 3 turns instead of
-// two groups of four per thread, all positions of a turn in flight together.
-// The ballots of the turns give every contact's place.  A warp whose rows
+// and its lanes test one candidate each: 3 turns instead of two groups of
+// four per thread.  (One turn at a time: two or four in flight cost the
+// registers of one or two blocks more per SM and lose, 55 and 60 against 48 us
+// per launch.)  The ballots of the turns give every contact's place.  A warp whose rows
 // hold more than WIN candidates goes through them in windows, once to count
 // and once more to write.
 // (The body of k_test for block `vblock`, so that a persistent kernel can
@@ -863,45 +864,35 @@ __device__ __forceinline__ void test_body(const TestArgs& A, int vblock, TestWar
     __syncwarp();
     const int Tw = T - w0 < WIN ? T - w0 : WIN;
     int run = 0;
-    for (int f0 = 0; f0 < Tw; f0 += 128) {
-      double4 xq[4];
+    for (int f0 = 0; f0 < Tw; f0 += 32) {
+      const int f = f0 + lane;
+      bool hit = false;
+      if (f < Tw) {
+        const int q = W.q[f];
+        const double4 xq = ld32(A.X + q);
+        const int own_f = W.own[f];
+        const double4 a = W.x[own_f & 31];
+        double Rij[3] = {__dsub_rn(xq.x, a.x), __dsub_rn(xq.y, a.y), __dsub_rn(xq.z, a.z)};
+        const DevParams* P = &P0;
+        if (one) {
+          if (!(fabs(Rij[0]) < hx)) Rij[0] = image_rn(Rij[0], P0.box, 0);
+          if (!(fabs(Rij[1]) < hy)) Rij[1] = image_rn(Rij[1], P0.box, 1);
+          if (!(fabs(Rij[2]) < hz)) Rij[2] = image_rn(Rij[2], P0.box, 2);
+        } else {
+          P = A.P + A.sysid[p0 - lane + (own_f & 31)];
 #pragma unroll
-      for (int u = 0; u < 4; u++) {
-        const int f = f0 + 32 * u + lane;
-        if (f < Tw) xq[u] = ld32(A.X + W.q[f]);
-      }
-#pragma unroll
-      for (int u = 0; u < 4; u++) {
-        const int f = f0 + 32 * u + lane;
-        bool hit = false;
-        if (f < Tw) {
-          const int own_f = W.own[f];
-          const double4 a = W.x[own_f & 31];
-          double Rij[3] = {__dsub_rn(xq[u].x, a.x), __dsub_rn(xq[u].y, a.y),
-                           __dsub_rn(xq[u].z, a.z)};
-          const DevParams* P = &P0;
-          if (one) {
-            if (!(fabs(Rij[0]) < hx)) Rij[0] = image_rn(Rij[0], P0.box, 0);
-            if (!(fabs(Rij[1]) < hy)) Rij[1] = image_rn(Rij[1], P0.box, 1);
-            if (!(fabs(Rij[2]) < hz)) Rij[2] = image_rn(Rij[2], P0.box, 2);
-          } else {
-            P = A.P + A.sysid[p0 - lane + (own_f & 31)];
-#pragma unroll
-            for (int k = 0; k < 3; k++) Rij[k] = min_image_rn(Rij[k], P->box, k);
-          }
-          const int cq = PP || P->nc == 1 ? 0 : A.comp[W.q[f]];
-          const double md = min_dij_sq_rn<PP>(*P, PP ? 0 : own_f >> 8, a.w, cq, xq[u].w);
-          hit = __dsub_rn(md, sumsq3_rn(Rij)) > 0.0;
+          for (int k = 0; k < 3; k++) Rij[k] = min_image_rn(Rij[k], P->box, k);
         }
-        if (f0 + 32 * u < Tw) {
-          const unsigned b = __ballot_sync(FULL, hit);
-          if (lane == 0) {
-            W.mask[(f0 >> 5) + u] = b;
-            W.pre[(f0 >> 5) + u] = run;
-          }
-          run += __popc(b);
-        }
+        const int cq = PP || P->nc == 1 ? 0 : A.comp[q];
+        const double md = min_dij_sq_rn<PP>(*P, PP ? 0 : own_f >> 8, a.w, cq, xq.w);
+        hit = __dsub_rn(md, sumsq3_rn(Rij)) > 0.0;
       }
+      const unsigned b = __ballot_sync(FULL, hit);
+      if (lane == 0) {
+        W.mask[f0 >> 5] = b;
+        W.pre[f0 >> 5] = run;
+      }
+      run += __popc(b);
     }
     if (lane == 0) {
       W.mask[(Tw + 31) >> 5] = 0u;
