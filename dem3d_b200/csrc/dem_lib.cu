@@ -1822,6 +1822,7 @@ int launch_chunk(dem_ctx* c, int phase, int first = 0, int steps = 0) {
       cr.walls = c->wall_dev;
       cr.table = c->dp;
       cr.nw = (int)c->wm.size();
+      c->walls_moved = true;
     }
   } else if (!c->bar) {
     CK(cudaMalloc(&c->bar, 2 * sizeof(unsigned)));
