@@ -136,12 +136,12 @@ def pair_bytes_per_particle(mixed, update, z_pp):
     """Algorithmic DRAM bytes of one pair-kernel launch per particle (0.5*z_pp
     contacts): per contact its list entry 8 and i's place 4 read, the pair's
     history record (key 4 + 36 B FP32 / 48 B FP64) read, the "i" half
-    (48 / 80 B) and the "j" half (48 / 80 B + its count 4) written, and in
+    (36 / 72 B) and the "j" half (48 / 80 B + its count 4) written, and in
     the history-updating pass the new record written.  The two particles'
     positions and velocities are their own data (L1/L2)."""
     rec = 4 + (36 if mixed else 48)
-    half = 48 if mixed else 80
-    per = 8 + 4 + rec + half + half + 4 + (rec if update else 0)
+    ihalf, jhalf = (36, 48) if mixed else (72, 80)
+    per = 8 + 4 + rec + ihalf + jhalf + 4 + (rec if update else 0)
     return 0.5 * z_pp * per
 
 
@@ -150,8 +150,8 @@ def fold_bytes_per_particle(mixed, epi, z_pp, z_pw=0.0, nw=0, nprev=3):
       reads: cell 4, rank 4, "j" count 4 (reset), matched bits 4, place in
         the contact list 8, position + R 32 (and the FP64 velocity copies 48
         in FP64 mode, the FP32 ones 24 with walls), the "i" halves and the
-        "j" halves of its contacts (0.5*z_pp each, 48 / 80 B), wall flags and
-        records;
+        "j" halves of its contacts (0.5*z_pp each, 36 / 72 and 48 / 80 B),
+        wall flags and records;
       epi "predict" (pass 1, src/MDEM.f90:296-331, history-updating): the
         record count 4 read and written, new wall records; ring nprev*72
         read, Particle v,w 48 read (mixed), ring slot 72 + the corrector's
@@ -163,10 +163,10 @@ def fold_bytes_per_particle(mixed, epi, z_pp, z_pw=0.0, nw=0, nprev=3):
         (mixed) read, Particle x,v,w 72 read and written, Predicted a,alpha
         48 + next-pass copies + cell 4 written."""
     vel = 24 if mixed else 48
-    half = 48 if mixed else 80
+    halves = 36 + 48 if mixed else 72 + 80
     wrec = 4 + (36 if mixed else 48)
     base = (4 + 4 + 4 + 4 + 8 + 32 + (0 if mixed else 48) + (24 if mixed and nw else 0)
-            + z_pp * half + nw * 4 + z_pw * (wrec - 4))
+            + 0.5 * z_pp * halves + nw * 4 + z_pw * (wrec - 4))
     sums = 72 if nprev else 0
     if epi == "predict":
         base += 8 + nw * 4 + z_pw * (wrec - 4)

@@ -11,15 +11,15 @@
 //     stayed, in their previous order).
 // K2  candidate rows: for every particle, the partners within MinDij + skin
 //     in the order the reference's sweep meets them (src/MForces.f90:173-272),
-//     rebuilt by one warp per particle around relinked cells, and for every
-//     particle when the accumulated displacement bound reaches 0.4 skin.
-// K2+K4 pass kernel: one thread per particle (original index order) applies
-//     the reference's overlap test to its candidates, evaluates every contact
-//     in the reference's orientation ("i" = the particle visited first) and
-//     adds the contributions in the order of the sweep, so that the forces
-//     are bit-identical to ComputeAccelerations (src/MForces.f90:145-335).
-//     The AB predictor / AM corrector (src/MDEM.f90:296-365) run in its
-//     epilogue, which also hashes the next position into its cell.
+//     rebuilt by a warp per row near the spheres that changed cell, and for
+//     every particle when the accumulated displacement bound reaches 0.4 skin.
+// K4  force pass, a test, a pair and a fold kernel: the reference's overlap
+//     test on the candidates, every contact once in the reference's
+//     orientation ("i" = the particle visited first), the contributions added
+//     in the order of the sweep, so that the forces are bit-identical to
+//     ComputeAccelerations (src/MForces.f90:145-335).  The AB predictor / AM
+//     corrector (src/MDEM.f90:296-365) run in the fold's epilogue, which also
+//     hashes the next position into its cell.
 // K3  history: records owned by imin are double-buffered; a pass that updates
 //     them writes a fresh table (new/updated contacts + records of pairs that
 //     the sweep did not visit, as the reference keeps those untouched).
@@ -666,13 +666,14 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(LIST_THREADS)
 }
 
 // ---------------------------------------------------------------------------
-// K2+K4: after the relink and the candidate rows, a force pass is three
+// K4: after the relink and the candidate rows, a force pass is three
 // kernels.
 //
-// k_test (both precisions): one thread per particle as "i" of its row
-//   applies the reference's overlap test DeltaDijSq = MinDijSq - DijSq > 0
-//   (src/MForces.f90:218-224, exact FP64) to its candidates and writes its
-//   contacts to the pass's contact list, together and in row order.
+// k_test (both precisions): a warp lays the rows of its 32 particles end to
+//   end, applies the reference's overlap test DeltaDijSq = MinDijSq - DijSq > 0
+//   (src/MForces.f90:218-224, exact FP64) with a lane per candidate, and
+//   writes each particle's contacts to the pass's contact list, together and
+//   in row order.
 // k_pair_fp64 / k_pair_mixed: one thread per contact of the list evaluates
 //   it once (src/MForces.f90:199-252, CommonCalculations :339-387) with the
 //   pair's history record (looked up in i's table, then j's), writes the "i"

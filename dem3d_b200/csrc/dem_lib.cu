@@ -1095,8 +1095,8 @@ int prepare_side(dem_ctx* c, int side) {
   return DEM_OK;
 }
 
-// relink towards the prepared assignment (the candidate rows around the
-// relinked cells are rebuilt by the test kernel)
+// relink towards the prepared assignment and rebuild the candidate rows near
+// the particles that changed cell
 void pass_lists(dem_ctx* c, int side, bool update, int tag, bool early) {
   early = early && c->early_launch && !c->slab;
   const int b = c->par ^ 1;
