@@ -849,7 +849,7 @@ __global__ void __launch_bounds__(128, MINB) k_pair_fp64(PassArgs<double4, doubl
 // The fold kernel (FP64): p's block of the sweep, its Force and Torque in
 // sweep order, a = F/m, alpha = T/I, then the integrator epilogue.  WALLS:
 // some system has walls.
-template <bool PP, int EPI, bool WALLS, bool WAIT = false>
+template <bool PP, int EPI, bool WALLS>
 __device__ __forceinline__ void fold_fp64_body(const PassArgs<double4, double2>& A, int vblock,
                                                double* stage) {
   __shared__ double s_w[WALLS ? NWM : 1][128];  // |FN| of each wall contact
@@ -866,10 +866,6 @@ __device__ __forceinline__ void fold_fp64_body(const PassArgs<double4, double2>&
   const double4 p4 = ld32(A.X + p);
   const double4 pv4 = ld32(A.v4 + p);
   const double2 pw2 = A.w2[p];
-  // (none of these are written by the pair kernel, and when this kernel is
-  // scheduled the kernels before that one have completed: see
-  // pass_kernel_entry)
-  if (WAIT) pass_kernel_entry();
   const int ni = A.in_cnt[p];
   const unsigned matched = A.matched[p];
   // one decision for the warp (with walls, for the block: it meets block
@@ -1081,12 +1077,12 @@ __device__ __forceinline__ void fold_fp64_body(const PassArgs<double4, double2>&
 // read in 32-byte pieces.)
 template <bool PP, int EPI, bool WALLS, bool STRIDE>
 __global__ void __launch_bounds__(128, WALLS ? 4 : 5) k_fold_fp64(PassArgs<double4, double2> A) {
+  pass_kernel_entry();
   __shared__ __align__(16) double stage[EpiStage<EPI, false>::SIZE];
   if (!STRIDE) {
-    fold_fp64_body<PP, EPI, WALLS, true>(A, blockIdx.x, stage);
+    fold_fp64_body<PP, EPI, WALLS>(A, blockIdx.x, stage);
     return;
   }
-  pass_kernel_entry();
   const int nvb = (A.n + 127) / 128;
   for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
     fold_fp64_body<PP, EPI, WALLS>(A, vb, stage);

@@ -411,7 +411,7 @@ __global__ void __launch_bounds__(128, MINB) k_pair_mixed(PassArgs<float4, float
 // (FP32), a = F/m, alpha = T/I, then the FP64 integrator epilogue.  WALLS:
 // some system has walls; CONE: some wall is a cone.  (Body for block
 // `vblock` of particles.)
-template <bool PP, int EPI, bool WALLS, bool CONE, bool WAIT = false>
+template <bool PP, int EPI, bool WALLS, bool CONE>
 __device__ __forceinline__ void fold_mixed_body(const PassArgs<float4, float2>& A,
                                                 const MixedView& V, int vblock, double* stage) {
   __shared__ float s_w[WALLS ? NWM : 1][128];  // |FN| of each wall contact
@@ -426,10 +426,6 @@ __device__ __forceinline__ void fold_mixed_body(const PassArgs<float4, float2>& 
   const int nc = A.ccount[p];
   const int st0 = A.cstart[p];
   const double4 p4 = ld32(A.X + p);
-  // (none of these are written by the pair kernel, and when this kernel is
-  // scheduled the kernels before that one have completed: see
-  // pass_kernel_entry)
-  if (WAIT) pass_kernel_entry();
   const int ni = A.in_cnt[p];
   const unsigned matched = A.matched[p];
   // one decision for the warp (with walls, for the block: it meets block
@@ -634,12 +630,12 @@ __device__ __forceinline__ void fold_mixed_body(const PassArgs<float4, float2>& 
 template <bool PP, int EPI, bool WALLS, bool CONE, bool STRIDE>
 __global__ void __launch_bounds__(128, EPI == EPI_CORRECT && !WALLS ? 7 : 5)
     k_fold_mixed(PassArgs<float4, float2> A, MixedView V) {
+  pass_kernel_entry();
   __shared__ __align__(16) double stage[EpiStage<EPI, true>::SIZE];
   if (!STRIDE) {
-    fold_mixed_body<PP, EPI, WALLS, CONE, true>(A, V, blockIdx.x, stage);
+    fold_mixed_body<PP, EPI, WALLS, CONE>(A, V, blockIdx.x, stage);
     return;
   }
-  pass_kernel_entry();
   const int nvb = (A.n + 127) / 128;
   for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
     fold_mixed_body<PP, EPI, WALLS, CONE>(A, V, vb, stage);

@@ -485,17 +485,17 @@ __device__ __forceinline__ void epilogue(const PassArgs<V4, W2>& A, const DevPar
   }
 }
 
-// Start of every kernel of a force pass (relink, rows, test, pair, fold).  A
-// kernel launched with programmatic stream serialization may be
-// scheduled while the kernel before it in the stream is still running; it
+// First statement of every kernel of a force pass (relink, rows, lists, test,
+// pair, fold).  A kernel launched with programmatic stream serialization may
+// be scheduled while the kernel before it in the stream is still running; it
 // waits here until that kernel has completed and its writes are visible, and
 // then allows the next kernel of the pass to be scheduled (whose blocks take
 // the SM slots this kernel's last blocks free, and wait in turn).  Without
-// that launch attribute both instructions return at once.  Before the wait a
-// kernel touches nothing that the kernel ahead of it writes.  What the kernels
-// further ahead wrote may be read: a kernel allows its successor only after
-// its own wait, so when a fold is scheduled the pair kernel's blocks have all
-// passed theirs, and the test kernel and all before it have completed.
+// that launch attribute both instructions return at once.  Nothing is read
+// before the wait, not even what kernels further ahead wrote: those have
+// completed by then (a kernel allows its successor only after its own wait),
+// but their writes are promised to be visible only to threads that have
+// waited, and a block may start on an SM whose L1 holds older values.
 __device__ __forceinline__ void pass_kernel_entry() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
