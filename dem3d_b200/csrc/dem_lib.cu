@@ -1199,7 +1199,8 @@ int grow_rows(dem_ctx* c, int need) {
   CK(cudaStreamSynchronize(c->stream));
   cudaFree(c->rows.cand);
   c->rows.cand = nullptr;
-  CK(cudaMalloc(&c->rows.cand, sizeof(int) * (size_t)std::max(c->n, 1) * kc));
+  // (room for every particle that can still be poured, as at dem_set_state)
+  CK(cudaMalloc(&c->rows.cand, sizeof(int) * (size_t)std::max(c->ncap, 1) * kc));
   c->kc = kc;
   c->rows.kc = kc;
   drop_graphs(c);
