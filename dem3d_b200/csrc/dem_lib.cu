@@ -1755,6 +1755,14 @@ bool chunk_cluster(const dem_ctx* c) {
          c->n <= CLUSTER_MAX;
 }
 
+// Steps after which a cluster launch's program repeats: the ring's slots are
+// back in their places (it holds nprev past steps and a spare slot) and so are
+// the two history tables.  2, 2, 6 and 4 steps at method orders 1 to 4.
+int cluster_period(const dem_ctx* c) {
+  const int slots = c->nprev + 1;
+  return slots % 2 ? 2 * slots : slots;
+}
+
 // Record `steps` MoveParticles steps as the passes of one persistent chunk
 // into prog[phase] (the host bookkeeping is left as it was, as by
 // capture_steps).  Recording launches nothing.
@@ -1815,6 +1823,7 @@ int launch_chunk(dem_ctx* c, int phase, int first = 0, int steps = 0) {
   ClusterRun cr{};
   if (steps > 0) {
     cr.stop = c->stop_on_escape ? 1 : 0;
+    cr.period = c->prog_n[phase];
     if (!c->wm.empty()) {
       fill_wall_slots(c, first, steps);  // the previous launch has completed
       if (!c->wall_dev) CK(cudaMalloc(&c->wall_dev, sizeof(dem_wall) * NWM * WALL_SLOTS));
@@ -2204,7 +2213,7 @@ int run_chunk(dem_ctx* c, int step, int G, int mode, int* done_out, bool* stoppe
   int phase = (c->nprev > 0 ? c->ringmap[c->nprev] : 0) * 4 + c->hcur * 2 + c->par;
   if (mode != CHUNK_GRAPH) {
     if (!c->prog[phase]) {
-      st = record_chunk(c, 4, phase);
+      st = record_chunk(c, mode == CHUNK_CLUSTER ? cluster_period(c) : G, phase);
       if (st) return st;
     }
     st = mode == CHUNK_CLUSTER ? launch_chunk(c, phase, step, G) : launch_chunk(c, phase);
@@ -3260,9 +3269,11 @@ int dem_move_particles_euler(dem_ctx* c) {
   return read_counters(c);
 }
 
-// The main loop.  Steps are replayed from CUDA graphs of G = 4 steps (the
-// period of the ring rotation (<= 4 slots) and of the history double buffer);
-// every kernel in a graph first checks the abort word.  Before each replay
+// The main loop.  Steps are replayed from CUDA graphs of G = 4 steps, one graph
+// per rotation phase (ring spare slot, history parity, list parity) that a
+// chunk can start from: at method order 3 the ring's three slots come back
+// after three steps, so that the chunks' phases go round.  Every kernel in a
+// graph first checks the abort word.  Before each replay
 // the history tables are grown if the last updating pass came within
 // HEADROOM records of the capacity.  If a pass inside a replay still
 // overflows, it records its step index and every later kernel of the replay

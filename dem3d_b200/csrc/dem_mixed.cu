@@ -662,7 +662,7 @@ __device__ __forceinline__ void fold_blocks_mixed(const ChunkPassMx& sp, double*
 }
 // CLUSTER: the launch is one cluster instead (ClusterRun), for systems so
 // small that a pass is a chain of latencies: no launch boundaries, a hardware
-// barrier between the phases, npass passes of a program of 8 that repeats, and
+// barrier between the phases, npass passes of a program that repeats, and
 // the whole register file of an SM for each block.
 template <bool PP, bool WALLS, bool CONE, bool CLUSTER>
 __global__ void __launch_bounds__(128, CLUSTER ? 1 : 3)
@@ -683,7 +683,7 @@ __global__ void __launch_bounds__(128, CLUSTER ? 1 : 3)
     return true;
   };
   for (int k = 0; k < npass; k++) {
-    load_pass(sp, prog + (CLUSTER ? k & 7 : k));
+    load_pass(sp, prog + (CLUSTER ? k % cr.period : k));
     if (CLUSTER) cluster_pass(sp, cr, k);
     chunk_relink(sp, gwarp, nwarps, sh[threadIdx.x >> 5]);
     if (!sync()) return;

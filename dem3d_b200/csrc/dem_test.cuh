@@ -997,11 +997,14 @@ struct GridSync {
 
 // A launch of one cluster (small systems): the hardware cluster barrier, the
 // walls of each step of the launch (copied into the system's table after the
-// step's predictor; NULL: walls at rest) and whether escapes stop the launch.
+// step's predictor; NULL: walls at rest), whether escapes stop the launch, and
+// the passes of its program, which it repeats (whole periods of the ring's
+// rotation and of the history's double buffer).
 struct ClusterRun {
   const dem_wall* walls;
   DevParams* table;
   int nw, stop;
+  int period;
 };
 // release / acquire at cluster scope: what every thread of the cluster wrote
 // before is visible to every thread after
@@ -1127,7 +1130,7 @@ __device__ __noinline__ void chunk_test(const CP& p, TestWarp* warps) {
 }
 
 // The start of pass k of a cluster launch: its own tag (the pass number in the
-// launch; the program repeats every 8 passes), the escape stop before a
+// launch; the program repeats), the escape stop before a
 // step's first pass, and the walls of the step before its second one.
 template <class CP>
 __device__ __forceinline__ void cluster_pass(CP& p, const ClusterRun& c, int k) {
