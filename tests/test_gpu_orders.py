@@ -30,6 +30,15 @@ def _bed(make, n, order, precision, moving):
     return s
 
 
+def _hopper(make, precision):
+    w = configs.hopper(n=600, seed=1005)
+    w.params.precision = precision
+    s = make(w.params)
+    s.set_state(w.pos, w.vel, w.omega, comp=w.comp, radius=w.radius)
+    s.initialize_cell_distribution()
+    return s
+
+
 def _same(a, b):
     assert a.n == b.n
     x, y = a.get_state(), b.get_state()
@@ -92,3 +101,14 @@ def test_graphs_and_persistent_chunks(mode, order, precision):
     _follow(a, others, 8)
     assert mode == 0 or a.persistent_blocks() > 0
     assert a.ncol() > 0
+
+
+def test_cluster_and_separate_kernels_agree_on_a_cone_in_mixed_precision():
+    a, b = _hopper(DEMSystem, P.PREC_MIXED), _hopper(DEMSystem, P.PREC_MIXED)
+    b.set_profiling(True)
+    for s in (a, b):
+        s.run(1, 700)
+    steps = _launches(a, 701, 800), _launches(b, 701, 800)
+    assert steps[0] <= 100 and steps[1] >= 800
+    _same(a, b)
+    assert np.count_nonzero(a.get_contacts()["iw"] == 0) > 0  # the cone is touched
