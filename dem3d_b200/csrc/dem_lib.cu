@@ -1629,6 +1629,16 @@ int apply_walls(dem_ctx* c, int k) {
   return DEM_OK;
 }
 
+// The device walls as they stood before a chunk's copies ran: those at c->time,
+// or, if they had not moved yet, those of the parameter table.
+int restore_walls(dem_ctx* c, bool moved) {
+  if (moved) return apply_walls(c, 0);
+  CK(cudaMemcpyAsync(reinterpret_cast<char*>(c->dp) + offsetof(DevParams, walls),
+                     c->hsys[0].walls, sizeof(dem_wall) * c->wm.size(), cudaMemcpyHostToDevice,
+                     c->stream));
+  return DEM_OK;
+}
+
 // the host copy of system 0's walls follows the device one (before any
 // upload of the parameter table, and for dem_get_walls)
 void sync_host_walls(dem_ctx* c) {
@@ -2188,6 +2198,8 @@ constexpr int CHUNK_CLUSTER = 2;     // up to CLUSTER_STEPS steps as one cluster
 int run_chunk(dem_ctx* c, int step, int G, int mode, int* done_out, bool* stopped, bool* fresh) {
   const int HEADROOM = 2;
   const double dt = c->params.time_step;
+  const double time0 = c->time;
+  const bool moved0 = c->walls_moved;
   *stopped = false;
   int st = *fresh ? DEM_OK : read_counters(c);
   if (st) return st;
@@ -2267,11 +2279,19 @@ int run_chunk(dem_ctx* c, int step, int G, int mode, int* done_out, bool* stoppe
     c->last_side = 1;
   }
   step += done;
-  c->time = (double)(step - 1) * dt;
+  // (a chunk that stopped in its first step: the time before it, which need
+  // not be (step - 1)*dt, as after the Euler start-up)
+  c->time = done > 0 ? (double)(step - 1) * dt : time0;
+  if ((escape_stop || failed_pass >= 0) && !c->wm.empty()) {
+    // a graph's later wall copies ran: back to the walls before the step (a
+    // cluster launch copies no walls past a stopped pass)
+    c->walls_moved = done > 0 || moved0;
+    if (mode != CHUNK_CLUSTER) {
+      st = restore_walls(c, c->walls_moved);
+      if (st) return st;
+    }
+  }
   if (escape_stop) {
-    // the replay's later wall copies ran: back to the walls of step-1
-    st = apply_walls(c, 0);
-    if (st) return st;
     CK(cudaMemsetAsync(&c->cnt->abort, 0, 2 * sizeof(int), c->stream));  // abort, abort_tag
     CK(cudaMemsetAsync(&c->cnt->escape_stop, 0, sizeof(int), c->stream));
     *done_out = done;
@@ -2279,9 +2299,6 @@ int run_chunk(dem_ctx* c, int step, int G, int mode, int* done_out, bool* stoppe
     return DEM_OK;
   }
   if (failed_pass >= 0) {
-    // the replay's later wall uploads ran: back to the walls of step-1
-    st = apply_walls(c, 0);
-    if (st) return st;
     // the failed step: its first pass ran up to the failure (relink done),
     // or its first pass completed and its second one failed
     c->par ^= 1;

@@ -1131,7 +1131,9 @@ __device__ __noinline__ void chunk_test(const CP& p, TestWarp* warps) {
 
 // The start of pass k of a cluster launch: its own tag (the pass number in the
 // launch; the program repeats), the escape stop before a
-// step's first pass, and the walls of the step before its second one.
+// step's first pass, and the walls of the step before its second one (not
+// past a stopped pass, which the host repeats with the walls as they stand;
+// what stops the launch has done so before this pass, but for errors).
 template <class CP>
 __device__ __forceinline__ void cluster_pass(CP& p, const ClusterRun& c, int k) {
   if (threadIdx.x == 0) {
@@ -1139,7 +1141,7 @@ __device__ __forceinline__ void cluster_pass(CP& p, const ClusterRun& c, int k) 
     p.a.tag = k;
     p.rl.stop_tag = c.stop && (k & 1) == 0 ? k : -1;
   }
-  if (c.walls && (k & 1) && blockIdx.x == 0) {
+  if (c.walls && (k & 1) && blockIdx.x == 0 && *(volatile const int*)&p.rl.cnt->abort == 0) {
     const int words = c.nw * (int)(sizeof(dem_wall) / sizeof(double));
     const double* src = (const double*)(c.walls + (size_t)(k >> 1) * NWM);
     double* dst = (double*)c.table->walls;  // (one system)
