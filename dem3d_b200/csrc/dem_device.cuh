@@ -177,18 +177,23 @@ struct CellLists {
   int2* mlist;
   int* rstamp;
   int mcap;
-  // each cell's list copied in order into SLOT_CAP slots ([cell*SLOT_CAP +
-  // k]) and its length (slot_n > SLOT_CAP: only the first SLOT_CAP are
-  // copied; -1: not current): the candidate rows read a neighbour cell with
+  // each cell's list copied in order into scap slots ([cell*scap + k]) and its
+  // length (slot_n > scap: only the first scap are copied; -1: not current): the candidate rows read a neighbour cell with
   // independent loads instead of walking its links one after the other
   int* slot;
   int* slot_n;
+  int scap;
   // the reference's index of the particle stored at each place, when the
   // storage is kept in cell order (the relink orders arrivals by it); NULL:
   // stored in the reference's order
   const int* gid;
 };
-constexpr int SLOT_CAP = 64;
+// scap is SLOT_MAX, or half of it where the slots of a wide grid would take
+// more than an eighth of the free memory.  (A bed of 1M spheres of two sizes,
+// up to 40 in a cell: 728 us per step with 64 slots, 834 with 32, whose relink
+// and rows walk the longer lists; one size, at most 8 in a cell: no
+// difference.)
+constexpr int SLOT_MAX = 64;
 // movers one relink records for the row kernel (more: every stamped row is
 // rebuilt)
 constexpr int MLIST_CAP = 4096;

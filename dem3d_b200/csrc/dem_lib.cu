@@ -2100,7 +2100,7 @@ int permute_particles(dem_ctx* c, const int* pi) {
   remap(c->L.mnext, n);
   remap(c->L.head, nc);
   remap(c->L.arr_head, nc);
-  remap(c->L.slot, nc * SLOT_CAP);
+  remap(c->L.slot, nc * c->L.scap);
   for (int b = 0; b < 2; b++) remap(c->H[b].key, (long long)c->H[b].cap * c->H[b].n);
   remap(c->rows.cand, (long long)c->rows.kc * n);
   CK(cudaStreamSynchronize(c->stream));
@@ -2747,7 +2747,12 @@ int dem_set_state(dem_ctx* c, int32_t n, const int32_t* comp, const double* radi
     CK(cudaMalloc(&L.rflag, sizeof(int) * NC));
     CK(cudaMalloc(&L.dlist[0], sizeof(int) * NC));
     CK(cudaMalloc(&L.dlist[1], sizeof(int) * NC));
-    CK(cudaMalloc(&L.slot, sizeof(int) * NC * SLOT_CAP));
+    // (lists of up to SLOT_MAX entries in slots, unless those of a wide, mostly
+    // empty grid would take much of the memory)
+    size_t room = 0, all = 0;
+    CK(cudaMemGetInfo(&room, &all));
+    L.scap = sizeof(int) * NC * SLOT_MAX <= room / 8 ? SLOT_MAX : SLOT_MAX / 2;
+    CK(cudaMalloc(&L.slot, sizeof(int) * NC * (size_t)L.scap));
     CK(cudaMalloc(&L.slot_n, sizeof(int) * NC));
     CK(cudaMemsetAsync(L.slot_n, 0xFF, sizeof(int) * NC, c->stream));
     L.mcap = MLIST_CAP;

@@ -42,7 +42,7 @@ __device__ __forceinline__ double min_dij_sq_rn(const DevParams& P, int ca, doub
   return P.min_dij_sq[ca * NCM + cb];
 }
 
-// Copy cell c's list into its slots (the first SLOT_CAP entries) and record
+// Copy cell c's list into its slots (the first scap entries) and record
 // its length; a walk longer than n (corrupt links) records -1.
 __device__ __forceinline__ void copy_slots(const CellLists& L, int c, int first, int n) {
   int k = 0;
@@ -51,7 +51,7 @@ __device__ __forceinline__ void copy_slots(const CellLists& L, int c, int first,
       k = -1;
       break;
     }
-    if (k < SLOT_CAP) L.slot[(size_t)c * SLOT_CAP + k] = q;
+    if (k < L.scap) L.slot[(size_t)c * L.scap + k] = q;
     k++;
   }
   L.slot_n[c] = k;
@@ -140,7 +140,7 @@ __device__ __forceinline__ bool relink_links(const CellLists& L, const int* cell
 // this pass rebuilds every candidate row.
 // (The body of k_relink; warp / nwarps: this warp's index among the warps
 // that share the work, `sh` RELINK_ROOM ints of shared memory of its own.)
-constexpr int RELINK_ROOM = SLOT_CAP + 32;
+constexpr int RELINK_ROOM = SLOT_MAX + 32;
 __device__ __forceinline__ void relink_body(const DevParams* __restrict__ PT,
                                             const int* __restrict__ cellsys, const CellLists& L,
                                             int par, int n, int update, int stop_tag,
@@ -202,9 +202,9 @@ __device__ __forceinline__ void relink_body(const DevParams* __restrict__ PT,
     const int c = L.dlist[par][i];
     const int len = L.slot_n[c];
     const int ah = L.arr_head[c];
-    const int* sl = L.slot + (size_t)c * SLOT_CAP;
-    const int e0 = lane < len && len <= SLOT_CAP ? sl[lane] : -1;
-    const int e1 = lane + 32 < len && len <= SLOT_CAP ? sl[lane + 32] : -1;
+    const int* sl = L.slot + (size_t)c * L.scap;
+    const int e0 = lane < len && len <= L.scap ? sl[lane] : -1;
+    const int e1 = lane + 32 < len && len <= L.scap ? sl[lane + 32] : -1;
     const DevParams& P = sys_params(PT, cellsys, c);
     if (!in_slab(P, c)) {
       // a cell another slab advances (a particle of this slab left for it):
@@ -227,7 +227,7 @@ __device__ __forceinline__ void relink_body(const DevParams* __restrict__ PT,
       if (lane == na) arr = a;
       na++;
     }
-    if (len >= 0 && len <= SLOT_CAP && na <= 32) {
+    if (len >= 0 && len <= L.scap && na <= 32) {
       const bool s0 = e0 >= 0 && cell_new[e0] == c;
       const bool s1 = e1 >= 0 && cell_new[e1] == c;
       const unsigned b0 = __ballot_sync(FULL, s0), b1 = __ballot_sync(FULL, s1);
@@ -251,7 +251,7 @@ __device__ __forceinline__ void relink_body(const DevParams* __restrict__ PT,
       for (int k = lane; k < len2; k += 32) {
         const int x = sh[k];
         L.next[x] = k + 1 < len2 ? sh[k + 1] : -1;
-        if (k < SLOT_CAP) L.slot[(size_t)c * SLOT_CAP + k] = x;
+        if (k < L.scap) L.slot[(size_t)c * L.scap + k] = x;
       }
       if (lane == 0) {
         L.head[c] = len2 > 0 ? sh[0] : -1;
@@ -500,10 +500,10 @@ __device__ __noinline__ void build_row(const DevParams& P, int n, int p, int c,
            P.nx * (axis_wrap(jy, P.ny, P.pbc[1]) + P.ny * axis_wrap(jz, P.nz, P.pbc[2]));
   }
   if (cw >= 0) len = L.slot_n[cw];
-  const int* own = L.slot + (size_t)c * SLOT_CAP;
+  const int* own = L.slot + (size_t)c * L.scap;
   // (p's place in its list; entries past the list's end are old ones)
-  const int w0 = own[lane], w1 = own[lane + 32];
-  if (__any_sync(FULL, len < 0 || len > SLOT_CAP)) {
+  const int w0 = own[lane], w1 = lane + 32 < L.scap ? own[lane + 32] : -1;
+  if (__any_sync(FULL, len < 0 || len > L.scap)) {
     build_row_links<PP>(P, n, p, c, X, comp, L, R, cnt, tag);
     return;
   }
@@ -541,7 +541,7 @@ __device__ __noinline__ void build_row(const DevParams& P, int n, int p, int c,
     }
     const int cj = __shfl_sync(FULL, cw, j), sj = __shfl_sync(FULL, skip, j),
               ej = __shfl_sync(FULL, excl, j);
-    return (size_t)cj * SLOT_CAP + (sj + f - ej);
+    return (size_t)cj * L.scap + (sj + f - ej);
   };
   int m = 0;
   for (int f = 0; f < T; f += 64) {
@@ -598,10 +598,10 @@ __device__ __forceinline__ bool build_row_thread(const DevParams& P, int n, int 
       cw = P.coff + axis_wrap(jx, P.nx, P.pbc[0]) +
            P.nx * (axis_wrap(jy, P.ny, P.pbc[1]) + P.ny * axis_wrap(jz, P.nz, P.pbc[2]));
     }
-    const int4* sl = (const int4*)(L.slot + (size_t)cw * SLOT_CAP);
+    const int4* sl = (const int4*)(L.slot + (size_t)cw * L.scap);
     int4 s = sl[0];  // (the first entries with the length)
     const int len = L.slot_n[cw];
-    if (len < 0 || len > SLOT_CAP) return false;
+    if (len < 0 || len > L.scap) return false;
     for (int k0 = 0; k0 < len; k0 += 4) {
       if (k0 > 0) s = sl[k0 >> 2];
       const int q[4] = {s.x, s.y, s.z, s.w};
@@ -732,8 +732,8 @@ __device__ __forceinline__ void rows_body(const TestArgs& A, int warp, int nwarp
     const int len = L.slot_n[b];
     const double4 q4 = ld32(A.X + r.x);
     const int cq = PP ? 0 : A.comp[r.x];
-    const int* sl = L.slot + (size_t)b * SLOT_CAP;
-    const bool slots = len >= 0 && len <= SLOT_CAP;
+    const int* sl = L.slot + (size_t)b * L.scap;
+    const bool slots = len >= 0 && len <= L.scap;
     int at = L.head[b];  // (a list that does not fit the slots: its next 32)
     for (int k0 = 0; slots ? k0 < len : (at != -1 && k0 < n); k0 += 32) {
       int x = -1;
