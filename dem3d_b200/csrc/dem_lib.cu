@@ -175,6 +175,7 @@ struct dem_ctx {
   bool slab = false;
   int* gstamp = nullptr;
   int gepoch = 0;
+  int slab_cap = 0;  // particles that gstamp, slab_list and slab_ghosts are laid out for
   int slab_z0 = 0, slab_z1 = 0;
   int* slab_list = nullptr;   // particles of a layer / migrants (scratch, [ncap])
   int* slab_ghosts = nullptr; // the ghosts received this pass
@@ -1978,6 +1979,26 @@ int slab_layer(const dem_ctx* c, int z) {
 // whether the slab has a layer above / below it (periodic z: always)
 bool slab_has_up(const dem_ctx* c) { return c->hsys[0].pbc[2] || c->slab_z1 < slab_nz(c); }
 bool slab_has_down(const dem_ctx* c) { return c->hsys[0].pbc[2] || c->slab_z0 > 0; }
+
+// the slab's arrays for the current capacity (a later dem_set_state may bring
+// more particles than the one before dem_slab_set_range)
+int ensure_slab_arrays(dem_ctx* c) {
+  const int N = std::max(c->ncap, 1);
+  if (c->slab_cap >= N) return DEM_OK;
+  CK(cudaStreamSynchronize(c->stream));
+  cudaFree(c->gstamp);
+  cudaFree(c->slab_list);
+  cudaFree(c->slab_ghosts);
+  c->gstamp = c->slab_list = c->slab_ghosts = nullptr;
+  c->slab_cap = 0;
+  CK(cudaMalloc(&c->gstamp, sizeof(int) * (size_t)N));
+  CK(cudaMemset(c->gstamp, 0xFF, sizeof(int) * (size_t)N));
+  CK(cudaMalloc(&c->slab_list, sizeof(int) * (size_t)std::max(N, slab_nxy(c))));
+  CK(cudaMalloc(&c->slab_ghosts, sizeof(int) * (size_t)N));
+  if (!c->slab_count) CK(cudaMalloc(&c->slab_count, sizeof(int) * 4));
+  c->slab_cap = N;
+  return DEM_OK;
+}
 
 // the particles of layer z into c->slab_list; returns their count
 int slab_list_layer(dem_ctx* c, int z, int* count) {
@@ -3961,13 +3982,9 @@ int dem_slab_set_range(dem_ctx* c, int32_t z0, int32_t z1) {
   c->slab_z0 = z0;
   c->slab_z1 = z1;
   c->removal = false;  // particles leave a slab for its neighbour, not the system
-  if (!c->gstamp) {
-    CK(cudaMalloc(&c->gstamp, sizeof(int) * (size_t)std::max(c->ncap, 1)));
-    CK(cudaMalloc(&c->slab_list, sizeof(int) * (size_t)std::max(c->ncap, slab_nxy(c))));
-    CK(cudaMalloc(&c->slab_ghosts, sizeof(int) * (size_t)std::max(c->ncap, 1)));
-    CK(cudaMalloc(&c->slab_count, sizeof(int) * 4));
-  }
-  CK(cudaMemset(c->gstamp, 0xFF, sizeof(int) * (size_t)std::max(c->ncap, 1)));
+  st = ensure_slab_arrays(c);
+  if (st) return st;
+  CK(cudaMemset(c->gstamp, 0xFF, sizeof(int) * (size_t)c->slab_cap));
   c->n_ghosts = 0;
   drop_graphs(c);
   // room for the "j" results a slab receives as well as its own: the
@@ -3989,6 +4006,7 @@ int dem_slab_phase(dem_ctx* c, int32_t step, int32_t pass, int32_t phase) {
   switch (phase) {
     case DEM_SLAB_RELINK:
       st = ensure_drag(c);
+      if (!st) st = ensure_slab_arrays(c);
       if (st) return st;
       c->slab_rm = current_map(c);
       if (c->prepared != side) {
