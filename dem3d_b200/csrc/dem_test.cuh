@@ -149,12 +149,13 @@ __device__ __forceinline__ void relink_body(const DevParams* __restrict__ PT,
   const int lane = threadIdx.x & 31;
   const bool first_thread = warp == 0 && lane == 0;
   // (the status words, the dirty-cell count and the pass number requested
-  // together)
-  const int abort0 = cnt->abort;
+  // together; the abort word may be set meanwhile, so one lane's reading
+  // decides for the warp, whose lanes meet in the loops below)
+  const int abort1 = lane == 0 ? cnt->abort : 0;
   const unsigned long long escaped = cnt->escaped;
   const int m = cnt->n_dirty[par];
   const int stamp = cnt->pass_id + 1;  // fold kernels advance pass_id, not this one
-  if (abort0) return;
+  if (__shfl_sync(FULL, abort1, 0)) return;
   // inside a captured chunk, particles that left the box in the last step
   // stop the chunk before this step (the host runs UpdateParticleList); the
   // count is final here (written by the previous kernel), so every block
@@ -694,11 +695,11 @@ __device__ __forceinline__ void rows_body(const TestArgs& A, int warp, int nwarp
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   Counters* const cnt = A.cnt;
-  const int abort0 = cnt->abort;
+  const int abort1 = lane == 0 ? cnt->abort : 0;  // (one reading for the warp)
   const bool full = cnt->full_due != 0;
   const int stamp = cnt->pass_id + 1;
   const int nm = cnt->n_mlist[stamp & 1];
-  if (abort0) return;
+  if (__shfl_sync(FULL, abort1, 0)) return;
   const int n = A.n;
   const CellLists& L = A.L;
   auto build = [&](int p, int c) {
