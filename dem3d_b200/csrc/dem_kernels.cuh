@@ -1111,13 +1111,16 @@ __device__ __forceinline__ void fold_blocks_fp64(const ChunkPass64& sp, double* 
     __syncthreads();
   }
 }
-// CLUSTER: the launch is one cluster instead (ClusterRun), for systems so
+// MINB: blocks an SM holds.  1: the launch is one cluster instead (ClusterRun),
+// for systems so
 // small that a pass is a chain of latencies: no launch boundaries, a hardware
 // barrier between the phases, npass passes of a program that repeats, and
 // the whole register file of an SM for each block.
-template <bool PP, bool WALLS, bool CLUSTER>
-__global__ void __launch_bounds__(128, CLUSTER ? 1 : 3)
+// A cooperative launch takes 3 or 4 (chunk_blocks_per_sm).
+template <bool PP, bool WALLS, int MINB>
+__global__ void __launch_bounds__(128, MINB)
     k_chunk_fp64(const ChunkPass64* __restrict__ prog, int npass, GridSync g, ClusterRun cr) {
+  constexpr bool CLUSTER = MINB == 1;
   __shared__ ChunkPass64 sp;
   // (the larger of the two epilogues')
   __shared__ __align__(16) double stage[EpiStage<EPI_PREDICT, false>::SIZE];

@@ -1861,9 +1861,12 @@ int launch_chunk(dem_ctx* c, int phase, int first = 0, int steps = 0) {
                     c->stream, &c->chunk_blocks, steps > 0 ? &cr : nullptr);
   } else {
     const ChunkPass64* prog = (const ChunkPass64*)c->prog[phase];
+    const int mb = chunk_blocks_per_sm(want);
 #define CCASE(PPV, W)                                                                      \
-  e = steps > 0 ? launch_cluster(k_chunk_fp64<PPV, W, true>, prog, np, cr, c->stream)       \
-                : coop_launch64(k_chunk_fp64<PPV, W, false>, prog, np, g, want, c->stream, \
+  e = steps > 0 ? launch_cluster(k_chunk_fp64<PPV, W, 1>, prog, np, cr, c->stream)         \
+      : mb == 3 ? coop_launch64(k_chunk_fp64<PPV, W, 3>, prog, np, g, want, c->stream,     \
+                                &c->chunk_blocks)                                          \
+                : coop_launch64(k_chunk_fp64<PPV, W, 4>, prog, np, g, want, c->stream,     \
                                 &c->chunk_blocks)
     if (walls) {
       if (c->pp) CCASE(true, true);

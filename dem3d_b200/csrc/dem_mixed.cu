@@ -660,13 +660,16 @@ __device__ __forceinline__ void fold_blocks_mixed(const ChunkPassMx& sp, double*
     __syncthreads();
   }
 }
-// CLUSTER: the launch is one cluster instead (ClusterRun), for systems so
+// MINB: blocks an SM holds.  1: the launch is one cluster instead (ClusterRun),
+// for systems so
 // small that a pass is a chain of latencies: no launch boundaries, a hardware
 // barrier between the phases, npass passes of a program that repeats, and
 // the whole register file of an SM for each block.
-template <bool PP, bool WALLS, bool CONE, bool CLUSTER>
-__global__ void __launch_bounds__(128, CLUSTER ? 1 : 3)
+// A cooperative launch takes 3 or 4 (chunk_blocks_per_sm).
+template <bool PP, bool WALLS, bool CONE, int MINB>
+__global__ void __launch_bounds__(128, MINB)
     k_chunk_mixed(const ChunkPassMx* __restrict__ prog, int npass, GridSync g, ClusterRun cr) {
+  constexpr bool CLUSTER = MINB == 1;
   __shared__ ChunkPassMx sp;
   // (the larger of the two epilogues')
   __shared__ __align__(16) double stage[EpiStage<EPI_PREDICT, true>::SIZE];
@@ -937,10 +940,13 @@ cudaError_t mixed_chunk(bool pp, bool walls, bool cone,
                         const ChunkPass<float4, float2, MixedView>* prog, int npass, GridSync g,
                         int want_blocks, cudaStream_t st, int* blocks_out,
                         const ClusterRun* cluster) {
+  const int mb = chunk_blocks_per_sm(want_blocks);
 #define CCASE(PPV, W, CN)                                                                      \
-  return cluster ? launch_cluster(k_chunk_mixed<PPV, W, CN, true>, prog, npass, *cluster, st)  \
-                 : launch_chunk(k_chunk_mixed<PPV, W, CN, false>, prog, npass, g, want_blocks, \
-                                st, blocks_out)
+  return cluster ? launch_cluster(k_chunk_mixed<PPV, W, CN, 1>, prog, npass, *cluster, st)      \
+         : mb == 3 ? launch_chunk(k_chunk_mixed<PPV, W, CN, 3>, prog, npass, g, want_blocks, st, \
+                                  blocks_out)                                                    \
+                   : launch_chunk(k_chunk_mixed<PPV, W, CN, 4>, prog, npass, g, want_blocks, st, \
+                                  blocks_out)
   if (!walls) {
     if (pp) CCASE(true, false, false);
     CCASE(false, false, false);

@@ -1064,6 +1064,15 @@ __device__ __forceinline__ bool grid_sync(const GridSync& g) {
 
 struct NoView {};
 
+// Blocks per SM of a cooperative chunk launch that has work for `want` blocks.
+// Up to three on each of the 148 SMs the phases are chains of latencies, and
+// 168 registers a thread are worth more than room for a fourth block (20,000
+// spheres on a floor 82 us per step, 91 with four; 16 systems of 200 to 2,000
+// spheres 80 and 84); past that a fourth block's warps hide more than its 0.2
+// to 1.2 kB of spills a thread cost (216k jammed spheres 488, 524 with three;
+// 1M dense 722 and 801; 64 systems of 200 to 20,000 352 and 363).
+inline int chunk_blocks_per_sm(int want) { return want > 3 * 148 ? 4 : 3; }
+
 // Host side: `k` (a chunk kernel) as one cluster of 16 blocks, or of 8 where
 // the device does not take 16.
 template <class K, class CP>
