@@ -87,7 +87,6 @@ struct Counters {
   int abort;         // nonzero: later kernels of a captured sequence do nothing
   int abort_tag;     // 1 + 2*(step within a captured chunk) + pass of the failing pass
   int n_dirty[2];    // cells in dirty list b (transition to cell assignment b)
-  int n_repair;      // cells whose particles' candidate rows are rebuilt this pass
   int full_due;      // this pass rebuilds every candidate row
   int force_full;    // the next pass must rebuild every row (new state, grown rows)
   int row_overflow;  // a candidate row needed more than kc entries
@@ -102,7 +101,8 @@ struct Counters {
   unsigned int disp_max;  // FP32 bits (rounded up) of the largest displacement of one pass
   double disp_acc;   // sum of disp_max since the last full rebuild
   int escape_stop;   // a captured chunk stopped before a step: particles had left the box
-  int pass_id;       // force passes completed; a cell stamped pass_id + 1 has rows to rebuild
+  int pass_id;       // force passes completed; a cell stamped pass_id + 1 is read by rows that
+                     // this pass may have to rebuild
   int barrier_timeout;  // a grid-wide barrier of a persistent launch gave up waiting
   int n_mlist[2];  // entries of CellLists::mlist recorded by the relinks of even / odd stamps
 };
@@ -203,9 +203,11 @@ constexpr int MLIST_CAP = 4096;
 // of src/MForces.f90:199-272: the rest of p's cell list, then the half-shell
 // cells in FirstNeighbour order), as original indices, in that order.
 // meta = the row length; rank = p's position in its cell's list, which with
-// the cell gives the place of p's block in the sweep.  A row stays valid
-// while no cell of its 27-cell neighbourhood gains or loses a particle and
-// no particle has moved skin/2 since the last full rebuild.
+// the cell gives the place of p's block in the sweep.  A row serves until a
+// particle within MinDij + skin of p enters or leaves one of its cells (a
+// farther one left out, or left in, changes no contact before the next full
+// rebuild), or until a particle may have moved 0.4 skin since the last full
+// rebuild, which renews every row.
 struct Rows {
   int* cand;
   int* meta;
@@ -256,8 +258,6 @@ __device__ __forceinline__ void st32(F8* a, const F8& r) {
                : "memory");
 }
 // a velocity copy (double4: one access; float4: 16 bytes)
-__device__ __forceinline__ double4 ldv(const double4* a) { return ld32(a); }
-__device__ __forceinline__ float4 ldv(const float4* a) { return *a; }
 __device__ __forceinline__ void stv(double4* a, double4 r) { st32(a, r); }
 __device__ __forceinline__ void stv(float4* a, float4 r) { *a = r; }
 

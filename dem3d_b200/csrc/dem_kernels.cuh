@@ -648,9 +648,8 @@ __global__ void __launch_bounds__(128) k_rows(const __grid_constant__ TestArgs A
 }
 
 // Relink and rows of a small system in one launch: one cluster of 8 blocks,
-// whose hardware barrier orders the two (a launch boundary less per pass,
-// where a pass is a chain of launches that each take a few microseconds:
-// 12.5k spheres 70.9 -> 67.8 us per step, 2,000 spheres 59.4 -> 53.9).
+// whose hardware barrier orders the two: a launch less per pass, where a pass
+// is a chain of launches that each take a few microseconds (MERGED_LISTS_MAX).
 template <bool PP>
 __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(LIST_THREADS)
     k_lists(const __grid_constant__ RelinkArgs R, const __grid_constant__ TestArgs A) {
@@ -836,7 +835,7 @@ __device__ __forceinline__ void pair_fp64_body(const PassArgs<double4, double2>&
     atomicExch(&A.cnt->in_overflow, 1);
     set_abort(A.cnt, A.tag);
   }
-  publish_counts_block(A.cnt, update, n_col, 0u, 0u, (unsigned)need, (unsigned)need_in);
+  publish_pair_block(A.cnt, update, n_col, (unsigned)need, (unsigned)need_in);
 }
 
 template <bool PP, int MINB>

@@ -652,11 +652,21 @@ StateArrays make_state(double* base, size_t n) {
 // K1: initial distribution (DistributeParticles3D) of the Particle positions
 
 constexpr int LIST_BLOCKS = 148;   // relink and list kernels (grid-stride)
-constexpr int ROWS_BLOCKS = 148 * 4;  // row kernel (grid-stride, 4 warps each)
+// row kernel (grid-stride, 4 warps each): four blocks an SM, from where it
+// gains no more (1M jammed spheres, us per launch of the row kernel with 1, 2,
+// 4 and 8: 51, 31, 22, 22; 1M spheres of two sizes: 24, 22, 22, 22)
+constexpr int ROWS_BLOCKS = 148 * 4;
 // systems whose steps are one launch of one cluster: a thread per sphere
 constexpr int CLUSTER_MAX = 2048;
-// systems whose relink and rows are one launch of one cluster: its 64 warps
-// rebuild this many rows at once in about a launch's time
+// systems whose relink and rows are one launch of one cluster.  A call of its
+// own is a launch shorter by it (us per call on 3,000, 8,000 and 16,000
+// spheres on a floor: 96, 96, 98 against 98, 99, 102; 8,000 jammed 112 against
+// 117); in replayed graphs, where the two kernels are launched ahead of their
+// turn, one cluster is as fast or a little slower (52.8, 56.4, 58.9 us per
+// step against 51.3, 54.8, 57.5; 8,000 jammed 75.7 against 75.2; 16 systems
+// of 200 to 2,000 60.2 against 59.4).  Past 16,384 its 64 warps fall behind
+// where many rows change (32,000 of two sizes: 20 us per launch against 8 and 16
+// side by side, 89.7 per step against 89.0).
 constexpr int MERGED_LISTS_MAX = 16384;
 
 // the slots of every cell from its list (after the lists were built or
@@ -699,7 +709,7 @@ int init_cells(dem_ctx* c) {
   }
   refresh_slots(c);
   // no transition pending; the first pass builds every candidate row
-  CK(cudaMemsetAsync(&c->cnt->n_dirty[0], 0, 3 * sizeof(int), c->stream));
+  CK(cudaMemsetAsync(&c->cnt->n_dirty[0], 0, 2 * sizeof(int), c->stream));
   CK(cudaMemsetAsync(&c->cnt->movers_pending, 0, sizeof(unsigned long long), c->stream));
   CK(cudaMemsetAsync(&c->cnt->disp_max, 0, sizeof(unsigned), c->stream));
   CK(cudaMemsetAsync(&c->cnt->disp_acc, 0, sizeof(double), c->stream));
@@ -3289,7 +3299,7 @@ int dem_move_particles(dem_ctx* c, int32_t step) {
   int st = validate_ready(c);
   if (st) return st;
   if (chunk_cluster(c)) {
-    // one launch and one look at the counters instead of ten and three
+    // one launch and two looks at the counters instead of ten and three
     c->stop_on_escape = false;
     int done = 0;
     bool stopped = false, fresh = false;

@@ -397,7 +397,7 @@ __device__ __forceinline__ void pair_mixed_body(const PassArgs<float4, float2>& 
     atomicExch(&A.cnt->in_overflow, 1);
     set_abort(A.cnt, A.tag);
   }
-  publish_counts_block(A.cnt, update, n_col, 0u, 0u, (unsigned)need, (unsigned)need_in);
+  publish_pair_block(A.cnt, update, n_col, (unsigned)need, (unsigned)need_in);
 }
 
 template <bool PP, int MINB>

@@ -66,52 +66,30 @@ __device__ __forceinline__ void publish_disp(Counters* cnt, double d2) {
   if ((threadIdx.x & 31) == 0 && m) atomicMax(&cnt->disp_max, m);
 }
 
-// Per-warp pass statistics: one atomic per counter per warp.
-__device__ __forceinline__ void publish_counts(Counters* cnt, bool update, unsigned n_col,
-                                               unsigned n_pc, unsigned n_wc, unsigned need) {
+// The pair kernel's statistics over the block (one atomic per counter per
+// block of at most 256 threads): new records, the most records and the most
+// "j" results a particle needs.  All threads of the block call.
+__device__ __forceinline__ void publish_pair_block(Counters* cnt, bool update, unsigned n_col,
+                                                   unsigned need, unsigned need_in) {
   const unsigned FULL = 0xffffffffu;
-  n_col = __reduce_add_sync(FULL, n_col);
-  n_pc = __reduce_add_sync(FULL, n_pc);
-  n_wc = __reduce_add_sync(FULL, n_wc);
-  need = __reduce_max_sync(FULL, need);
-  if ((threadIdx.x & 31) == 0) {
-    if (need) atomicMax(&cnt->need_capacity, (int)need);
-    if (n_col) atomicAdd(update ? &cnt->ncol_pending : &cnt->ncol, (unsigned long long)n_col);
-    if (n_pc) atomicAdd(&cnt->pair_contacts, (unsigned long long)n_pc);
-    if (n_wc) atomicAdd(&cnt->wall_contacts, (unsigned long long)n_wc);
-  }
-}
-
-// The same statistics summed over the block first (one atomic per counter
-// per block of at most 256 threads), together with the largest number of
-// "j" records a particle received.  All threads of the block call.
-__device__ __forceinline__ void publish_counts_block(Counters* cnt, bool update, unsigned n_col,
-                                                     unsigned n_pc, unsigned n_wc,
-                                                     unsigned need, unsigned need_in) {
-  const unsigned FULL = 0xffffffffu;
-  __shared__ unsigned s_c[8][5];
+  __shared__ unsigned s_c[8][3];
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const unsigned v[5] = {__reduce_add_sync(FULL, n_col), __reduce_add_sync(FULL, n_pc),
-                         __reduce_add_sync(FULL, n_wc), __reduce_max_sync(FULL, need),
+  const unsigned v[3] = {__reduce_add_sync(FULL, n_col), __reduce_max_sync(FULL, need),
                          __reduce_max_sync(FULL, need_in)};
   if (lane == 0)
 #pragma unroll
-    for (int k = 0; k < 5; k++) s_c[wid][k] = v[k];
+    for (int k = 0; k < 3; k++) s_c[wid][k] = v[k];
   __syncthreads();
   if (threadIdx.x == 0) {
-    unsigned t[5] = {0u, 0u, 0u, 0u, 0u};
+    unsigned t[3] = {0u, 0u, 0u};
     for (int w = 0; w < (int)(blockDim.x >> 5); w++) {
       t[0] += s_c[w][0];
-      t[1] += s_c[w][1];
-      t[2] += s_c[w][2];
-      t[3] = t[3] > s_c[w][3] ? t[3] : s_c[w][3];
-      t[4] = t[4] > s_c[w][4] ? t[4] : s_c[w][4];
+      t[1] = t[1] > s_c[w][1] ? t[1] : s_c[w][1];
+      t[2] = t[2] > s_c[w][2] ? t[2] : s_c[w][2];
     }
     if (t[0]) atomicAdd(update ? &cnt->ncol_pending : &cnt->ncol, (unsigned long long)t[0]);
-    if (t[1]) atomicAdd(&cnt->pair_contacts, (unsigned long long)t[1]);
-    if (t[2]) atomicAdd(&cnt->wall_contacts, (unsigned long long)t[2]);
-    if (t[3]) atomicMax(&cnt->need_capacity, (int)t[3]);
-    if (t[4]) atomicMax(&cnt->need_in, (int)t[4]);
+    if (t[1]) atomicMax(&cnt->need_capacity, (int)t[1]);
+    if (t[2]) atomicMax(&cnt->need_in, (int)t[2]);
   }
 }
 

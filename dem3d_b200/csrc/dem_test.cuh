@@ -169,7 +169,6 @@ __device__ __forceinline__ void relink_body(const DevParams* __restrict__ PT,
   }
   if (first_thread) {
     const DevParams& P = PT[0];  // the integrator settings are shared
-    cnt->n_repair = 0;
     cnt->n_mlist[(stamp & 1) ^ 1] = 0;  // for the next pass's relink
     cnt->n_dirty[par ^ 1] = 0;
     cnt->movers = cnt->movers_pending;
