@@ -98,7 +98,10 @@ struct Counters {
   int n_contacts;    // length of this pass's contact list
   int list_error;    // a cell-list walk exceeded its bound (corrupt lists)
   int nonfinite;     // a particle position became NaN or infinite
-  unsigned int disp_max;  // FP32 bits (rounded up) of the largest displacement of one pass
+  // FP32 bits (rounded up) of the largest displacement of one pass.  Not in the
+  // line of the abort word, which every warp of the fold reads while others
+  // raise this one (64 systems with floors: 61.8 us per launch, apart 60.2).
+  alignas(128) unsigned int disp_max;
   double disp_acc;   // sum of disp_max since the last full rebuild
   int escape_stop;   // a captured chunk stopped before a step: particles had left the box
   int pass_id;       // force passes completed; a cell stamped pass_id + 1 is read by rows that
