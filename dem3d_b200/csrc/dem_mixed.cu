@@ -418,25 +418,27 @@ __device__ __forceinline__ void fold_mixed_body(const PassArgs<float4, float2>& 
   __shared__ int s_abort;
   const int p0 = vblock * blockDim.x + threadIdx.x;
   const int p = p0 < A.n ? p0 : 0;
-  // the integrator's columns and the particle's own data are requested
-  // together, ahead of the abort word
-  stage_epilogue<EPI, true>(A, vblock * blockDim.x, stage);
+  // requested together: the abort word (one decision for the warp; with walls,
+  // for the block, which meets block barriers later), what the contact results
+  // hang on, the particle's own data, then the integrator's columns.  (The
+  // columns first: 119.7 us per launch at 1M spheres with 0.8 contacts each
+  // instead of 116.7, 416 instead of 398 at 4M.  The FP64 fold has them first
+  // and loses the other way round, 131.5 instead of 128.4.)
+  int stop = 0;
+  if (threadIdx.x == 0 || (!WALLS && (threadIdx.x & 31) == 0)) stop = A.cnt->abort;
+  const int ni = A.in_cnt[p];
+  const unsigned matched = A.matched[p];
   const int c = A.cell_cur[p];
   const int rank = A.rank[p];
   const int nc = A.ccount[p];
   const int st0 = A.cstart[p];
   const double4 p4 = ld32(A.X + p);
-  const int ni = A.in_cnt[p];
-  const unsigned matched = A.matched[p];
-  // one decision for the warp (with walls, for the block: it meets block
-  // barriers later)
-  int stop = 0;
+  stage_epilogue<EPI, true>(A, vblock * blockDim.x, stage);
   if (WALLS) {
-    if (threadIdx.x == 0) s_abort = A.cnt->abort;
+    if (threadIdx.x == 0) s_abort = stop;
     __syncthreads();
     stop = s_abort;
   } else {
-    if ((threadIdx.x & 31) == 0) stop = A.cnt->abort;
     stop = __shfl_sync(0xffffffffu, stop, 0);
   }
   if (stop) {
@@ -622,7 +624,8 @@ __device__ __forceinline__ void fold_mixed_body(const PassArgs<float4, float2>& 
 // budget: 5 blocks of 128 per SM, 96 registers, no spills without cones; the
 // corrector without walls, which needs fewer, 7 blocks, 72 registers (1M
 // spheres, mean of the two kernels: 127 -> 119 us per launch with 0.8
-// contacts each, 198 -> 189 with 6.6; with walls it would spill, 61 -> 65 us).
+// contacts each, 198 -> 189 with 6.6, both 2 less since its requests are in
+// today's order; with walls it would spill, 61 -> 65 us).
 // The predictor at 6 blocks loses on the dense packing (210 against 196) what
 // it gains on the thin one; one record in flight instead of two: 134 against
 // 127.  Before the columns were staged, the records read in 32-byte pieces
