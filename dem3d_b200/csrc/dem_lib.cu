@@ -245,6 +245,7 @@ int fail(dem_ctx* c, int code, const std::string& msg) {
 
 int cuda_fail(dem_ctx* c, cudaError_t e, const char* where) {
   std::string m = std::string("CUDA error in ") + where + ": " + cudaGetErrorString(e);
+  (void)cudaGetLastError();  // (reported here, not once more by the next call)
   return fail(c, DEM_ERR_CUDA, m);
 }
 
@@ -384,6 +385,7 @@ void free_lists(dem_ctx* c) {
                &L.mnext, &L.dflag, &L.rflag,   &L.dlist[0], &L.dlist[1],
                &L.slot,  &L.slot_n, &L.rstamp};
   cudaFree(L.mlist);
+  L.mlist = nullptr;
   for (int** q : f) {
     cudaFree(*q);
     *q = nullptr;
@@ -827,10 +829,8 @@ int grow_contacts(dem_ctx* c, int need) {
   if (cap > (1ll << 30)) return fail(c, DEM_ERR_CAPACITY, "contact list beyond 2^30 contacts");
   if (cap == c->cl_cap) return DEM_OK;
   CK(cudaStreamSynchronize(c->stream));
-  int st = alloc_contacts(c, (int)cap);
-  if (st) return st;
   drop_graphs(c);
-  return DEM_OK;
+  return alloc_contacts(c, (int)cap);
 }
 
 // more "j" records per particle (the records only live within a pass)
@@ -839,10 +839,8 @@ int grow_incoming(dem_ctx* c, int need) {
   while (cap < need) cap *= 2;
   if (cap == c->in_cap) return DEM_OK;
   CK(cudaStreamSynchronize(c->stream));
-  int st = alloc_incoming(c, cap);
-  if (st) return st;
   drop_graphs(c);
-  return DEM_OK;
+  return alloc_incoming(c, cap);
 }
 
 // room for the two-kernel handover of a pass (counts start at zero)
@@ -850,6 +848,7 @@ int ensure_pass_buffers(dem_ctx* c) {
   const int N = std::max(c->ncap, 1);
   if (c->pass_cap >= N) return DEM_OK;
   CK(cudaStreamSynchronize(c->stream));
+  drop_graphs(c);
   cudaFree(c->in_cnt);
   cudaFree(c->wall_part);
   cudaFree(c->cstart);
@@ -873,7 +872,6 @@ int ensure_pass_buffers(dem_ctx* c) {
   const size_t parts = (size_t)blocks_for(N, 128) * NWM;
   CK(cudaMalloc(&c->wall_part, sizeof(double) * parts));
   CK(cudaMemset(c->wall_part, 0, sizeof(double) * parts));
-  drop_graphs(c);
   return alloc_incoming(c, c->in_cap);
 }
 
@@ -1205,13 +1203,13 @@ int grow_rows(dem_ctx* c, int need) {
   int kc = std::max(need, c->kc + c->kc / 2);
   kc = std::min((kc + 7) / 8 * 8, KC_MAX);
   CK(cudaStreamSynchronize(c->stream));
+  drop_graphs(c);
   cudaFree(c->rows.cand);
   c->rows.cand = nullptr;
   // (room for every particle that can still be poured, as at dem_set_state)
   CK(cudaMalloc(&c->rows.cand, sizeof(int) * (size_t)std::max(c->ncap, 1) * kc));
   c->kc = kc;
   c->rows.kc = kc;
-  drop_graphs(c);
   return DEM_OK;
 }
 
@@ -1231,21 +1229,16 @@ int finish_pass(dem_ctx* c, int side, bool update, double dt, int epi, const Rin
     if (attempt >= 8) return fail(c, DEM_ERR_CAPACITY, "capacity cannot be grown");
     st = clear_abort(c);
     if (st) return st;
-    if (h.overflow) {
-      st = grow_history(c, std::max(h.need_capacity, c->hcap + 1));
-      if (st) return st;
-    }
-    if (h.in_overflow) {
-      st = grow_incoming(c, std::max(h.need_in, c->in_cap + 1));
-      if (st) return st;
-    }
-    if (h.cl_overflow) {
-      st = grow_contacts(c, std::max(h.need_cl, c->cl_cap + 1));
-      if (st) return st;
+    if (h.overflow) st = grow_history(c, std::max(h.need_capacity, c->hcap + 1));
+    if (!st && h.in_overflow) st = grow_incoming(c, std::max(h.need_in, c->in_cap + 1));
+    if (!st && h.cl_overflow) st = grow_contacts(c, std::max(h.need_cl, c->cl_cap + 1));
+    if (!st && h.row_overflow) st = grow_rows(c, h.need_kc);
+    if (st) {
+      // the pass is left between its relink and its end
+      c->cells_ready = false;
+      return st;
     }
     if (h.row_overflow) {
-      st = grow_rows(c, h.need_kc);
-      if (st) return st;
       const int one = 1;
       CK(cudaMemcpyAsync(&c->cnt->full_due, &one, sizeof(int), cudaMemcpyHostToDevice,
                          c->stream));
@@ -1670,6 +1663,13 @@ int validate_ready(dem_ctx* c) {
   if (!c->cells_ready)
     return fail(c, DEM_ERR_STATE, "cell distribution not initialised (call "
                                   "dem_initialize_cell_distribution)");
+  // an array that was freed to grow and found no memory
+  const void* const arrays[] = {c->rows.cand, c->irec,    c->in_rec, c->in_cnt,
+                                c->matched,   c->cstart, c->ccount, c->wall_part};
+  bool lost = (c->nprev > 0 && !c->amsum) || (c->fluid && !c->drag);
+  for (const void* a : arrays) lost = lost || !a;
+  if (lost)
+    return fail(c, DEM_ERR_STATE, "device memory ran out while an array grew; set the state again");
   return DEM_OK;
 }
 
@@ -2102,9 +2102,10 @@ int permute_particles(dem_ctx* c, const int* pi) {
   col(c->rows.rank, 4);
   // the candidate rows move with their particles and are renamed below:
   // the same partners in the same order, so no row is rebuilt
-  slab_col(C, c->rows.cand, 4, c->rows.kc, (long long)n * 4);
-  col(c->in_cnt, 4);
-  col(c->matched, 4);
+  // (none of these three after a growth that found no memory: validate_ready)
+  if (c->rows.cand) slab_col(C, c->rows.cand, 4, c->rows.kc, (long long)n * 4);
+  if (c->in_cnt) col(c->in_cnt, 4);
+  if (c->matched) col(c->matched, 4);
   if (C.overflow) return fail(c, DEM_ERR_STATE, "reorder: too many particle arrays");
   size_t most = 0;
   for (int k = 0; k < C.n; k++) most = std::max(most, (size_t)C.elem[k] * C.rows[k] * (size_t)n);
@@ -2133,7 +2134,7 @@ int permute_particles(dem_ctx* c, const int* pi) {
   remap(c->L.arr_head, nc);
   remap(c->L.slot, nc * c->L.scap);
   for (int b = 0; b < 2; b++) remap(c->H[b].key, (long long)c->H[b].cap * c->H[b].n);
-  remap(c->rows.cand, (long long)c->rows.kc * n);
+  if (c->rows.cand) remap(c->rows.cand, (long long)c->rows.kc * n);
   CK(cudaStreamSynchronize(c->stream));
   cudaFree(tmp);
   cudaFree(inv);
@@ -2737,6 +2738,7 @@ int dem_set_state(dem_ctx* c, int32_t n, const int32_t* comp, const double* radi
   CK(cudaStreamSynchronize(c->stream));
   drop_graphs(c);
   free_state(c);
+  c->state_set = c->cells_ready = false;  // (until every array is there)
   c->n = n;
   // Component(:)%Number, and room for pouring up to the targets
   c->comp_count.assign((size_t)std::max(c->params.n_components, 0), 0);
@@ -4012,7 +4014,8 @@ int dem_slab_phase(dem_ctx* c, int32_t step, int32_t pass, int32_t phase) {
   const bool update = pass == 0;
   const int epi = pass == 0 ? EPI_PREDICT : EPI_CORRECT;
   const double dt = c->params.time_step;
-  int st = DEM_OK;
+  int st = validate_ready(c);
+  if (st) return st;
   switch (phase) {
     case DEM_SLAB_RELINK:
       st = ensure_drag(c);
@@ -4064,7 +4067,8 @@ int dem_slab_pack(dem_ctx* c, int32_t what, void* buf, int64_t cap, int64_t* byt
   if (!c || !buf || !bytes) return DEM_ERR_INVALID;
   if (!c->slab) return fail(c, DEM_ERR_STATE, "slab: dem_slab_set_range first");
   int count = 0;
-  int st = DEM_OK;
+  int st = validate_ready(c);
+  if (st) return st;
   std::vector<int> extra;
   switch (what) {
     case DEM_SLAB_GHOSTS: {
@@ -4166,7 +4170,8 @@ int dem_slab_unpack(dem_ctx* c, int32_t what, const void* buf, int64_t bytes) {
   if (!c->slab) return fail(c, DEM_ERR_STATE, "slab: dem_slab_set_range first");
   std::vector<int> h;
   int64_t body = 0;
-  int st = slab_read_head(c, buf, bytes, what, h, &body);
+  int st = validate_ready(c);
+  if (!st) st = slab_read_head(c, buf, bytes, what, h, &body);
   if (st) return st;
   const int count = h[1], rec = h[2];
   const char* recs = (const char*)buf + body;
