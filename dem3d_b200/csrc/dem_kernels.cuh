@@ -648,8 +648,8 @@ __global__ void __launch_bounds__(128) k_rows(const __grid_constant__ TestArgs A
 }
 
 // Relink and rows of a small system in one launch: one cluster of 8 blocks,
-// whose hardware barrier orders the two: a launch less per pass, where a pass
-// is a chain of launches that each take a few microseconds (MERGED_LISTS_MAX).
+// whose hardware barrier orders the two; a launch less per pass where the host
+// launches each (MERGED_LISTS_MAX).
 template <bool PP>
 __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(LIST_THREADS)
     k_lists(const __grid_constant__ RelinkArgs R, const __grid_constant__ TestArgs A) {

@@ -660,15 +660,17 @@ constexpr int LIST_BLOCKS = 148;   // relink and list kernels (grid-stride)
 constexpr int ROWS_BLOCKS = 148 * 4;
 // systems whose steps are one launch of one cluster: a thread per sphere
 constexpr int CLUSTER_MAX = 2048;
-// systems whose relink and rows are one launch of one cluster.  A call of its
-// own is a launch shorter by it (us per call on 3,000, 8,000 and 16,000
-// spheres on a floor: 96, 96, 98 against 98, 99, 102; 8,000 jammed 112 against
-// 117); in replayed graphs, where the two kernels are launched ahead of their
-// turn, one cluster is as fast or a little slower (52.8, 56.4, 58.9 us per
-// step against 51.3, 54.8, 57.5; 8,000 jammed 75.7 against 75.2; 16 systems
-// of 200 to 2,000 60.2 against 59.4).  Past 16,384 its 64 warps fall behind
-// where many rows change (32,000 of two sizes: 20 us per launch against 8 and 16
-// side by side, 89.7 per step against 89.0).
+// systems whose relink and rows are one launch of one cluster where the host
+// launches every kernel by itself (single calls, the Euler start-up): a launch
+// less (us per call on 3,000, 8,000 and 16,000 spheres on a floor: 96, 96, 98
+// against 98, 99, 102; 8,000 jammed 112 against 117).  In a captured chunk the
+// two kernels cost no launch and are scheduled ahead of their turn, which the
+// two parts of one cluster are not (merged against two kernels, us per step:
+// 8,000 and 16,000 on a floor 55.6 and 57.4 against 53.8 and 56.3, a shaken
+// hopper of 12,000 70.1 against 68.5; 16 systems of 200 to 2,000 59.5 against
+// 59.7, 8,000 jammed level).  Past 16,384 the cluster's 64 warps fall behind
+// where many rows change (32,000 of two sizes: 20 us per launch against 8 and
+// 16 side by side).
 constexpr int MERGED_LISTS_MAX = 16384;
 
 // the slots of every cell from its list (after the lists were built or
@@ -1113,7 +1115,7 @@ void pass_lists(dem_ctx* c, int side, bool update, int tag, bool early) {
     c->rec_rl = R;
     return;
   }
-  if (!c->slab && c->n > 0 && c->n <= MERGED_LISTS_MAX) {
+  if (!c->slab && !c->capturing && c->n > 0 && c->n <= MERGED_LISTS_MAX) {
     const TestArgs T = test_args(c, side, tag);
     if (c->pp) launch_early(c, early, "lists", k_lists<true>, 8u, (unsigned)LIST_THREADS, R, T);
     else launch_early(c, early, "lists", k_lists<false>, 8u, (unsigned)LIST_THREADS, R, T);

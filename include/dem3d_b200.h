@@ -383,10 +383,10 @@ int dem_get_tuning(dem_ctx* ctx, double* skin_factor, int32_t* pass_variant);
  * its order).
  *  - launch_mode: how dem_run issues its 4-step chunks.  0 (default): a
  *    CUDA graph of the chunk's kernels (relink, rows, test, pair, fold per
- *    force pass: 10 launches per step; 8 up to 16,384 particles); one system
- *    of up to 2,048 particles without fluid drag runs its steps (also that of
- *    dem_move_particles) as one launch of one thread-block cluster.  1: one persistent cooperative launch per
- *    chunk, as many blocks of 128 threads as fit on the GPU at once, which
+ *    force pass: 10 launches per step); one system of up to 2,048 particles
+ *    without fluid drag runs its steps (also that of dem_move_particles) as
+ *    one launch of one thread-block cluster.  1: one persistent cooperative
+ *    launch per chunk, as many blocks of 128 threads as fit on the GPU at once, which
  *    step through the 8 passes' phases with grid-wide barriers between them
  *    (every wait bounded: see dem_set_persistent_barrier).  Chunks with
  *    moving walls, fluid drag or kernel profiling run as graphs.

@@ -98,7 +98,7 @@ def test_graphs_and_persistent_chunks(mode, order, precision):
     a.set_launch_shape(launch_mode=mode)
     b.set_profiling(True)
     others = [b] if precision else [b, make(oracle_system)]
-    _follow(a, others, 8)
+    _follow(a, others, 10)
     assert mode == 0 or a.persistent_blocks() > 0
     assert a.ncol() > 0
 
