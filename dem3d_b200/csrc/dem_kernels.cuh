@@ -659,8 +659,7 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(LIST_THREADS)
   const int warp = blockIdx.x * (LIST_THREADS / 32) + w, nwarps = 8 * (LIST_THREADS / 32);
   relink_body(R.PT, R.cellsys, R.L, R.par, R.n, R.update, R.stop_tag, R.cnt, warp, nwarps, sh[w]);
   __threadfence();
-  asm volatile("barrier.cluster.arrive.release.aligned;\n"
-               "barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  cluster_sync();
   rows_body<PP>(A, warp, nwarps);
 }
 

@@ -1009,6 +1009,7 @@ struct ClusterRun {
 // release / acquire at cluster scope: what every thread of the cluster wrote
 // before is visible to every thread after
 __device__ __forceinline__ void cluster_sync() {
+  __syncwarp();  // (the aligned forms take whole warps; the phases end with lanes apart)
   asm volatile("barrier.cluster.arrive.release.aligned;\n"
                "barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
