@@ -1236,8 +1236,8 @@ int finish_pass(dem_ctx* c, int side, bool update, double dt, int epi, const Rin
     if (!st && h.cl_overflow) st = grow_contacts(c, std::max(h.need_cl, c->cl_cap + 1));
     if (!st && h.row_overflow) st = grow_rows(c, h.need_kc);
     if (st) {
-      // the pass is left between its relink and its end
-      c->cells_ready = false;
+      // (no memory: the pass is left between its relink and its end)
+      if (st == DEM_ERR_CUDA) c->cells_ready = false;
       return st;
     }
     if (h.row_overflow) {
